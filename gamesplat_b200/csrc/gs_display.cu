@@ -15,6 +15,8 @@
 // against it.
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "gs_common.cuh"
 #include "gs_display.h"
 
@@ -23,51 +25,87 @@ namespace gs {
 __device__ __forceinline__ float det_exp2f(float x) { return det_expf(mul(x, kLn2f)); }
 __device__ __forceinline__ float det_log2f(float x) { return mul(det_logf(x), kInvLn2); }
 
-__device__ __forceinline__ float lut_entry(const uint16_t* __restrict__ lut, int n, int x, int y, int z, int c) {
-    const int i = ((z * n + y) * n + x) * 3 + c;
-    return dv((float)__ldg(lut + i), 65535.0f);
+// The table the display kernel reads: the uploaded uint16 lattice as floats
+// (entry / 65535, the division the shader does per fetch), 16 bytes a point.
+__global__ void display_table_kernel(const uint16_t* __restrict__ lut, size_t points, float4* __restrict__ table) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < points; i += (size_t)gridDim.x * blockDim.x) {
+        const uint16_t* a = lut + i * 3;
+        table[i] = make_float4(dv((float)a[0], 65535.0f), dv((float)a[1], 65535.0f), dv((float)a[2], 65535.0f), 0.0f);
+    }
 }
 
-__global__ void display_lut_kernel(DisplayParams p) {
+int launch_display_table(const uint16_t* lut, int lut_size, float4* table, uint32_t num_sms, cudaStream_t s) {
+    const size_t points = (size_t)lut_size * lut_size * lut_size;
+    const size_t grid = std::min((points + 255) / 256, (size_t)num_sms * 16);
+    display_table_kernel<<<(unsigned)grid, 256, 0, s>>>(lut, points, table);
+    return 1;
+}
+
+// g_mix with the weights 1 - a and a in hand.
+__device__ __forceinline__ float mix_w(float x, float y, float wx, float wy) { return add(mul(x, wx), mul(y, wy)); }
+
+// Bound by instruction issue (~600 warp instructions a pixel, most of them
+// the three deterministic logarithms and their divisions), not by the 24
+// bytes a pixel moves: 35 us at 1920x1080 with a 33^3 table, against 72 us
+// when every fetch was three uint16 loads and three divisions by 65535 (24 of
+// each a pixel).  Points interleaved with their +x neighbour (one 32-byte load
+// for two fetches) measured the same 35 us with twice the table.
+__global__ void __launch_bounds__(256) display_lut_kernel(DisplayParams p) {
     const size_t npix = (size_t)p.width * p.height;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= npix) return;
+    uint2 h = __ldg(reinterpret_cast<const uint2*>(p.in_rgba16f) + i);
     const float gain = det_exp2f(p.exposure_ev);
     const float lo_clamp = det_exp2f(p.log2_min);
     const float range = sub(p.log2_max, p.log2_min);
-    const float top = (float)(p.lut_size - 1);
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += (size_t)gridDim.x * blockDim.x) {
-        const uint2 h = reinterpret_cast<const uint2*>(p.in_rgba16f)[i];
+    const int n = p.lut_size, nn = n * n;
+    const float top = (float)(n - 1);
+    for (;;) {
+        const size_t next = i + stride;
+        const bool more = next < npix;
+        uint2 hn = make_uint2(0u, 0u);
+        if (more) hn = __ldg(reinterpret_cast<const uint2*>(p.in_rgba16f) + next);
         const float2 rg = __half22float2(*reinterpret_cast<const __half2*>(&h.x));
         const float2 ba = __half22float2(*reinterpret_cast<const __half2*>(&h.y));
-        if (!p.lut) {
+        if (!p.table) {
             p.out_rgba32f[i] = make_float4(rg.x, rg.y, ba.x, ba.y);
-            continue;
-        }
-        const float rad[3] = {mul(rg.x, gain), mul(rg.y, gain), mul(ba.x, gain)};
-        int lo[3], hi[3];
-        float f[3];
+        } else {
+            const float rad[3] = {mul(rg.x, gain), mul(rg.y, gain), mul(ba.x, gain)};
+            int lo[3], up[3];
+            float f[3], e[3];   // weights of the upper and the lower lattice point
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            float s = g_clamp(dv(sub(det_log2f(g_max(rad[c], lo_clamp)), p.log2_min), range), 0.0f, 1.0f);
-            if (s != s) s = 0.0f;   // NaN input: first lattice entry (as the oracle)
-            const float pc = mul(s, top);
-            const float fl = floorf(pc);
-            lo[c] = (int)fl;
-            hi[c] = min(lo[c] + 1, p.lut_size - 1);
-            f[c] = sub(pc, fl);
+            for (int c = 0; c < 3; ++c) {
+                float s = g_clamp(dv(sub(det_log2f(g_max(rad[c], lo_clamp)), p.log2_min), range), 0.0f, 1.0f);
+                if (s != s) s = 0.0f;   // NaN input: first lattice entry (as the oracle)
+                const float pc = mul(s, top);
+                const float fl = floorf(pc);
+                lo[c] = (int)fl;
+                up[c] = lo[c] + 1 < n ? 1 : 0;
+                f[c] = sub(pc, fl);
+                e[c] = sub(1.0f, f[c]);
+            }
+            const int base = lo[2] * nn + lo[1] * n + lo[0];
+            const int dx = up[0], dy = up[1] ? n : 0, dz = up[2] ? nn : 0;
+            const float4* t = p.table + base;
+            const float4 l000 = __ldg(t), l100 = __ldg(t + dx), l010 = __ldg(t + dy), l110 = __ldg(t + dy + dx);
+            const float4 l001 = __ldg(t + dz), l101 = __ldg(t + dz + dx), l011 = __ldg(t + dz + dy),
+                         l111 = __ldg(t + dz + dy + dx);
+            const float ex = e[0], fx = f[0], ey = e[1], fy = f[1], ez = e[2], fz = f[2];
+            auto trilinear = [&](float a000, float a100, float a010, float a110, float a001, float a101, float a011,
+                                 float a111) {
+                const float a = mix_w(mix_w(a000, a100, ex, fx), mix_w(a010, a110, ex, fx), ey, fy);
+                const float b = mix_w(mix_w(a001, a101, ex, fx), mix_w(a011, a111, ex, fx), ey, fy);
+                return mix_w(a, b, ez, fz);
+            };
+            const float o[3] = {trilinear(l000.x, l100.x, l010.x, l110.x, l001.x, l101.x, l011.x, l111.x),
+                                trilinear(l000.y, l100.y, l010.y, l110.y, l001.y, l101.y, l011.y, l111.y),
+                                trilinear(l000.z, l100.z, l010.z, l110.z, l001.z, l101.z, l011.z, l111.z)};
+            p.out_rgba32f[i] = make_float4(o[0], o[1], o[2], 1.0f);
         }
-        float o[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const int n = p.lut_size;
-            const float a = g_mix(g_mix(lut_entry(p.lut, n, lo[0], lo[1], lo[2], c), lut_entry(p.lut, n, hi[0], lo[1], lo[2], c), f[0]),
-                                  g_mix(lut_entry(p.lut, n, lo[0], hi[1], lo[2], c), lut_entry(p.lut, n, hi[0], hi[1], lo[2], c), f[0]),
-                                  f[1]);
-            const float b = g_mix(g_mix(lut_entry(p.lut, n, lo[0], lo[1], hi[2], c), lut_entry(p.lut, n, hi[0], lo[1], hi[2], c), f[0]),
-                                  g_mix(lut_entry(p.lut, n, lo[0], hi[1], hi[2], c), lut_entry(p.lut, n, hi[0], hi[1], hi[2], c), f[0]),
-                                  f[1]);
-            o[c] = g_mix(a, b, f[2]);
-        }
-        p.out_rgba32f[i] = make_float4(o[0], o[1], o[2], 1.0f);
+        if (!more) break;
+        i = next;
+        h = hn;
     }
 }
 

@@ -81,7 +81,7 @@ struct gs_ctx {
     std::string last_error;
 
     // display transform LUT (gsanim 0.3 "layers" scenes)
-    uint16_t* display_lut = nullptr;
+    float4* display_table = nullptr;     // lut_size^3 points, then the uint16 lattice they came from
     int lut_size = 0;
     float lut_log2_min = 0.0f, lut_log2_max = 0.0f;
 
@@ -1249,7 +1249,7 @@ void gs_destroy(gs_ctx* c) {
     if (c->fc_stream) cudaStreamSynchronize(c->fc_stream);
     release_scene(c);
     release_targets(c);
-    dfree(c->display_lut);
+    dfree(c->display_table);
     if (c->h_fc) cudaFreeHost(c->h_fc);
     if (c->h_bin_fc) cudaFreeHost(c->h_bin_fc);
     if (c->h_slot_fc) cudaFreeHost(c->h_slot_fc);
@@ -1561,15 +1561,20 @@ int gs_set_display_lut(gs_ctx* c, const uint16_t* lut, uint32_t lut_size, float 
     cudaSetDevice(c->device);
     // a queued gs_display may still read the old table
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return cuda_fail(c, cudaGetLastError(), "stream sync");
-    dfree(c->display_lut);
+    dfree(c->display_table);
     c->lut_size = 0;
     if (!lut) return GS_OK;
     // src/gaussian_loader_gsanim.cpp:237,244
     if (lut_size < 2 || lut_size > 256) return fail(c, GS_ERR_BAD_ARG, "display LUT size must be 2..256");
     if (!(log2_min < log2_max)) return fail(c, GS_ERR_BAD_ARG, "display LUT needs log2_min < log2_max");
-    const size_t count = (size_t)lut_size * lut_size * lut_size * 3;
-    GS_CUDA(c, dalloc(&c->display_lut, count * sizeof(uint16_t)));
-    GS_CUDA(c, cudaMemcpy(c->display_lut, lut, count * sizeof(uint16_t), cudaMemcpyHostToDevice));
+    // one allocation: the float table the kernel reads and, behind it, the uint16 lattice it is made from
+    const size_t points = (size_t)lut_size * lut_size * lut_size, raw_bytes = points * 3 * sizeof(uint16_t);
+    GS_CUDA(c, dalloc(&c->display_table, points * sizeof(float4) + raw_bytes));
+    uint16_t* raw = reinterpret_cast<uint16_t*>(c->display_table + points);
+    GS_CUDA(c, cudaMemcpyAsync(raw, lut, raw_bytes, cudaMemcpyHostToDevice, c->stream));
+    gs::launch_display_table(raw, (int)lut_size, c->display_table, c->num_sms, c->stream);
+    GS_CUDA(c, cudaGetLastError());
+    GS_CUDA(c, cudaStreamSynchronize(c->stream));   // the caller may reuse `lut` on return
     c->lut_size = (int)lut_size;
     c->lut_log2_min = log2_min;
     c->lut_log2_max = log2_max;
@@ -1586,7 +1591,7 @@ int gs_display(gs_ctx* c, const uint16_t* rgba16f_in, float* rgba32f_out, int wi
     p.out_rgba32f = reinterpret_cast<float4*>(rgba32f_out);
     p.width = width;
     p.height = height;
-    p.lut = c->lut_size ? c->display_lut : nullptr;
+    p.table = c->lut_size ? c->display_table : nullptr;
     p.lut_size = c->lut_size;
     p.log2_min = c->lut_log2_min;
     p.log2_max = c->lut_log2_max;

@@ -21,7 +21,9 @@
 
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "gs_common.cuh"
 #include "gs_internal.h"
@@ -751,52 +753,149 @@ __global__ void __launch_bounds__(kCullThreads, 6) cull_project_half_kernel(Cull
     }
 }
 
-// Colours of a frame's binned records for another gsanim appearance state
-// (a frame of a state batch: the geometry, order and tiles of the frame stay,
-// the colours change).  Record i (sorted position) gets the colour the
-// projection pass would give its splat under the state of `p`: the same row,
-// deltas, view direction, SH degree and operations (animate_row, sh_eval,
-// shaders/cull.glsl:125-164, 323-417), bias and clamp.
-__global__ void __launch_bounds__(128) recolour_kernel(CullParams p, const RasterRecord* __restrict__ records,
-                                                       float4* __restrict__ colours) {
+// Colours of a frame's binned records under the appearance states of a batch:
+// record i (sorted position) gets, per frame, the colour the projection pass
+// would give its splat under that frame's states: the same row, deltas, view
+// direction, SH degree and operations (animate_row, sh_eval,
+// shaders/cull.glsl:125-164, 323-417), bias and clamp.  A thread takes a record
+// through every frame: the 256-byte row, the direction and the SH basis are
+// read and evaluated once, and a frame costs its 48 (blended: 96) delta bytes,
+// read as 16-byte loads (a delta row is 48 bytes).  Colours leave through
+// shared memory so that a group's rows are written whole.  Issue-bound: ~13
+// operations a coefficient of a blended frame.  1M rows, 16 blended frames:
+// 16 launches of 182 us (byte loads, row and basis per frame) before.
+constexpr int kRecolourThreads = 128;
+
+// int8 k of a word (already xor 0x80808080) as float: 2^23 + 128 + q has q's bits, biased, in its low mantissa byte
+__device__ __forceinline__ float int8_of(uint32_t biased, int k) {
+    return __uint_as_float(__byte_perm(biased, 0x4B000000u, 0x7440u + (uint32_t)k)) - 8388736.0f;
+}
+
+template <int kGroup>
+__global__ void __launch_bounds__(kRecolourThreads) recolour_states_kernel(CullParams p,
+                                                                           const RasterRecord* __restrict__ records,
+                                                                           StateBatch st, int first, int frames,
+                                                                           float* __restrict__ colours) {
+    pdl_wait();
+    constexpr int kRow = 3 * kGroup;                       // floats of a record in a group
+    __shared__ float s_col[kRecolourThreads][kRow + 1];    // odd stride: a thread's row in its own banks
+    __shared__ __align__(16) float s_scale[48];
+    const int t = threadIdx.x;
+    if (t < 48) s_scale[t] = p.anim_scales[t];
     const uint32_t n_vis = p.fc->visible_count;
     CamRegs cam;
     load_cam(p.cam, cam);
-    // the shader blends whenever the weight is positive, states 0 and 0
-    // included (gsanim_sample returns {0, 0, w} between two linear keys of
-    // the base state), and (1 - w) x + w x need not round to x
-    const bool animated = p.anim_deltas != nullptr && (p.anim_state_a != 0 || p.anim_weight > 0.0f);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_vis; i += gridDim.x * blockDim.x) {
-        const uint32_t id = records[i].splat_id;
-        if (id >= p.n) continue;
-        float4 row[16];
+    __syncthreads();
+    for (uint32_t i0 = blockIdx.x * kRecolourThreads; i0 < n_vis; i0 += gridDim.x * kRecolourThreads) {
+        const uint32_t i = i0 + t;
+        const uint32_t id = i < n_vis ? records[i].splat_id : kSentinel;
+        const bool ok = id < p.n;   // a splat without tile entries has no record: its slot may hold anything
+        float base[48], Y[16];
+        int terms = 1;
+        if (ok) {
+            const float4* row = p.rows + (size_t)id * 16;
+            const float4 c0 = __ldg(row), c3 = __ldg(row + 3);
+            base[0] = c3.x;
+            base[1] = c3.y;
+            base[2] = c3.z;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) row[k] = __ldg(p.rows + (size_t)id * 16 + k);
-        const float4 c0 = row[0];
-        const float vz = add(add(add(mul(cam.V[2], c0.x), mul(cam.V[6], c0.y)), mul(cam.V[10], c0.z)), cam.V[14]);
-        if (animated) {
-            float4 c3 = row[3];
-            animate_row(p, id, row, c3);
+            for (int q = 0; q < 12; ++q) {
+                const float4 f4 = __ldg(row + 4 + q);
+                const float f[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int slot = 4 * q + e;   // 3k + c
+                    if (slot < 45) base[3 + (slot % 3) * 15 + slot / 3] = f[e];
+                }
+            }
+            const float vz = add(add(add(mul(cam.V[2], c0.x), mul(cam.V[6], c0.y)), mul(cam.V[10], c0.z)), cam.V[14]);
+            const float ddx = sub(c0.x, cam.camw[0]), ddy = sub(c0.y, cam.camw[1]), ddz = sub(c0.z, cam.camw[2]);
+            const float len = __fsqrt_rn(add(add(mul(ddx, ddx), mul(ddy, ddy)), mul(ddz, ddz)));
+            int eff = p.sh_degree;
+            if (p.sh_lod_distance > 0.0f && (-vz) > p.sh_lod_distance) eff = 0;
+            terms = sh_terms(eff);
+            sh_basis(dv(ddx, len), dv(ddy, len), dv(ddz, len), eff, true, Y);
         }
-        const float ddx = sub(c0.x, cam.camw[0]), ddy = sub(c0.y, cam.camw[1]), ddz = sub(c0.z, cam.camw[2]);
-        const float len = __fsqrt_rn(add(add(mul(ddx, ddx), mul(ddy, ddy)), mul(ddz, ddz)));
-        const float x = dv(ddx, len), y = dv(ddy, len), z = dv(ddz, len);
-        int eff = p.sh_degree;
-        if (p.sh_lod_distance > 0.0f && (-vz) > p.sh_lod_distance) eff = 0;
-        float res[3];
-        sh_eval(row, x, y, z, eff, res);
-        colours[i] = make_float4(g_max(add(res[0], 0.5f), 0.0f), g_max(add(res[1], 0.5f), 0.0f),
-                                 g_max(add(res[2], 0.5f), 0.0f), 0.0f);
+        for (int f0 = 0; f0 < frames; f0 += kGroup) {
+            for (int g = 0; g < kGroup; ++g) {
+                float res[3] = {0.0f, 0.0f, 0.0f};
+                if (ok && f0 + g < frames) {
+                    const int fr = first + f0 + g, sa = st.a[fr], sb = st.b[fr];
+                    const float w = st.w[fr], w1 = sub(1.0f, w);
+                    const bool blend = w > 0.0f;   // states 0 and 0 included, as the shader blends
+                    uint4 da[3] = {}, db[3] = {};
+                    if (sa) {
+                        const uint4* d = reinterpret_cast<const uint4*>(p.anim_deltas + ((size_t)(sa - 1) * p.n + id) * 48u);
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) da[q] = __ldg(d + q);
+                    }
+                    if (blend && sb) {
+                        const uint4* d = reinterpret_cast<const uint4*>(p.anim_deltas + ((size_t)(sb - 1) * p.n + id) * 48u);
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) db[q] = __ldg(d + q);
+                    }
+                    // coefficient j of the frame, then its SH term (per channel in the order of sh_eval)
+                    auto eval = [&](auto blended) {
+                        constexpr bool kBlend = decltype(blended)::value;
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) {
+                            const uint32_t wa[4] = {da[q].x ^ 0x80808080u, da[q].y ^ 0x80808080u, da[q].z ^ 0x80808080u,
+                                                    da[q].w ^ 0x80808080u};
+                            const uint32_t wb[4] = {db[q].x ^ 0x80808080u, db[q].y ^ 0x80808080u, db[q].z ^ 0x80808080u,
+                                                    db[q].w ^ 0x80808080u};
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) {
+                                const int j = 16 * q + e;
+                                const float sc = s_scale[j];
+                                float v = base[j];
+                                if (sa) v = add(base[j], mul(int8_of(wa[e >> 2], e & 3), sc));
+                                if (kBlend) {
+                                    float u = base[j];
+                                    if (sb) u = add(base[j], mul(int8_of(wb[e >> 2], e & 3), sc));
+                                    v = add(mul(w1, v), mul(w, u));
+                                }
+                                if (j < 3) res[j] = mul(SH_C0, v);
+                                else if ((j - 3) % 15 + 1 < terms) res[(j - 3) / 15] = add(res[(j - 3) / 15], mul(Y[(j - 3) % 15 + 1], v));
+                            }
+                        }
+                    };
+                    if (blend) eval(std::true_type{});
+                    else eval(std::false_type{});
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) res[c] = g_max(add(res[c], 0.5f), 0.0f);
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c) s_col[t][c * kGroup + g] = res[c];
+            }
+            __syncthreads();
+            float4* dst = reinterpret_cast<float4*>(colours + ((size_t)(f0 / kGroup) * p.n + i0) * kRow);
+            const int quads = (int)min((uint32_t)kRecolourThreads, n_vis - i0) * (kRow / 4);
+            for (int q = t; q < quads; q += kRecolourThreads) {
+                const float* src = &s_col[q / (kRow / 4)][4 * (q % (kRow / 4))];
+                dst[q] = make_float4(src[0], src[1], src[2], src[3]);
+            }
+            __syncthreads();
+        }
     }
 }
 
-int launch_recolour(const CullParams& p, const RasterRecord* records, float4* colours, uint32_t num_sms,
-                    cudaStream_t s) {
-    uint32_t grid = (p.n + 127) / 128;
+int launch_recolour_states(const CullParams& p, const RasterRecord* records, const StateBatch& st, int frames,
+                           float* colours, uint32_t num_sms, cudaStream_t s) {
+    uint32_t grid = (p.n + kRecolourThreads - 1) / kRecolourThreads;
     if (grid > num_sms * 8) grid = num_sms * 8;
-    if (grid == 0) return 0;
-    recolour_kernel<<<grid, 128, 0, s>>>(p, records, colours);
-    return 1;
+    if (grid == 0 || frames <= 0) return 0;
+    int launches = 0;
+    const int g8 = state_groups8(frames), in8 = std::min(frames, 8 * g8);
+    if (g8) {
+        launch_pdl(recolour_states_kernel<8>, dim3(grid), dim3(kRecolourThreads), 0, s, p, records, st, 0, in8, colours);
+        ++launches;
+    }
+    if (state_groups4(frames)) {
+        launch_pdl(recolour_states_kernel<4>, dim3(grid), dim3(kRecolourThreads), 0, s, p, records, st, 8 * g8,
+                   frames - 8 * g8, colours + (size_t)g8 * p.n * 24u);
+        ++launches;
+    }
+    return launches;
 }
 
 // Pass 3, gsanim 0.3 assets only (shaders/cull.glsl:141-148, 354-416): the

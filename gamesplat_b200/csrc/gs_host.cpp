@@ -224,7 +224,7 @@ struct gs_ctx {
     uint32_t* batch_first = nullptr;              // device: prefix sums of tiles (+ the ticket word)
     uint32_t* h_batch_first = nullptr;            // pinned
     uint32_t batch_cap = 0;
-    float4* state_colours = nullptr;              // anim batches: n x states colours
+    float* state_colours = nullptr;               // anim batches: gs::state_colour_floats(n, frames) floats
     size_t state_colours_cap = 0;
     cudaEvent_t batch_event = nullptr;
     cudaEvent_t params_event = nullptr;           // after the last copy out of h_batch_params / h_batch_first
@@ -1893,7 +1893,7 @@ int gs_render_features(gs_ctx* c, const gs_camera* cam, void* features_out) {
 // ---- batches ---------------------------------------------------------------
 namespace {
 
-constexpr uint32_t kMaxBatch = 256;
+constexpr uint32_t kMaxBatch = gs::kMaxBatchFrames;
 
 int ensure_batch(gs_ctx* c, uint32_t count) {
     if (c->slots.size() < count) c->slots.resize(count);
@@ -2160,12 +2160,12 @@ int gs_render_anim_batch(gs_ctx* c, const gs_camera* cam, const int32_t* states_
             return fail(c, GS_ERR_BAD_ARG, "bad appearance state in the batch");
     }
     cudaSetDevice(c->device);
-    if ((rc = ensure_batch(c, count))) return rc;
-    const size_t need = (size_t)count * c->n;
+    if ((rc = ensure_batch(c, 1))) return rc;
+    const size_t need = gs::state_colour_floats(c->n, (int)count);
     if (c->state_colours_cap < need) {
         dfree(c->state_colours);
         c->state_colours_cap = 0;
-        GS_CUDA(c, dalloc(&c->state_colours, need * sizeof(float4)));
+        GS_CUDA(c, dalloc(&c->state_colours, need * sizeof(float)));
         c->state_colours_cap = need;
     }
     nvtxRangePushA("gs_render_anim_batch");
@@ -2185,32 +2185,29 @@ int gs_render_anim_batch(gs_ctx* c, const gs_camera* cam, const int32_t* states_
         nvtxRangePop();
         return rc;
     }
-    // per state: the colours of the frame's records, and the raster parameters
+    // the colours of the frame's records under every frame's states, then all frames' images
+    gs::StateBatch st{};
+    gs::StateOuts images{};
+    for (uint32_t k = 0; k < count; ++k) {
+        st.a[k] = states_a[k];
+        st.b[k] = states_b ? states_b[k] : 0;
+        st.w[k] = weights ? weights[k] : 0.0f;
+        images.out[k] = static_cast<uint16_t*>(outs[k]);
+    }
     FrameSlot& f0 = c->slots[0];
     swap_slot(c, f0);
-    const int sa = c->anim_a, sb = c->anim_b;
-    const float sw = c->anim_w;
-    const gs::RasterParams base = c->h_batch_params[0];
     {
         StageScope sc(c, ST_CULL);
-        for (uint32_t k = 0; k < count; ++k) {
-            c->anim_a = states_a[k];
-            c->anim_b = states_b ? states_b[k] : 0;
-            c->anim_w = weights ? weights[k] : 0.0f;
-            gs::CullParams p = cull_params(c);
-            float4* colours = c->state_colours + (size_t)k * c->n;
-            sc.add(gs::launch_recolour(p, c->records, colours, c->num_sms, c->stream));
-            gs::RasterParams r = base;
-            r.colours = colours;
-            r.out_rgba16f = static_cast<uint16_t*>(outs[k]);
-            c->h_batch_params[k] = r;
-        }
+        sc.add(gs::launch_recolour_states(cull_params(c), c->records, st, (int)count, c->state_colours, c->num_sms,
+                                          c->stream));
     }
-    c->anim_a = sa;
-    c->anim_b = sb;
-    c->anim_w = sw;
+    {
+        StageScope sc(c, ST_RASTER);
+        gs::RasterParams r = c->h_batch_params[0];
+        r.colours = reinterpret_cast<const float4*>(c->state_colours);
+        sc.add(gs::launch_raster_states(r, images, (int)count, c->stream));
+    }
     swap_slot(c, f0);
-    rc = raster_batch(c, count);
     cudaStreamWaitEvent(c->stream, c->fc_event, 0);   // after gs_render's copy of h_fc
     cudaMemcpyAsync(c->h_fc, c->slots[0].fc, sizeof(FrameCounters), cudaMemcpyDeviceToHost, c->stream);
     cudaEventRecord(c->fc_event, c->stream);

@@ -185,7 +185,7 @@ struct RasterParams {
     const uint2* tile_ranges;        // [start, end) per tile
     const uint32_t* tile_order;      // tiles by descending work (CTA b rasterizes tile_order[b])
     const uint32_t* tile_count;      // optional: CTAs b >= *tile_count do nothing (a tile list of the frame)
-    const float4* colours;           // optional: r, g, b per record, replacing the records' colour
+    const float4* colours;           // state batches: per record the colours of kStates frames (StateBatch)
     int width, height, tiles_x, tiles_y;
     int tile_w, tile_h;              // tile shape: 16x16, or 32x8 / 8x32 (alpha mode)
     float bg;
@@ -235,8 +235,25 @@ int launch_cull(const CullParams& p, uint32_t num_sms, cudaStream_t s);
 int launch_gather_heads(const float4* rows, float4* heads, uint32_t n, uint32_t num_sms, cudaStream_t s,
                         uint32_t row_chunks = 16);
 int launch_pack_half_rows(const float4* rows, float4* half_rows, uint32_t n, uint32_t num_sms, cudaStream_t s);
-int launch_recolour(const CullParams& p, const RasterRecord* records, float4* colours, uint32_t num_sms,
-                    cudaStream_t s);
+// State batches (gs_render_anim_batch): frames of one geometry that differ in
+// colours only.  The frames are taken in groups of 8 (the last one of 4 when
+// that holds the rest); a group's colours lie together per record, channel
+// by channel: 3 x group-width floats, group after group, cap records each.
+constexpr int kMaxBatchFrames = 256;
+struct StateBatch {
+    int32_t a[kMaxBatchFrames], b[kMaxBatchFrames];   // appearance states of each frame and
+    float w[kMaxBatchFrames];                         // their blend weight (gs_set_anim_state)
+};
+struct StateOuts {
+    uint16_t* out[kMaxBatchFrames];
+};
+inline int state_groups8(int frames) { return frames / 8 + (frames % 8 > 4 ? 1 : 0); }
+inline int state_groups4(int frames) { return frames % 8 > 0 && frames % 8 <= 4 ? 1 : 0; }
+inline size_t state_colour_floats(size_t cap, int frames) {
+    return cap * (24u * (size_t)state_groups8(frames) + 12u * (size_t)state_groups4(frames));
+}
+int launch_recolour_states(const CullParams& p, const RasterRecord* records, const StateBatch& st, int frames,
+                           float* colours, uint32_t num_sms, cudaStream_t s);
 int launch_sort(const SortParams& p, uint32_t num_sms, cudaStream_t s);
 int launch_bin(const BinParams& p, uint32_t n_cap, uint32_t num_sms, cudaStream_t s);
 int launch_tile_ranges(const SortPlan* tile_plan, const FrameCounters* fc, uint32_t entry_cap, uint2* ranges,
@@ -250,6 +267,8 @@ int launch_raster_stochastic2(const RasterParams& p, cudaStream_t s);
 int launch_raster_batch_alpha(const RasterParams* frames, const uint32_t* first, uint32_t nframes, uint32_t* ticket,
                               uint32_t grid, int tile_w, cudaStream_t s);
 void raster_batch_occupancy(int* blocks_per_sm);
+// the frames of a state batch into outs (p.colours: launch_recolour_states' buffer of p.record_cap records a group)
+int launch_raster_states(const RasterParams& p, const StateOuts& outs, int frames, cudaStream_t s);
 
 int launch_wait_probe(const unsigned long long* status, FrameCounters* fc, uint32_t epoch, int which, uint32_t limit,
                       cudaStream_t s);

@@ -66,11 +66,6 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
-// Byte offset of weight (k = tap * cin + ci, n = co) in the K-major B image.
-__host__ __device__ constexpr int wimage_offset(int k, int n, int cout) {
-    return (k >> 3) * (cout * 16) + (n >> 3) * 128 + (n & 7) * 16 + (k & 7) * 2;
-}
-
 __device__ __forceinline__ uint4 bf16x8_add(uint4 a, uint4 b) {
     uint4 r;
     const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
@@ -497,15 +492,16 @@ __global__ void __launch_bounds__(kThreads) conv_wgrad_kernel(WgradArgs a) {
 // ---------------------------------------------------------------------------
 // Weight packing: FP32 masters [tap][cin][cout] -> the bf16 B-operand image of
 // the forward convolution, or of the transposed convolution that gives the
-// input gradient (cin' = cout, cout' = cin, tap' = 8 - tap).
+// input gradient (cin' = cout, cout' = cin, tap' = 8 - tap).  For the
+// stage-level convolutions; the denoiser packs its layers together
+// (dn::launch_pack_params).
 // ---------------------------------------------------------------------------
-__global__ void pack_weights_kernel(const float* __restrict__ w, int cin, int cout, int transposed, int cut_cout,
+__global__ void pack_weights_kernel(const float* __restrict__ w, int cin, int cout, int transposed,
                                     uint8_t* __restrict__ image) {
     const int total = 9 * cin * cout;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int co = i % cout, ci = (i / cout) % cin, tap = i / (cin * cout);
-        // cut_cout: the output channel whose gradient stops at this layer (zero in the transposed image)
-        const float v = (transposed && co == cut_cout) ? 0.0f : w[i];
+        const float v = w[i];
         int k, nn, cdim;
         if (!transposed) {
             k = tap * cin + ci;
@@ -574,10 +570,9 @@ int launch_wgrad(int cin, int cout, int load_mode, const WgradArgs& a, int grid,
     return -1;
 }
 
-int launch_pack_weights(const float* w, int cin, int cout, int transposed, uint8_t* image, cudaStream_t s,
-                        int cut_cout) {
+int launch_pack_weights(const float* w, int cin, int cout, int transposed, uint8_t* image, cudaStream_t s) {
     const int total = 9 * cin * cout;
-    pack_weights_kernel<<<(total + 255) / 256, 256, 0, s>>>(w, cin, cout, transposed, cut_cout, image);
+    pack_weights_kernel<<<(total + 255) / 256, 256, 0, s>>>(w, cin, cout, transposed, image);
     return 1;
 }
 

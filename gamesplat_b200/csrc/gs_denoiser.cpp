@@ -71,8 +71,7 @@ struct gs_denoiser {
     float* out = nullptr;
     // training
     size_t tcap = 0;
-    float4* pred = nullptr;
-    float *mom = nullptr, *tmp = nullptr, *bmom = nullptr, *part = nullptr, *bpart = nullptr;
+    float* part = nullptr;      // SSIM partials, 9 planes
     bf16 *dout = nullptr, *dz4 = nullptr, *du = nullptr, *dz3 = nullptr, *dz2 = nullptr, *dp1 = nullptr,
          *dz1 = nullptr;
     int last_n = 0, last_h = 0, last_w = 0;
@@ -96,12 +95,7 @@ static void release_acts(gs_denoiser* d) {
 }
 
 static void release_train(gs_denoiser* d) {
-    dfree(d->pred);
-    dfree(d->mom);
-    dfree(d->tmp);
-    dfree(d->bmom);
     dfree(d->part);
-    dfree(d->bpart);
     dfree(d->dout);
     dfree(d->dz4);
     dfree(d->du);
@@ -129,9 +123,7 @@ static int ensure_train(gs_denoiser* d, size_t pix) {
     if (pix <= d->tcap) return GS_OK;
     release_train(d);
     const size_t half = pix / 4 + 1;
-    if (dalloc(&d->pred, pix) || dalloc(&d->mom, pix * 15) || dalloc(&d->tmp, pix * 15) ||
-        dalloc(&d->bmom, pix * 15) || dalloc(&d->part, pix * 9) || dalloc(&d->bpart, pix * 9) ||
-        dalloc(&d->dout, pix * kOutC) || dalloc(&d->dz4, pix * kHidC) || dalloc(&d->du, pix * kHidC) ||
+    if (dalloc(&d->part, pix * 9) || dalloc(&d->dout, pix * kOutC) || dalloc(&d->dz4, pix * kHidC) || dalloc(&d->du, pix * kHidC) ||
         dalloc(&d->dz3, half * kHidC) || dalloc(&d->dz2, half * kHidC) || dalloc(&d->dp1, half * kHidC) ||
         dalloc(&d->dz1, pix * kHidC)) {
         release_train(d);
@@ -141,14 +133,19 @@ static int ensure_train(gs_denoiser* d, size_t pix) {
     return GS_OK;
 }
 
-static void pack_images(gs_denoiser* d, cudaStream_t s) {
-    for (int l = 0; l < gs::dn::kLayers; ++l) {
-        conv::launch_pack_weights(d->params + w_offset(l), kNet[l].cin, kNet[l].cout, 0, d->wimg[l], s);
+static ParamImages param_images(const gs_denoiser* d) {
+    ParamImages im{};
+    im.layers = kLayers;
+    for (int l = 0; l < kLayers; ++l)
         // the error estimate (channel 4 of the last layer) trains the last layer only: its gradient
         // does not reach the trunk, whose features would otherwise chase their own growing error
-        conv::launch_pack_weights(d->params + w_offset(l), kNet[l].cin, kNet[l].cout, 1, d->wimg_t[l], s,
-                                  l == gs::dn::kLayers - 1 ? kErrChannel : -1);
-    }
+        im.layer[l] = {(int)w_offset(l), kNet[l].cin, kNet[l].cout, l == kLayers - 1 ? kErrChannel : -1, d->wimg[l],
+                       d->wimg_t[l]};
+    return im;
+}
+
+static void pack_images(gs_denoiser* d, cudaStream_t s) {
+    launch_pack_params(param_images(d), d->params, (int)param_count(), s);
     d->images_valid = true;
 }
 
@@ -287,18 +284,13 @@ int loss(gs_denoiser* d, const bf16* x, const float* out, const float4* target, 
     if (rc) return rc;
     cudaMemsetAsync(d->acc, 0, 4 * sizeof(float), d->stream);
     const bool ssim = ssim_weight > 0.0f && h > 10 && w > 10;
-    launch_head_moments(out, x, target, (int)pix, d->pred, ssim ? d->mom : nullptr, d->stream);
     float ssim_scale = 0.0f;
     if (ssim) {
-        launch_blur(d->mom, n, h, w, 15, 0, d->tmp, d->stream);
-        launch_blur(d->tmp, n, h, w, 15, 1, d->bmom, d->stream);
-        launch_ssim_partials(d->bmom, n, h, w, d->part, d->acc, d->stream);
-        launch_blur(d->part, n, h, w, 9, 0, d->tmp, d->stream);
-        launch_blur(d->tmp, n, h, w, 9, 1, d->bpart, d->stream);
+        launch_ssim_partials(out, x, target, n, h, w, d->part, d->acc, d->stream);
         ssim_scale = ssim_weight / (3.0f * (float)n * (float)(h - 10) * (float)(w - 10));
     }
-    launch_loss_grad(out, d->pred, target, ssim ? d->bpart : nullptr, (int)pix, 1.0f / (4.0f * (float)pix),
-                     ssim_scale, err_weight / (float)pix, dout, d->acc, d->stream);
+    launch_loss_grad(out, x, target, ssim ? d->part : nullptr, n, h, w, 1.0f / (4.0f * (float)pix), ssim_scale,
+                     err_weight / (float)pix, dout, d->acc, d->stream);
     return GS_OK;
 }
 
@@ -506,9 +498,9 @@ int gs_denoiser_adam(gs_denoiser* d, float lr) {
     d->adam_t += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float bc1 = 1.0f - (float)std::pow(b1, d->adam_t), bc2 = 1.0f - (float)std::pow(b2, d->adam_t);
-    launch_adam(d->params, d->grads, d->adam_m, d->adam_v, (int)param_count(), lr, b1, b2, 1e-8f, bc1, bc2,
-                d->stream);
-    pack_images(d, d->stream);
+    launch_adam(param_images(d), d->params, d->grads, d->adam_m, d->adam_v, (int)param_count(), lr, b1, b2, 1e-8f, bc1,
+                bc2, d->stream);
+    d->images_valid = true;
     return launched(d, GS_OK);
 }
 

@@ -17,13 +17,7 @@
 // (thread t = TMEM lane t = pixel t) for the epilogue (bias, ReLU, ReLU
 // mask, bf16 / f32 store).
 //
-// conv_wgrad_kernel: dW[tap, cin][cout] = sum over pixels of
-// X[p + tap][cin] * dY[p][cout], a GEMM with M = 9 * Cin (tiles of 128 rows),
-// N = Cout, K = pixels, both operands MN-major (channels contiguous per
-// pixel, as NHWC stores them).  Each CTA accumulates its share of 64-pixel
-// row segments in TMEM and adds the result to dW with FP32 atomics.  The
-// first padding row of the M range holds the constant 1, so its row of dW is
-// the bias gradient (sum over pixels of dY).
+// conv_wgrad_kernel: the weight gradient, K = pixels; see there.
 //
 // Every wait is bounded; a wait that runs out sets err[0] and the kernel
 // frees its TMEM and returns.
@@ -378,109 +372,209 @@ __global__ void __launch_bounds__(kThreads) conv_fwd_kernel(ConvArgs a) {
 // ---------------------------------------------------------------------------
 // Weight gradient.
 // ---------------------------------------------------------------------------
-constexpr int kKBlock = 64;                       // pixels per K block
-constexpr int kGroupBytes = kKBlock * 16 + 16;    // one 8-channel group of a K block (+16: bank spread)
-
-__host__ __device__ constexpr int wgrad_mtiles(int cin) { return (9 * cin + 1 + 127) / 128; }
-__host__ __device__ constexpr int tmem_cols_for(int c) { return c <= 32 ? 32 : c <= 64 ? 64 : c <= 128 ? 128 : 256; }
+// dW[ky][kx][ci][co] = sum over pixels of X[p + (ky - 1, kx - 1)][ci] dY[p][co]:
+// K = pixels, both operands MN-major (8 channels of a pixel are 16 bytes, as
+// NHWC stores them).  A CTA takes strips of 128 pixels by up to 4 rows; the
+// strip's X rows with their halo sit in shared memory once, row slot after row
+// slot, so that the 16 row groups of one M = 128 operand, all a column of
+// 8 channels apart, are the rows y - 1, y, y + 1 (and what lies below them:
+// rows of D past 3 x Cin, never read) and tap kx is the same operand started
+// kx pixels further.  Per output row: 3 taps x 8 K-steps MMAs into 3
+// accumulators.  Two stages: the strip after the next is copied (cp.async)
+// while one is multiplied, and MMAs of consecutive strips queue without a
+// wait between them.  The bias gradient is summed from the staged dY by the
+// threads while the MMAs run.  Bound by the shared-memory reads of the MMAs
+// and the L2 reads of the strips (1.5 reads of X for 4 rows); 8 x 256 x 256
+// pixels, 32 -> 32 channels: 262 us (load mode 1) when every tap was gathered
+// from global memory and nothing overlapped; figures now at launch_wgrad.
+constexpr int kWgThreads = 256;
+constexpr int kWgPx = 128;    // pixels of a strip
+constexpr int kWgRows = 4;    // output rows of a strip, at most
+// A channel group of a dY row: 2 or 4 of them are copied by a quarter warp (as col_bytes)
+__host__ __device__ constexpr int wg_dcol(int cout) { return kWgPx * 16 + (cout / 8 == 2 ? 64 : 32); }
+// row slots of a stage: the rows of a strip, its halo, and what an M = 128 operand of the last row spans
+__host__ __device__ constexpr int wg_slots(int cin) { return kWgRows - 1 + 128 / cin; }
+__host__ __device__ constexpr int wg_x_bytes(int cin) { return wg_slots(cin) * (cin / 8) * col_bytes(cin); }
+__host__ __device__ constexpr int wg_stage_bytes(int cin, int cout) {
+    return wg_x_bytes(cin) + kWgRows * (cout / 8) * wg_dcol(cout);
+}
 
 template <int kCin, int kCout, int kLoad>
-__global__ void __launch_bounds__(kThreads) conv_wgrad_kernel(WgradArgs a) {
-    constexpr int kMT = wgrad_mtiles(kCin);
-    constexpr int kA = 16 * kGroupBytes;           // one M tile: 16 groups of 8 rows
-    constexpr int kCols = tmem_cols_for(kMT * kCout);
+__global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(WgradArgs a, int rows) {
+    constexpr int kG = kCin / 8, kGo = kCout / 8;
+    constexpr int kCol = col_bytes(kCin), kSlot = kG * kCol, kDcol = wg_dcol(kCout), kDrow = kGo * kDcol;
+    constexpr int kStage = wg_stage_bytes(kCin, kCout), kX = wg_x_bytes(kCin);
     constexpr uint32_t kIdesc = umma::idesc_bf16(128, kCout, 1, 1);
+    constexpr int kCols = 128;   // TMEM: 3 accumulators of kCout columns
     extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* s_a = smem;
-    uint8_t* s_b = smem + kMT * kA;
-    __shared__ __align__(8) uint64_t s_bar;
+    __shared__ __align__(8) uint64_t s_bar[2];   // MMA completion, one per stage
     __shared__ uint32_t s_taddr;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    __shared__ float s_db[kWgThreads / 32][kCout];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     if (tid == 0) {
-        mbar_init(&s_bar, 1);
+        mbar_init(&s_bar[0], 1);
+        mbar_init(&s_bar[1], 1);
         mbar_fence_init();
     }
     if (warp == 0) umma::tmem_alloc(&s_taddr, kCols);
+    // the slots no strip fills are operands too (their products are never read)
+    for (int i = tid; i < 2 * kStage / 16; i += kWgThreads) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
-    const uint32_t taddr = s_taddr;
-    const uint32_t a_base = smem_u32(s_a), b_base = smem_u32(s_b);
-    const int blocks_x = (a.w + kKBlock - 1) / kKBlock;
-    const int total = a.n * a.h * blocks_x;
-    uint32_t phase = 0;
-    bool failed = false, any = false;
+    const uint32_t taddr = s_taddr, base = smem_u32(smem);
+    const int strips_x = (a.w + kWgPx - 1) / kWgPx, bands = (a.h + rows - 1) / rows;
+    const int total = a.n * bands * strips_x;
     const ConvArgs ca{a.x, a.xh, a.n, a.h, a.w};
 
-    for (int blk = blockIdx.x; blk < total && !failed; blk += gridDim.x) {
-        const int xb = blk % blocks_x, row = blk / blocks_x;
-        const int y = row % a.h, n = row / a.h, x0 = xb * kKBlock;
-        // A: rows m = tap * cin + ci (8-row groups never straddle a tap), K = pixels
-        for (int q = tid; q < kMT * 16 * kKBlock; q += kThreads) {
-            const int k = q % kKBlock, grp = q / kKBlock;      // grp = tile * 16 + group
-            const int m0 = grp * 8;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (m0 < 9 * kCin) {
-                const int tap = m0 / kCin, cg = (m0 % kCin) >> 3;
-                v = load_granule<kCin, kLoad>(ca, n, y + tap / 3 - 1, x0 + k + tap % 3 - 1, cg);
-            } else if (m0 == 9 * kCin && x0 + k < a.w) {
-                v.x = 0x3F80u;   // bf16 1.0 in row m0 (the bias row), zero in rows m0+1..m0+7
-            }
-            *reinterpret_cast<uint4*>(s_a + (grp >> 4) * kA + (grp & 15) * kGroupBytes + k * 16) = v;
-        }
-        // B: dY, rows = output channels, K = pixels
-        for (int q = tid; q < (kCout / 8) * kKBlock; q += kThreads) {
-            const int k = q % kKBlock, g = q / kKBlock;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (x0 + k < a.w) {
-                const size_t pix = ((size_t)n * a.h + y) * a.w + x0 + k;
-                v = __ldg(reinterpret_cast<const uint4*>(a.dy + pix * kCout) + g);
-            }
-            *reinterpret_cast<uint4*>(s_b + g * kGroupBytes + k * 16) = v;
-        }
-        umma::fence_smem_to_async();
-        __syncthreads();
-        if (tid == 0) {
-            umma::fence_after_sync();
-#pragma unroll
-            for (int t = 0; t < kMT; ++t) {
-#pragma unroll
-                for (int kk = 0; kk < kKBlock / 16; ++kk) {
-                    const uint64_t ad = umma::smem_desc(a_base + (uint32_t)(t * kA + kk * 256), 128u,
-                                                        (uint32_t)kGroupBytes);
-                    const uint64_t bd = umma::smem_desc(b_base + (uint32_t)(kk * 256), 128u, (uint32_t)kGroupBytes);
-                    umma::mma_bf16(taddr + (uint32_t)(t * kCout), ad, bd, kIdesc, (any || kk > 0) ? 1u : 0u);
+    struct Strip {
+        int n, y0, x0, rows, px;   // px: pixels in whole K-steps
+    };
+    auto strip_at = [&](int item) {
+        Strip s;
+        s.x0 = (item % strips_x) * kWgPx;
+        const int q = item / strips_x;
+        s.n = q / bands;
+        s.y0 = (q % bands) * rows;
+        s.rows = min(rows, a.h - s.y0);
+        s.px = (min(kWgPx, a.w - s.x0) + 15) & ~15;
+        return s;
+    };
+    // X rows y0 - 1 .. y0 + rows (zero outside the image) into slots 0 ..., dY rows behind them
+    auto load = [&](int stage, int item) {
+        const Strip s = strip_at(item);
+        uint8_t* xs = smem + stage * kStage;
+        uint8_t* ds = xs + kX;
+        const int row_q = (s.px + 2) * kG;
+        for (int r = 0; r < s.rows + 2; ++r) {
+            const int y = s.y0 - 1 + r;
+            if (kLoad == 0) {
+                const bool row_in = y >= 0 && y < a.h;
+                const __nv_bfloat16* rowp = a.x + ((size_t)s.n * a.h + (row_in ? y : 0)) * a.w * kCin;
+                for (int q = tid; q < row_q; q += kWgThreads) {
+                    const int hp = q / kG, g = q % kG, x = s.x0 - 1 + hp;
+                    const bool in = row_in && x >= 0 && x < a.w;
+                    cp_async16(xs + r * kSlot + g * kCol + hp * 16, in ? rowp + (size_t)x * kCin + g * 8 : a.x,
+                               in ? 16u : 0u);
+                }
+            } else {
+                for (int q = tid; q < row_q; q += kWgThreads) {
+                    const int hp = q / kG, g = q % kG;
+                    *reinterpret_cast<uint4*>(xs + r * kSlot + g * kCol + hp * 16) =
+                        load_granule<kCin, kLoad>(ca, s.n, y, s.x0 - 1 + hp, g);
                 }
             }
-            umma::commit(&s_bar);
+        }
+        for (int r = 0; r < s.rows; ++r) {
+            const __nv_bfloat16* rowp = a.dy + ((size_t)s.n * a.h + s.y0 + r) * a.w * kCout;
+            for (int q = tid; q < s.px * kGo; q += kWgThreads) {
+                const int k = q / kGo, g = q % kGo, x = s.x0 + k;
+                const bool in = x < a.w;
+                cp_async16(ds + r * kDrow + g * kDcol + k * 16, in ? rowp + (size_t)x * kCout + g * 8 : a.dy, in ? 16u : 0u);
+            }
+        }
+        cp_async_commit();
+    };
+
+    uint32_t phase[2] = {0u, 0u};
+    bool failed = false, any = false;
+    float db[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // of channel group tid % kGo
+    int stage = 0;
+    if ((int)blockIdx.x < total) load(0, blockIdx.x);
+    for (int item = blockIdx.x; item < total; item += gridDim.x, stage ^= 1) {
+        asm volatile("cp.async.wait_all;" ::: "memory");   // this strip, copied while the last one was multiplied
+        umma::fence_smem_to_async();
+        if (__syncthreads_or(failed)) {
+            failed = true;
+            break;
+        }
+        const Strip s = strip_at(item);
+        if (tid == 0) {
+            umma::fence_after_sync();
+            const uint32_t xa = base + (uint32_t)(stage * kStage), da = xa + (uint32_t)kX;
+            for (int r = 0; r < s.rows; ++r)
+                for (int kk = 0; kk < s.px / 16; ++kk) {
+                    const uint64_t bd = umma::smem_desc(da + (uint32_t)(r * kDrow + kk * 256), 128u, (uint32_t)kDcol);
+#pragma unroll
+                    for (int kx = 0; kx < 3; ++kx) {
+                        const uint64_t ad =
+                            umma::smem_desc(xa + (uint32_t)(r * kSlot + kx * 16 + kk * 256), 128u, (uint32_t)kCol);
+                        umma::mma_bf16(taddr + (uint32_t)(kx * kCout), ad, bd, kIdesc, (any || r + kk > 0) ? 1u : 0u);
+                    }
+                }
+            umma::commit(&s_bar[stage]);
+        }
+        if (a.db) {   // pixels past the row are zero
+            const uint8_t* ds = smem + stage * kStage + kX + (tid % kGo) * kDcol;
+            for (int r = 0; r < s.rows; ++r)
+                for (int k = tid / kGo; k < s.px; k += kWgThreads / kGo) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(ds + r * kDrow + k * 16);
+                    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 f = __bfloat1622float2(p[e]);
+                        db[2 * e] += f.x;
+                        db[2 * e + 1] += f.y;
+                    }
+                }
+        }
+        const int next = item + (int)gridDim.x;
+        if (next < total) {
+            // the other stage: its MMAs (the previous strip's) read it to the end, and every
+            // thread is past its sum over it (the barrier above)
+            if (any) {
+                if (!mbar_wait_bounded(&s_bar[stage ^ 1], phase[stage ^ 1], kWaitLimit)) failed = true;
+                phase[stage ^ 1] ^= 1u;
+            }
+            load(stage ^ 1, next);
         }
         any = true;
-        if (!mbar_wait_bounded(&s_bar, phase, kWaitLimit)) failed = true;
-        phase ^= 1u;
-        umma::fence_after_sync();
-        if (__syncthreads_or(failed)) failed = true;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (any && !failed) {   // the last strip's MMAs complete after all earlier ones
+        if (!mbar_wait_bounded(&s_bar[stage ^ 1], phase[stage ^ 1], kWaitLimit)) failed = true;
+    }
+    if (__syncthreads_or(failed)) failed = true;
+    umma::fence_after_sync();
     if (any && !failed) {
-        // warp w holds rows 32w..32w+31 of every M tile
-        const int r = warp * 32 + (tid & 31);
+        // D rows m = ky * kCin + ci < 3 kCin of tap column kx; warps 0..3 read taps 0 and 1, warps 4..7 tap 2
+        const int m = (warp & 3) * 32 + lane;
+        const bool vec = (reinterpret_cast<uintptr_t>(a.dw) & 15u) == 0u;
+        if ((warp & 3) * 32 < 3 * kCin) {
+            for (int kx = warp < 4 ? 0 : 2; kx < (warp < 4 ? 2 : 3); ++kx) {
+                float v[32];
+                const uint32_t at = taddr + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(kx * kCout);
+                if (kCout == 32) umma::tmem_ld32(at, *reinterpret_cast<float(*)[32]>(v));
+                else umma::tmem_ld16(at, *reinterpret_cast<float(*)[16]>(v));
+                if (m < 3 * kCin) {
+                    float* dst = a.dw + ((size_t)((m / kCin) * 3 + kx) * kCin + m % kCin) * kCout;
+                    if (vec) {
 #pragma unroll
-        for (int t = 0; t < kMT; ++t) {
-            float v[32];
-            if (kCout == 32)
-                umma::tmem_ld32(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(t * kCout),
-                                *reinterpret_cast<float(*)[32]>(v));
-            else
-                umma::tmem_ld16(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(t * kCout),
-                                *reinterpret_cast<float(*)[16]>(v));
-            const int m = t * 128 + r;
-            if (m < 9 * kCin) {
+                        for (int c = 0; c < kCout / 4; ++c)
+                            atomicAdd(reinterpret_cast<float4*>(dst) + c,
+                                      make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]));
+                    } else {
 #pragma unroll
-                for (int c = 0; c < kCout; ++c) atomicAdd(a.dw + (size_t)m * kCout + c, v[c]);
-            } else if (m == 9 * kCin && a.db) {
-#pragma unroll
-                for (int c = 0; c < kCout; ++c) atomicAdd(a.db + c, v[c]);
+                        for (int c = 0; c < kCout; ++c) atomicAdd(dst + c, v[c]);
+                    }
+                }
             }
+        }
+    }
+    if (a.db) {
+        // lanes of one channel group, then the warps
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+#pragma unroll
+            for (int off = 16; off >= kGo; off >>= 1) db[e] += __shfl_xor_sync(0xffffffffu, db[e], off);
+            if (lane < kGo) s_db[warp][lane * 8 + e] = db[e];
+        }
+        __syncthreads();
+        if (tid < kCout && any && !failed) {
+            float sum = 0.0f;
+            for (int q = 0; q < kWgThreads / 32; ++q) sum += s_db[q][tid];
+            atomicAdd(a.db + tid, sum);
         }
     }
     if (failed && tid == 0) atomicOr(a.err, 1u);
@@ -532,17 +626,21 @@ static int launch_fwd_t(const ConvArgs& a, cudaStream_t s) {
 }
 
 template <int kCin, int kCout, int kLoad>
-static int launch_wgrad_t(const WgradArgs& a, int grid, cudaStream_t s) {
-    // + 2 groups: every address a descriptor can name, with either stride
-    // reading as either, stays inside the allocation
-    const size_t smem = (size_t)wgrad_mtiles(kCin) * 16 * kGroupBytes + (size_t)(kCout / 8 + 2) * kGroupBytes;
+static int launch_wgrad_t(const WgradArgs& a, int max_ctas, cudaStream_t s) {
+    // Rows of a strip: 4 (1.5 reads of X), fewer where that leaves less than
+    // two strips an SM: a 64 x 64 image of 8 has 128 strips of 4 rows.
+    const long strips = (long)a.n * ((a.w + kWgPx - 1) / kWgPx);
+    int rows = kWgRows;
+    while (rows > 1 && strips * ((a.h + rows - 1) / rows) < 2L * max_ctas) rows >>= 1;
+    const long total = strips * ((a.h + rows - 1) / rows);
+    const size_t smem = 2 * (size_t)wg_stage_bytes(kCin, kCout);
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(conv_wgrad_kernel<kCin, kCout, kLoad>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
         attr = true;
     }
-    conv_wgrad_kernel<kCin, kCout, kLoad><<<grid, kThreads, smem, s>>>(a);
+    conv_wgrad_kernel<kCin, kCout, kLoad><<<(unsigned)(total < max_ctas ? total : max_ctas), kWgThreads, smem, s>>>(a, rows);
     return 1;
 }
 
@@ -558,14 +656,14 @@ int launch_fwd(int cin, int cout, int load_mode, const ConvArgs& a, cudaStream_t
     return -1;
 }
 
-int launch_wgrad(int cin, int cout, int load_mode, const WgradArgs& a, int grid, cudaStream_t s) {
+int launch_wgrad(int cin, int cout, int load_mode, const WgradArgs& a, int max_ctas, cudaStream_t s) {
     if (a.n <= 0 || a.h <= 0 || a.w <= 0) return 0;
     if (load_mode == 0) {
-        if (cin == 16 && cout == 32) return launch_wgrad_t<16, 32, 0>(a, grid, s);
-        if (cin == 32 && cout == 32) return launch_wgrad_t<32, 32, 0>(a, grid, s);
-        if (cin == 32 && cout == 16) return launch_wgrad_t<32, 16, 0>(a, grid, s);
+        if (cin == 16 && cout == 32) return launch_wgrad_t<16, 32, 0>(a, max_ctas, s);
+        if (cin == 32 && cout == 32) return launch_wgrad_t<32, 32, 0>(a, max_ctas, s);
+        if (cin == 32 && cout == 16) return launch_wgrad_t<32, 16, 0>(a, max_ctas, s);
     } else {
-        if (cin == 32 && cout == 32) return launch_wgrad_t<32, 32, 1>(a, grid, s);
+        if (cin == 32 && cout == 32) return launch_wgrad_t<32, 32, 1>(a, max_ctas, s);
     }
     return -1;
 }

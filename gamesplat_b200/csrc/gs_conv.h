@@ -54,7 +54,8 @@ struct WgradArgs {
 // Supported (cin, cout, load mode): (16, 32, 0), (32, 32, 0), (32, 16, 0), (32, 32, 1).
 // Return the number of kernels launched, or -1 for an unsupported shape.
 int launch_fwd(int cin, int cout, int load_mode, const ConvArgs& a, cudaStream_t s);
-int launch_wgrad(int cin, int cout, int load_mode, const WgradArgs& a, int grid, cudaStream_t s);
+// max_ctas: the SMs of the device (one persistent CTA each)
+int launch_wgrad(int cin, int cout, int load_mode, const WgradArgs& a, int max_ctas, cudaStream_t s);
 // transposed: the image of the layer's input gradient
 int launch_pack_weights(const float* w, int cin, int cout, int transposed, uint8_t* image, cudaStream_t s);
 // Byte offset of weight (k = tap * cin + ci, n = co) in the K-major B image.

@@ -193,9 +193,7 @@ static int conv_wgrad(gs_denoiser* d, int l, const bf16* x, const bf16* xh, int 
     a.dw = d->grads + w_offset(l);
     a.db = d->grads + b_offset(l);
     a.err = d->err;
-    const long blocks = (long)n * h * ((w + 63) / 64);
-    const int grid = (int)std::max(1L, std::min<long>(blocks, (long)d->num_sms * 2));
-    return conv::launch_wgrad(L.cin, L.cout, L.load, a, grid, d->stream) < 0 ? GS_ERR_BAD_ARG : GS_OK;
+    return conv::launch_wgrad(L.cin, L.cout, L.load, a, (int)d->num_sms, d->stream) < 0 ? GS_ERR_BAD_ARG : GS_OK;
 }
 
 int forward(gs_denoiser* d, const bf16* x, int n, int h, int w, cudaStream_t s) {
@@ -567,7 +565,10 @@ int gs_conv3x3_wgrad_bf16(const void* x, const void* x_half, int n, int h, int w
     a.dw = dw;
     a.db = db;
     a.err = err;
-    if (gs::conv::launch_wgrad(cin, cout, x_half ? 1 : 0, a, 296, static_cast<cudaStream_t>(stream)) < 0)
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (gs::conv::launch_wgrad(cin, cout, x_half ? 1 : 0, a, sms > 0 ? sms : 148, static_cast<cudaStream_t>(stream)) < 0)
         return GS_ERR_BAD_ARG;
     return cudaGetLastError() == cudaSuccess ? GS_OK : GS_ERR_CUDA;
 }

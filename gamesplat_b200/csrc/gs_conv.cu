@@ -7,15 +7,15 @@
 //
 // conv_fwd_kernel (also the input gradient, with the transposed weights):
 // implicit GEMM with M = 128 output pixels of one image row, N = Cout,
-// K = 9 taps x Cin.  A CTA walks a column strip of 128 pixels down a run of
-// rows; three input rows (the row above, the row, the row below, 130 pixels
-// with the halo) sit in shared memory in the K-major core-matrix layout,
-// rows of 16 bytes one pixel apart, so the A operand of tap (ky, kx) is the
-// same buffer started kx pixels (kx * 16 bytes) further: no im2col copy.
-// Per output row the CTA loads one new input row, one thread issues
-// 9 * Cin / 16 MMAs into a TMEM accumulator, and the four warps read it back
-// (thread t = TMEM lane t = pixel t) for the epilogue (bias, ReLU, ReLU
-// mask, bf16 / f32 store).
+// K = 9 taps x Cin.  A persistent CTA walks column strips of 128 pixels down
+// its share of the rows; input rows (130 pixels with the halo) pass through a
+// ring of shared-memory slots in the K-major core-matrix layout, rows of
+// 16 bytes one pixel apart, so the A operand of tap (ky, kx) is the slot of row
+// y - 1 + ky started kx pixels (kx * 16 bytes) further: no im2col copy.  The
+// warps have fixed roles that meet only at mbarriers: 8 load rows, one thread
+// issues the 9 * Cin / 16 MMAs of a row into one of 4 TMEM accumulators, and 4
+// read accumulators back (thread t = TMEM lane t = pixel t) for the epilogue
+// (bias, ReLU, ReLU mask, bf16 / f32 store).
 //
 // conv_wgrad_kernel: the weight gradient, K = pixels; see there.
 //
@@ -24,12 +24,12 @@
 #include <cuda_bf16.h>
 
 #include "gs_conv.h"
+#include "gs_internal.h"
 #include "gs_umma.cuh"
 
 namespace gs {
 namespace conv {
 
-constexpr int kThreads = 128;
 constexpr int kHaloRows = 136;                  // 130 used (pixels x0-1 .. x0+128)
 // One 8-channel column of a halo row (kHaloRows pixels of 16 bytes) plus
 // padding.  Consecutive threads copy the kG columns of a pixel, then the next
@@ -42,14 +42,16 @@ constexpr uint32_t kWaitLimit = 1u << 22;
 
 __host__ __device__ constexpr int wimage_bytes(int cin, int cout) { return 9 * cin * cout * 2; }
 
-constexpr int kSlots = 4;   // halo rows resident: the three a row needs and the one being loaded
+// Roles of the forward kernel's warps (an epilogue warp's number is its TMEM lane quadrant).
+constexpr int kEpiWarps = 4, kLoadWarps = 8, kMmaWarp = kEpiWarps + kLoadWarps;
+constexpr int kFwdThreads = (kMmaWarp + 1) * 32;
+constexpr int kLoaders = kLoadWarps * 16;   // threads of a load group: the two groups take rows in turn
+constexpr int kSlots = 8;                   // halo rows in the ring
+constexpr int kAccs = 4;                    // TMEM accumulators of 32 columns
 
-constexpr int kHalfPix = 66;   // half-resolution pixels under a 130-pixel halo row
-
-// Dynamic shared memory of the forward kernel: the halo rows, the weight
-// image, and (load mode 1) the half-resolution rows staged beside them.
-__host__ __device__ constexpr int fwd_smem_bytes(int cin, int cout, int load = 0) {
-    return kSlots * (cin / 8) * col_bytes(cin) + wimage_bytes(cin, cout) + (load ? kSlots * kHalfPix * cin * 2 : 0);
+// Dynamic shared memory of the forward kernel: the halo rows and the weight image.
+__host__ __device__ constexpr int fwd_smem_bytes(int cin, int cout) {
+    return kSlots * (cin / 8) * col_bytes(cin) + wimage_bytes(cin, cout);
 }
 
 // 16-byte asynchronous global -> shared copy (zero-filled when src_bytes is 0).
@@ -59,6 +61,32 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t 
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Wait for phase `phase` of a barrier, suspended for up to a microsecond between tests; false after a second or so.
+__device__ __forceinline__ bool mbar_wait_suspend(uint64_t* bar, uint32_t phase) {
+    for (uint32_t i = 0; i < (1u << 20); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(phase), "r"(1000u)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// 32 bytes to global memory (32-byte aligned).
+__device__ __forceinline__ void st_global32(void* p, const uint4& a, const uint4& b) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z),
+                 "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+}
 
 __device__ __forceinline__ uint4 bf16x8_add(uint4 a, uint4 b) {
     uint4 r;
@@ -87,8 +115,43 @@ __device__ __forceinline__ uint4 load_granule(const ConvArgs& a, int n, int y, i
     return bf16x8_add(v, __ldg(reinterpret_cast<const uint4*>(a.xh + hp * kCin) + g));
 }
 
+// A run of rows [y0, y1) of one strip; a CTA's share of the units is a sequence of them.
+struct ConvRun {
+    int n, x0, y0, y1;
+};
+
+// The runs of a CTA: units (unit_rows rows of a strip, bands shifted up by
+// row_offset) are numbered strip by strip, and CTA b takes an equal share.
+struct ConvRuns {
+    int strips_x, bands, u, u1, unit_rows, row_offset, h;
+    __device__ __forceinline__ ConvRuns(const ConvArgs& a)
+        : strips_x((a.w + 127) / 128), bands((a.h + a.row_offset + a.unit_rows - 1) / a.unit_rows),
+          unit_rows(a.unit_rows), row_offset(a.row_offset), h(a.h) {
+        const long long total = (long long)a.n * strips_x * bands;
+        u = (int)(total * blockIdx.x / gridDim.x);
+        u1 = (int)(total * (blockIdx.x + 1) / gridDim.x);
+    }
+    __device__ __forceinline__ bool next(ConvRun& r) {
+        if (u >= u1) return false;
+        const int strip = u / bands, b0 = u - strip * bands;
+        const int ue = min(u1, (strip + 1) * bands);
+        r.n = strip / strips_x;
+        r.x0 = (strip % strips_x) * 128;
+        r.y0 = max(0, b0 * unit_rows - row_offset);
+        r.y1 = min(h, (ue - strip * bands) * unit_rows - row_offset);
+        u = ue;
+        return true;
+    }
+};
+
+// Bound by HBM: every input row of a strip is read once (and 2 more at each
+// end of a run), every output written once in 32-byte sectors.  Before, a CTA
+// of 128 threads did copy, MMAs and epilogue of a row in turn, at ~6 us a row
+// (four CTAs an SM) for 16 KB moved; with the roles apart four rows are in flight
+// per CTA (two CTAs an SM) and the MMAs of a row overlap the epilogue of the
+// ones before.  Times before and after at launch_fwd.
 template <int kCin, int kCout, int kLoad>
-__global__ void __launch_bounds__(kThreads) conv_fwd_kernel(ConvArgs a) {
+__global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
     static_assert(kCin % 16 == 0 && (kCout == 16 || kCout == 32), "channel counts");
     constexpr int kG = kCin / 8;                         // 16-byte columns per pixel
     constexpr int kColBytes = col_bytes(kCin);
@@ -96,277 +159,293 @@ __global__ void __launch_bounds__(kThreads) conv_fwd_kernel(ConvArgs a) {
     constexpr int kW = wimage_bytes(kCin, kCout);
     constexpr uint32_t kIdesc = umma::idesc_bf16(128, kCout, 0, 0);
     extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* s_halo = smem;                              // kSlots rows: row yy in slot (yy + 4) & 3
     uint8_t* s_w = smem + kSlots * kSlot;
-    constexpr int kHalfSlot = kHalfPix * kG * 16;
-    uint8_t* s_hstage = s_w + kW;                        // load mode 1: kSlots half rows
-    __shared__ __align__(8) uint64_t s_bar[2];   // MMA completion, one per accumulator
+    __shared__ __align__(8) uint64_t s_full[kSlots], s_empty[kSlots];        // a row has landed; its MMAs are done
+    __shared__ __align__(8) uint64_t s_afull[kAccs], s_aempty[kAccs];        // an accumulator is done; it was read
     __shared__ uint32_t s_taddr;
     __shared__ float s_bias[kCout];
     constexpr bool kPool = kCin == 16 && kCout == 32;   // the pooled output (conv1 of the denoiser)
-    __shared__ __align__(16) uint4 s_pool[kPool ? kThreads * 4 : 1];   // an even row's bf16 outputs
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    const int strips_x = (a.w + 127) / 128;
-    const int segs = (a.h + a.row_offset + a.rows_per_cta - 1) / a.rows_per_cta;
-    const int item = blockIdx.x;
-    if (item >= a.n * strips_x * segs) return;
-    const int seg = item % segs, strip = item / segs;
-    const int n = strip / strips_x, x0 = (strip % strips_x) * 128;
-    const int y0 = max(0, seg * a.rows_per_cta - a.row_offset);
-    const int y1 = min(a.h, seg * a.rows_per_cta - a.row_offset + a.rows_per_cta);
-    const int tid = threadIdx.x, warp = tid >> 5;
-
-    // weights: the packed image, copied verbatim; the bias
-    for (int i = tid; i < kW / 16; i += kThreads)
-        reinterpret_cast<uint4*>(s_w)[i] = __ldg(reinterpret_cast<const uint4*>(a.wimage) + i);
-    if (tid < kCout) s_bias[tid] = a.bias ? __ldg(a.bias + tid) : 0.0f;
     if (tid == 0) {
-        mbar_init(&s_bar[0], 1);
-        mbar_init(&s_bar[1], 1);
+        for (int k = 0; k < kSlots; ++k) {
+            mbar_init(&s_full[k], kLoaders);
+            mbar_init(&s_empty[k], 1);
+        }
+        for (int k = 0; k < kAccs; ++k) {
+            mbar_init(&s_afull[k], 1);
+            mbar_init(&s_aempty[k], kEpiWarps * 32);
+        }
         mbar_fence_init();
     }
-    if (warp == 0) umma::tmem_alloc(&s_taddr, 64);   // two accumulators of 32 columns
-
-    // Rows come in by cp.async, one row ahead of the MMAs (the copy of row
-    // y + 2 is in flight while row y is multiplied).  Load mode 1 also copies
-    // the half-resolution row under the halo into a staging buffer, and a
-    // pass over the landed row adds it in (FP32 sum rounded to bf16).
-    auto slot_of = [&](int yy) { return s_halo + ((yy + 4) & 3) * kSlot; };
-    auto hstage_of = [&](int yy) { return s_hstage + ((yy + 4) & 3) * kHalfSlot; };
-    auto issue_row = [&](int yy) {
-        uint8_t* slot = slot_of(yy);
-        const bool row_in = yy >= 0 && yy < a.h;
-        const __nv_bfloat16* rowp = a.x + ((size_t)n * a.h + (row_in ? yy : 0)) * a.w * kCin;
-        for (int q = tid; q < 130 * kG; q += kThreads) {
-            const int hp = q / kG, g = q - hp * kG;
-            const int x = x0 - 1 + hp;
-            const bool in = row_in && x >= 0 && x < a.w;
-            cp_async16(slot + g * kColBytes + hp * 16, in ? rowp + (size_t)x * kCin + g * 8 : a.x, in ? 16u : 0u);
-        }
-        if (kLoad == 1) {
-            const int hh = a.h >> 1, hw = a.w >> 1, hx0 = (x0 - 1) >> 1;
-            uint8_t* hs = hstage_of(yy);
-            const __nv_bfloat16* hrow = a.xh + ((size_t)n * hh + (row_in ? min(yy >> 1, hh - 1) : 0)) * hw * kCin;
-            for (int q = tid; q < kHalfPix * kG; q += kThreads) {
-                const int hp = q / kG, g = q - hp * kG;
-                // clamped like the row: an odd width's last pixel takes the last half pixel
-                const int hx = min(max(hx0 + hp, 0), hw - 1);
-                cp_async16(hs + q * 16, row_in ? hrow + (size_t)hx * kCin + g * 8 : a.xh, row_in ? 16u : 0u);
-            }
-        }
-        cp_async_commit();
-    };
-    // load mode 1: row yy's landed halo += its upsampled half-resolution row
-    auto combine_row = [&](int yy) {
-        if (yy < 0 || yy >= a.h) return;
-        uint8_t* slot = slot_of(yy);
-        const uint8_t* hs = hstage_of(yy);
-        const int hx0 = (x0 - 1) >> 1;
-        for (int q = tid; q < 130 * kG; q += kThreads) {
-            const int hp = q / kG, g = q - hp * kG;
-            const int x = x0 - 1 + hp;
-            if (x < 0 || x >= a.w) continue;
-            uint4* dst = reinterpret_cast<uint4*>(slot + g * kColBytes + hp * 16);
-            *dst = bf16x8_add(*dst, *reinterpret_cast<const uint4*>(hs + (((x >> 1) - hx0) * kG + g) * 16));
-        }
-    };
-    issue_row(y0 - 1);
-    issue_row(y0);
-    issue_row(y0 + 1);
-    if (kLoad == 1) {
-        asm volatile("cp.async.wait_group 1;" ::: "memory");   // rows y0 - 1 and y0
-        __syncthreads();
-        combine_row(y0 - 1);
-        combine_row(y0);
-    }
+    if (warp == kMmaWarp) umma::tmem_alloc(&s_taddr, kAccs * 32);
+    pdl_wait();   // launched as a programmatic dependent: nothing above touches global memory
+    // weights: the packed image, copied verbatim; the bias
+    for (int i = tid; i < kW / 16; i += kFwdThreads)
+        reinterpret_cast<uint4*>(s_w)[i] = __ldg(reinterpret_cast<const uint4*>(a.wimage) + i);
+    if (tid < kCout) s_bias[tid] = a.bias ? __ldg(a.bias + tid) : 0.0f;
+    umma::fence_smem_to_async();
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t taddr = s_taddr;
-    const uint32_t halo_base = smem_u32(s_halo), w_base = smem_u32(s_w);
-    uint32_t phase0 = 0, phase1 = 0;
+    ConvRuns runs(a);
+    ConvRun r;
     bool failed = false;
-    float err_sum = 0.0f, err_cnt = 0.0f;   // head mode: this thread's column of the band, in row order
-    // Two TMEM accumulators: the MMAs of row y (accumulator y & 1) run while
-    // the epilogue of row y - 1 reads the other one.
-    auto wait_mma = [&](int y) {   // row y's MMAs are done (every thread waits)
-        if (!mbar_wait_bounded(&s_bar[y & 1], (y & 1) ? phase1 : phase0, kWaitLimit)) failed = true;
-        if (y & 1) phase1 ^= 1u; else phase0 ^= 1u;
-    };
-    auto mma_row = [&](int y) {
-        if (tid == 0) {
-            umma::fence_after_sync();
-            const uint32_t acc_addr = taddr + (uint32_t)((y & 1) * 32);
-            uint32_t acc = 0;
-#pragma unroll
-            for (int ky = 0; ky < 3; ++ky) {
-                const uint32_t slot = halo_base + (uint32_t)(((y - 1 + ky + 4) & 3) * kSlot);
-#pragma unroll
-                for (int kx = 0; kx < 3; ++kx) {
-#pragma unroll
-                    for (int kb = 0; kb < kCin / 16; ++kb) {
-                        const uint64_t ad = umma::smem_desc(slot + (uint32_t)(2 * kb * kColBytes + kx * 16),
-                                                            (uint32_t)kColBytes, 128u);
-                        const int k0 = (ky * 3 + kx) * kCin + kb * 16;
-                        const uint64_t bd =
-                            umma::smem_desc(w_base + (uint32_t)((k0 >> 3) * kCout * 16), (uint32_t)(kCout * 16), 128u);
-                        umma::mma_bf16(acc_addr, ad, bd, kIdesc, acc);
-                        acc = 1;
-                    }
-                }
-            }
-            umma::commit(&s_bar[y & 1]);
-        }
-    };
-    auto epilogue = [&](int y) {   // row y's MMAs waited for
-        umma::fence_after_sync();
-        const uint32_t acc_addr = taddr + (uint32_t)((y & 1) * 32) + ((uint32_t)(warp * 32) << 16);
-        const int x = x0 + tid;
-        const size_t o = ((size_t)n * a.h + y) * a.w + x;
-        float v[32];
-        if (kCout == 32) {
-            umma::tmem_ld32(acc_addr, *reinterpret_cast<float(*)[32]>(v));
-        } else {
-            umma::tmem_ld16(acc_addr, *reinterpret_cast<float(*)[16]>(v));
-        }
-        if (x < a.w && !failed) {
-            if (a.bias) {
-#pragma unroll
-                for (int c = 0; c < kCout; ++c) v[c] += s_bias[c];
-            }
-            if (a.relu) {
-#pragma unroll
-                for (int c = 0; c < kCout; ++c) v[c] = fmaxf(v[c], 0.0f);
-            }
-            if (a.mask) {
-                const uint4* mp = reinterpret_cast<const uint4*>(a.mask + o * kCout);
-#pragma unroll
-                for (int q = 0; q < kCout / 8; ++q) {
-                    const uint4 mv = __ldg(mp + q);
-                    const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(&mv);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        if (!(__bfloat162float(mb[e]) > 0.0f)) v[q * 8 + e] = 0.0f;
-                }
-            }
-            if (kCout == 16 && a.head_x) {
-                // the denoised frame's pixel (head_rgba of the output step) and its error estimate
-                const uint4 xv = __ldg(reinterpret_cast<const uint4*>(a.head_x + o * 16));
-                const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(&xv);
-                const float4 px = make_float4(__bfloat162float(xb[5]) + v[0], __bfloat162float(xb[6]) + v[1],
-                                              __bfloat162float(xb[7]) + v[2], __bfloat162float(xb[3]) + v[3]);
-                __half2 h01 = __floats2half2_rn(px.x, px.y), h23 = __floats2half2_rn(px.z, px.w);
-                uint2 pk;
-                pk.x = *reinterpret_cast<uint32_t*>(&h01);
-                pk.y = *reinterpret_cast<uint32_t*>(&h23);
-                reinterpret_cast<uint2*>(a.head_out16)[o] = pk;
-                err_sum += fmaxf(v[4], 0.0f);
-                err_cnt += 1.0f;
-            }
-            if (a.out_bf16) {
-                uint4* op = reinterpret_cast<uint4*>(a.out_bf16 + o * kCout);
-#pragma unroll
-                for (int q = 0; q < kCout / 8; ++q) {
-                    uint4 pk;
-                    __nv_bfloat162* pb = reinterpret_cast<__nv_bfloat162*>(&pk);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) pb[e] = __floats2bfloat162_rn(v[q * 8 + 2 * e], v[q * 8 + 2 * e + 1]);
-                    op[q] = pk;
-                }
-            }
-            if (a.out_f32) {
-                float4* op = reinterpret_cast<float4*>(a.out_f32 + o * kCout);
-#pragma unroll
-                for (int q = 0; q < kCout / 4; ++q)
-                    op[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            }
-        }
-        if (kPool && a.pool_out) {
-            // 2x2 average of the bf16 outputs: (0 + (y, x) + (y, x + 1) + (y + 1, x) + (y + 1, x + 1)) * 0.25,
-            // the even row parked in shared memory, the right neighbour's by a lane shuffle
-            uint32_t pk[16];
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
-                pk[e] = *reinterpret_cast<uint32_t*>(&b2);
-            }
-            if ((y & 1) == 0) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) s_pool[tid * 4 + q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-            } else {
-                uint32_t nb[16];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) nb[e] = __shfl_xor_sync(0xffffffffu, pk[e], 1);
-                if ((x & 1) == 0 && x < a.w && !failed) {
-                    const uint32_t* up = reinterpret_cast<const uint32_t*>(&s_pool[tid * 4]);
-                    const uint32_t* un = reinterpret_cast<const uint32_t*>(&s_pool[(tid + 1) * 4]);
-                    uint32_t res[16];
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) {
-                        const uint32_t t4[4] = {up[e], un[e], pk[e], nb[e]};
-                        float acc0 = 0.0f, acc1 = 0.0f;
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&t4[k]));
-                            acc0 += f.x;
-                            acc1 += f.y;
-                        }
-                        __nv_bfloat162 r2 = __floats2bfloat162_rn(0.25f * acc0, 0.25f * acc1);
-                        res[e] = *reinterpret_cast<uint32_t*>(&r2);
-                    }
-                    const int hw2 = a.w >> 1;
-                    uint4* dp = reinterpret_cast<uint4*>(a.pool_out + (((size_t)n * (a.h >> 1) + (y >> 1)) * hw2 + (x >> 1)) * kCout);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) dp[q] = make_uint4(res[4 * q], res[4 * q + 1], res[4 * q + 2], res[4 * q + 3]);
-                }
-            }
-        }
-        umma::fence_before_sync();
-    };
 
-    bool broke = false;   // uniform over the CTA (from __syncthreads_or)
-    for (int y = y0; y < y1; ++y) {
-        if (y > y0) wait_mma(y - 1);    // its MMAs were the last readers of row y - 2's slot
-        issue_row(y + 2);               // into that slot
-        asm volatile("cp.async.wait_group 1;" ::: "memory");   // rows up to y + 1 have landed
-        if (kLoad == 1) {
-            __syncthreads();            // every thread's copies of row y + 1 are visible
-            combine_row(y + 1);
-        }
-        umma::fence_smem_to_async();
-        if (__syncthreads_or(failed)) {
-            failed = broke = true;
-            break;
-        }
-        mma_row(y);
-        if (y > y0) epilogue(y - 1);
-    }
-    if (!broke) {   // the whole CTA: the epilogue's TMEM loads are warp-collective
-        wait_mma(y1 - 1);
-        if (kPool && a.pool_out) __syncthreads();   // the even row parked by the previous epilogue
-        epilogue(y1 - 1);
-    }
-    if (kCout == 16 && a.head_x && !broke) {
-        // per tile (16 threads = 16 columns of the band): the sum of the error estimates and the
-        // pixel count, each over 16 lanes in a fixed order, then the tile's mean
+    if (warp >= kEpiWarps && warp < kMmaWarp) {
+        // ---- load: entry e of the ring (the run's rows y0 - 1 .. y1, then the next run's) by group e & 1
+        const int lt = (tid - kEpiWarps * 32) % kLoaders;
+        const uint32_t group = (uint32_t)((tid - kEpiWarps * 32) / kLoaders);
+        uint32_t e = 0;
+        int pending = -1;   // slot of this group's copied row that is not announced yet
+        while (!failed && runs.next(r)) {
+            for (int yy = r.y0 - 1; yy <= r.y1 && !failed; ++yy, ++e) {
+                if ((e & 1u) != group) continue;
+                const int slot = (int)(e % kSlots);
+                if (e >= kSlots && !mbar_wait_suspend(&s_empty[slot], (e / kSlots - 1u) & 1u)) {
+                    failed = true;
+                    break;
+                }
+                uint8_t* dst = smem + slot * kSlot;
+                const bool row_in = yy >= 0 && yy < a.h;
+                const __nv_bfloat16* rowp = a.x + ((size_t)r.n * a.h + (row_in ? yy : 0)) * a.w * kCin;
+                if (kLoad == 0) {
+                    // copied asynchronously; announced once the group's next row is on its way
+                    for (int q = lt; q < 130 * kG; q += kLoaders) {
+                        const int hp = q / kG, g = q - hp * kG, x = r.x0 - 1 + hp;
+                        const bool in = row_in && x >= 0 && x < a.w;
+                        cp_async16(dst + g * kColBytes + hp * 16, in ? rowp + (size_t)x * kCin + g * 8 : a.x, in ? 16u : 0u);
+                    }
+                    cp_async_commit();
+                    if (pending >= 0) {
+                        cp_async_wait_all_but_one();
+                        umma::fence_smem_to_async();
+                        mbar_arrive(&s_full[pending]);
+                    }
+                    pending = slot;
+                } else {
+                    // x + the 2x nearest upsampling of xh (FP32 sum rounded to bf16): all of a
+                    // thread's granules loaded before the first is stored
+                    constexpr int kPer = (130 * kG + kLoaders - 1) / kLoaders;
+                    const int hh = a.h >> 1, hw = a.w >> 1;
+                    const __nv_bfloat16* hrow = a.xh + ((size_t)r.n * hh + (row_in ? min(yy >> 1, hh - 1) : 0)) * hw * kCin;
+                    uint4 v[kPer], u[kPer];
 #pragma unroll
-        for (int off = 8; off; off >>= 1) {
-            err_sum += __shfl_xor_sync(0xffffffffu, err_sum, off);
-            err_cnt += __shfl_xor_sync(0xffffffffu, err_cnt, off);
+                    for (int k = 0; k < kPer; ++k) {
+                        const int q = lt + k * kLoaders, hp = q / kG, g = q - hp * kG, x = r.x0 - 1 + hp;
+                        v[k] = u[k] = make_uint4(0u, 0u, 0u, 0u);
+                        if (row_in && x >= 0 && x < a.w && q < 130 * kG) {
+                            v[k] = __ldg(reinterpret_cast<const uint4*>(rowp + (size_t)x * kCin) + g);
+                            u[k] = __ldg(reinterpret_cast<const uint4*>(hrow + (size_t)min(x >> 1, hw - 1) * kCin) + g);
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < kPer; ++k) {
+                        const int q = lt + k * kLoaders, hp = q / kG, g = q - hp * kG;
+                        if (q < 130 * kG) *reinterpret_cast<uint4*>(dst + g * kColBytes + hp * 16) = bf16x8_add(v[k], u[k]);
+                    }
+                    umma::fence_smem_to_async();
+                    mbar_arrive(&s_full[slot]);
+                }
+            }
         }
-        const int tx = (x0 >> 4) + (tid >> 4);
-        if ((tid & 15) == 0 && tx < a.tiles_x && err_cnt > 0.0f) {
-            const int ty = (a.h + a.row_offset) / 16 - 1 - seg;   // GL tile row of this band
-            const uint32_t tile = (uint32_t)(ty * a.tiles_x + tx);
-            const float mse = err_sum / err_cnt * 0.001f;
-            if (a.tile_err) a.tile_err[tile] = mse;
-            if (mse >= a.err_budget) a.fallback_tiles[atomicAdd(a.fallback_count, 1u)] = tile;
+        cp_async_wait_all();
+        if (pending >= 0) {
+            umma::fence_smem_to_async();
+            mbar_arrive(&s_full[pending]);
+        }
+    } else if (warp == kMmaWarp) {
+        // ---- multiply: one thread
+        if (lane == 0) {
+            const uint32_t halo_base = smem_u32(smem), w_base = smem_u32(s_w);
+            uint32_t e = 0, m = 0;   // ring entry of the row above; output rows so far
+            while (!failed && runs.next(r)) {
+                for (int y = r.y0; y < r.y1; ++y, ++e, ++m) {
+                    bool ok = true;
+                    for (uint32_t k = y == r.y0 ? 0u : 2u; k < 3u && ok; ++k)
+                        ok = mbar_wait_suspend(&s_full[(e + k) % kSlots], ((e + k) / kSlots) & 1u);
+                    const uint32_t acc = m % kAccs;
+                    if (ok && m >= kAccs) ok = mbar_wait_suspend(&s_aempty[acc], (m / kAccs - 1u) & 1u);
+                    if (!ok) {
+                        failed = true;
+                        break;
+                    }
+                    umma::fence_after_sync();
+                    uint32_t accumulate = 0;
+#pragma unroll
+                    for (int ky = 0; ky < 3; ++ky) {
+                        const uint32_t slot = halo_base + ((e + (uint32_t)ky) % kSlots) * (uint32_t)kSlot;
+#pragma unroll
+                        for (int kx = 0; kx < 3; ++kx) {
+#pragma unroll
+                            for (int kb = 0; kb < kCin / 16; ++kb) {
+                                const uint64_t ad = umma::smem_desc(slot + (uint32_t)(2 * kb * kColBytes + kx * 16),
+                                                                    (uint32_t)kColBytes, 128u);
+                                const int k0 = (ky * 3 + kx) * kCin + kb * 16;
+                                const uint64_t bd = umma::smem_desc(w_base + (uint32_t)((k0 >> 3) * kCout * 16),
+                                                                    (uint32_t)(kCout * 16), 128u);
+                                umma::mma_bf16(taddr + acc * 32u, ad, bd, kIdesc, accumulate);
+                                accumulate = 1;
+                            }
+                        }
+                    }
+                    umma::commit(&s_empty[e % kSlots]);   // this row was the last to read the row above it
+                    umma::commit(&s_afull[acc]);
+                }
+                if (!failed) {   // the run's last two halo rows
+                    umma::commit(&s_empty[e % kSlots]);
+                    umma::commit(&s_empty[(e + 1u) % kSlots]);
+                    e += 2u;
+                }
+            }
+            // every MMA of this CTA, and the last commit's arrival, is done before its shared memory and TMEM go
+            if (!failed && m > 0 && !mbar_wait_suspend(&s_empty[(e - 1u) % kSlots], ((e - 1u) / kSlots) & 1u)) failed = true;
+        }
+        __syncwarp();
+    } else {
+        // ---- epilogue: thread t holds pixel x0 + t of a row
+        uint32_t m = 0;
+        float err_sum = 0.0f, err_cnt = 0.0f;   // head mode: this thread's column of the band, in row order
+        uint32_t even[kPool ? 16 : 1];          // the bf16 outputs of the even row above (pooled output)
+        while (!failed && runs.next(r)) {
+            const int x = r.x0 + tid;
+            for (int y = r.y0; y < r.y1; ++y, ++m) {
+                const uint32_t acc = m % kAccs;
+                const size_t o = ((size_t)r.n * a.h + y) * a.w + x;
+                if (!mbar_wait_suspend(&s_afull[acc], (m / kAccs) & 1u)) {
+                    failed = true;
+                    break;
+                }
+                umma::fence_after_sync();
+                const uint32_t acc_addr = taddr + acc * 32u + ((uint32_t)(warp * 32) << 16);
+                float v[32];
+                if (kCout == 32) umma::tmem_ld32(acc_addr, *reinterpret_cast<float(*)[32]>(v));
+                else umma::tmem_ld16(acc_addr, *reinterpret_cast<float(*)[16]>(v));
+                umma::fence_before_sync();
+                mbar_arrive(&s_aempty[acc]);
+                uint32_t pk[kCout / 2];
+                if (a.bias) {
+#pragma unroll
+                    for (int c = 0; c < kCout; ++c) v[c] += s_bias[c];
+                }
+                if (a.relu) {
+#pragma unroll
+                    for (int c = 0; c < kCout; ++c) v[c] = fmaxf(v[c], 0.0f);
+                }
+                if (x < a.w) {
+                    if (a.mask) {
+                        const uint4* mp = reinterpret_cast<const uint4*>(a.mask + o * kCout);
+#pragma unroll
+                        for (int q = 0; q < kCout / 8; ++q) {
+                            const uint4 mv = __ldg(mp + q);
+                            const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(&mv);
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                if (!(__bfloat162float(mb[i]) > 0.0f)) v[q * 8 + i] = 0.0f;
+                        }
+                    }
+                    if (kCout == 16 && a.head_x) {
+                        // the denoised frame's pixel (head_rgba of the output step) and its error estimate
+                        const uint4 xv = __ldg(reinterpret_cast<const uint4*>(a.head_x + o * 16));
+                        const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(&xv);
+                        const float4 px = make_float4(__bfloat162float(xb[5]) + v[0], __bfloat162float(xb[6]) + v[1],
+                                                      __bfloat162float(xb[7]) + v[2], __bfloat162float(xb[3]) + v[3]);
+                        __half2 h01 = __floats2half2_rn(px.x, px.y), h23 = __floats2half2_rn(px.z, px.w);
+                        uint2 pk2;
+                        pk2.x = *reinterpret_cast<uint32_t*>(&h01);
+                        pk2.y = *reinterpret_cast<uint32_t*>(&h23);
+                        reinterpret_cast<uint2*>(a.head_out16)[o] = pk2;
+                        err_sum += fmaxf(v[4], 0.0f);
+                        err_cnt += 1.0f;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < kCout / 2; ++i) {
+                    __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                    pk[i] = *reinterpret_cast<uint32_t*>(&b2);
+                }
+                if (a.out_bf16 && x < a.w) {
+                    uint4* op = reinterpret_cast<uint4*>(a.out_bf16 + o * kCout);
+#pragma unroll
+                    for (int q = 0; q < kCout / 16; ++q) {
+                        const uint4 lo = make_uint4(pk[8 * q], pk[8 * q + 1], pk[8 * q + 2], pk[8 * q + 3]);
+                        const uint4 hi = make_uint4(pk[8 * q + 4], pk[8 * q + 5], pk[8 * q + 6], pk[8 * q + 7]);
+                        if (a.out_wide) {
+                            st_global32(op + 2 * q, lo, hi);
+                        } else {
+                            op[2 * q] = lo;
+                            op[2 * q + 1] = hi;
+                        }
+                    }
+                }
+                if (a.out_f32 && x < a.w) {
+                    float4* op = reinterpret_cast<float4*>(a.out_f32 + o * kCout);
+#pragma unroll
+                    for (int q = 0; q < kCout / 4; ++q)
+                        op[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                }
+                if (kPool && a.pool_out) {
+                    // 2x2 average of the bf16 outputs: (0 + (y, x) + (y, x + 1) + (y + 1, x) + (y + 1, x + 1)) * 0.25,
+                    // the right neighbour's by lane shuffles (runs hold whole row pairs)
+                    if ((y & 1) == 0) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) even[i] = pk[i];
+                    } else {
+                        const bool write = (x & 1) == 0 && x < a.w;
+                        uint4* dp = reinterpret_cast<uint4*>(
+                            a.pool_out + (((size_t)r.n * (a.h >> 1) + (y >> 1)) * (a.w >> 1) + (x >> 1)) * kCout);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            uint32_t res[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const uint32_t up = even[4 * q + i], down = pk[4 * q + i];
+                                const uint32_t t4[4] = {up, __shfl_xor_sync(0xffffffffu, up, 1), down,
+                                                        __shfl_xor_sync(0xffffffffu, down, 1)};
+                                float acc0 = 0.0f, acc1 = 0.0f;
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&t4[k]));
+                                    acc0 += f.x;
+                                    acc1 += f.y;
+                                }
+                                __nv_bfloat162 r2 = __floats2bfloat162_rn(0.25f * acc0, 0.25f * acc1);
+                                res[i] = *reinterpret_cast<uint32_t*>(&r2);
+                            }
+                            if (write) dp[q] = make_uint4(res[0], res[1], res[2], res[3]);
+                        }
+                    }
+                }
+                if (kCout == 16 && a.head_x && (y + 1 == r.y1 || (y + 1 + a.row_offset) % 16 == 0)) {
+                    // end of a band: per tile (16 threads = 16 columns) the sum of the error estimates and the
+                    // pixel count, each over 16 lanes in a fixed order, then the tile's mean
+#pragma unroll
+                    for (int off = 8; off; off >>= 1) {
+                        err_sum += __shfl_xor_sync(0xffffffffu, err_sum, off);
+                        err_cnt += __shfl_xor_sync(0xffffffffu, err_cnt, off);
+                    }
+                    const int tx = (r.x0 >> 4) + (tid >> 4);
+                    if ((tid & 15) == 0 && tx < a.tiles_x && err_cnt > 0.0f) {
+                        const int band = (y + a.row_offset) / 16;
+                        const int ty = (a.h + a.row_offset) / 16 - 1 - band;   // GL tile row of this band
+                        const uint32_t tile = (uint32_t)(ty * a.tiles_x + tx);
+                        const float mse = err_sum / err_cnt * 0.001f;
+                        if (a.tile_err) a.tile_err[tile] = mse;
+                        if (mse >= a.err_budget) a.fallback_tiles[atomicAdd(a.fallback_count, 1u)] = tile;
+                    }
+                    err_sum = err_cnt = 0.0f;
+                }
+            }
         }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");   // the prefetched rows past the run
-    if (failed && tid == 0) atomicOr(a.err, 1u);
+    if (failed && (lane == 0 || warp != kMmaWarp)) atomicOr(a.err, 1u);
+    umma::fence_before_sync();
     __syncthreads();
-    if (warp == 0) umma::tmem_dealloc(taddr, 64);
+    if (warp == kMmaWarp) {
+        umma::fence_after_sync();
+        umma::tmem_dealloc(taddr, kAccs * 32);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -611,17 +690,21 @@ __global__ void pack_weights_kernel(const float* __restrict__ w, int cin, int co
 }
 
 template <int kCin, int kCout, int kLoad>
-static int launch_fwd_t(const ConvArgs& a, cudaStream_t s) {
-    const int strips = a.n * ((a.w + 127) / 128);
-    const int segs = (a.h + a.row_offset + a.rows_per_cta - 1) / a.rows_per_cta;
-    const size_t smem = (size_t)fwd_smem_bytes(kCin, kCout, kLoad);
+static int launch_fwd_t(ConvArgs a, cudaStream_t s) {
+    const long strips = (long)a.n * ((a.w + 127) / 128);
+    const long units = strips * ((a.h + a.row_offset + a.unit_rows - 1) / a.unit_rows);
+    const size_t smem = (size_t)fwd_smem_bytes(kCin, kCout);
+    a.out_wide = (reinterpret_cast<uintptr_t>(a.out_bf16) & 31u) == 0u ? 1 : 0;
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(conv_fwd_kernel<kCin, kCout, kLoad>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
         attr = true;
     }
-    conv_fwd_kernel<kCin, kCout, kLoad><<<strips * segs, kThreads, smem, s>>>(a);
+    // two CTAs an SM; on small images one unit each at most
+    const long ctas = 2L * a.max_sms;
+    launch_pdl(conv_fwd_kernel<kCin, kCout, kLoad>, dim3((unsigned)(units < ctas ? units : ctas)), dim3(kFwdThreads), smem,
+               s, a);
     return 1;
 }
 

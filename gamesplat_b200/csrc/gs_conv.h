@@ -20,15 +20,17 @@ struct ConvArgs {
     const __nv_bfloat16* mask;  // Cout-channel tensor: outputs where mask <= 0 become 0 (ReLU backward); or null
     __nv_bfloat16* out_bf16;    // Cout channels, or null
     float* out_f32;             // Cout channels, or null
-    int rows_per_cta;
+    int unit_rows;              // rows that stay in one CTA: 1, 2 (pool_out) or 16 (head_x)
     uint32_t* err;              // bit 0 set if a bounded wait ran out
-    int row_offset;             // the row bands of the CTAs start at -row_offset (0: at row 0)
+    int row_offset;             // the units' row bands start at -row_offset (0: at row 0)
+    int max_sms;                // SMs of the device
+    int out_wide;               // out_bf16 is 32-byte aligned (set by launch_fwd)
     // (Cin = 16, Cout = 32, forward): also the 2x2 average of the bf16 output, n x h/2 x w/2 (h, w
-    // and rows_per_cta even), summed and rounded as the denoiser's pooling kernel does
+    // even, unit_rows 2), summed from zero in row order and rounded once
     __nv_bfloat16* pool_out;
     // Denoised-mode head (Cout = 16, forward, head_x set): the epilogue writes head_out16 =
     // RGBA16F (head_x[5..7] + o[0..2], head_x[3] + o[3]) instead of the outputs above and,
-    // per 16x16 tile of GL rows (rows_per_cta = 16 and row_offset aligning the bands with
+    // per 16x16 tile of GL rows (unit_rows = 16 and row_offset aligning the bands with
     // them), tile_err = mean(max(o[4], 0)) * 0.001, listing tiles at or above err_budget.
     const __nv_bfloat16* head_x;   // the network input (16 channels per pixel)
     uint16_t* head_out16;

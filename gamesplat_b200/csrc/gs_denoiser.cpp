@@ -149,13 +149,6 @@ static void pack_images(gs_denoiser* d, cudaStream_t s) {
     d->images_valid = true;
 }
 
-static int rows_per_cta(const gs_denoiser* d, int n, int h, int w) {
-    const long strips = (long)n * ((w + 127) / 128);
-    const long want = (long)d->num_sms * 8;   // enough CTAs for every SM's occupancy, a few rows each
-    long rows = (strips * h + want - 1) / want;
-    return (int)std::max(2L, std::min(64L, rows));
-}
-
 static int conv_fwd(gs_denoiser* d, int l, bool transposed, const bf16* x, const bf16* xh, int n, int h, int w,
                     const bf16* mask, bf16* out_bf16, float* out_f32, cudaStream_t s) {
     const Layer& L = kNet[l];
@@ -171,11 +164,12 @@ static int conv_fwd(gs_denoiser* d, int l, bool transposed, const bf16* x, const
     a.mask = mask;
     a.out_bf16 = out_bf16;
     a.out_f32 = out_f32;
-    a.rows_per_cta = rows_per_cta(d, n, h, w);
+    a.unit_rows = 1;
+    a.max_sms = (int)d->num_sms;
     a.err = d->err;
-    if (l == 0 && !transposed) {   // conv1 also writes p1 = avgpool2(e1): row bands of an even number of rows
+    if (l == 0 && !transposed) {   // conv1 also writes p1 = avgpool2(e1): row pairs stay together
         a.pool_out = d->p1;
-        a.rows_per_cta = (a.rows_per_cta + 1) & ~1;
+        a.unit_rows = 2;
     }
     const int cin = transposed ? L.cout : L.cin, cout = transposed ? L.cin : L.cout;
     return conv::launch_fwd(cin, cout, transposed ? 0 : L.load, a, s) < 0 ? GS_ERR_BAD_ARG : GS_OK;
@@ -238,7 +232,8 @@ int forward_frame(gs_denoiser* d, const bf16* x, int h, int w, uint16_t* out16, 
     a.wimage = d->wimg[4];
     a.bias = d->params + b_offset(4);
     a.relu = L.relu;
-    a.rows_per_cta = 16;
+    a.unit_rows = 16;
+    a.max_sms = (int)d->num_sms;
     a.row_offset = (16 - h % 16) % 16;
     a.err = d->err;
     a.head_x = x;
@@ -523,6 +518,13 @@ int gs_denoiser_status(gs_denoiser* d) {
 }
 
 // ---- stage-level convolutions ----------------------------------------------
+static int device_sms() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 148;
+}
+
 int gs_conv3x3_bf16(const void* x, const void* x_half, int n, int h, int w, int cin, int cout, const float* weights,
                     const float* bias, int relu, int transposed, const void* mask, void* out_bf16, float* out_f32,
                     void* image_scratch, uint32_t* err, void* stream) {
@@ -544,7 +546,8 @@ int gs_conv3x3_bf16(const void* x, const void* x_half, int n, int h, int w, int 
     a.mask = static_cast<const bf16*>(mask);
     a.out_bf16 = static_cast<bf16*>(out_bf16);
     a.out_f32 = out_f32;
-    a.rows_per_cta = 8;
+    a.unit_rows = 1;
+    a.max_sms = device_sms();
     a.err = err;
     const int ci = transposed ? cout : cin, co = transposed ? cin : cout;
     if (gs::conv::launch_fwd(ci, co, x_half ? 1 : 0, a, s) < 0) return GS_ERR_BAD_ARG;
@@ -565,10 +568,7 @@ int gs_conv3x3_wgrad_bf16(const void* x, const void* x_half, int n, int h, int w
     a.dw = dw;
     a.db = db;
     a.err = err;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (gs::conv::launch_wgrad(cin, cout, x_half ? 1 : 0, a, sms > 0 ? sms : 148, static_cast<cudaStream_t>(stream)) < 0)
+    if (gs::conv::launch_wgrad(cin, cout, x_half ? 1 : 0, a, device_sms(), static_cast<cudaStream_t>(stream)) < 0)
         return GS_ERR_BAD_ARG;
     return cudaGetLastError() == cudaSuccess ? GS_OK : GS_ERR_CUDA;
 }

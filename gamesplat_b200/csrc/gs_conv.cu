@@ -11,11 +11,13 @@
 // its share of the rows; input rows (130 pixels with the halo) pass through a
 // ring of shared-memory slots in the K-major core-matrix layout, rows of
 // 16 bytes one pixel apart, so the A operand of tap (ky, kx) is the slot of row
-// y - 1 + ky started kx pixels (kx * 16 bytes) further: no im2col copy.  The
-// warps have fixed roles that meet only at mbarriers: 8 load rows, one thread
-// issues the 9 * Cin / 16 MMAs of a row into one of 4 TMEM accumulators, and 4
-// read accumulators back (thread t = TMEM lane t = pixel t) for the epilogue
-// (bias, ReLU, ReLU mask, bf16 / f32 store).
+// y - 1 + ky started kx pixels (kx * 16 bytes) further: no im2col copy.  An MMA
+// takes a row for the three output rows it belongs to at once (N = 3 Cout, the
+// weights of ky = 2, 1, 0 side by side, the accumulators of consecutive rows
+// adjacent in TMEM).  The warps have fixed roles that meet only at mbarriers:
+// some load rows, one thread issues MMAs into a ring of 8 TMEM accumulators,
+// some read accumulators back (a thread = a TMEM lane = a pixel) for the
+// epilogue (bias, ReLU, ReLU mask, bf16 / f32 store).
 //
 // conv_wgrad_kernel: the weight gradient, K = pixels; see there.
 //
@@ -42,12 +44,13 @@ constexpr uint32_t kWaitLimit = 1u << 22;
 
 __host__ __device__ constexpr int wimage_bytes(int cin, int cout) { return 9 * cin * cout * 2; }
 
-// Roles of the forward kernel's warps (an epilogue warp's number is its TMEM lane quadrant).
-constexpr int kEpiWarps = 4, kLoadWarps = 8, kMmaWarp = kEpiWarps + kLoadWarps;
+// The forward kernel's warps: 12 that read accumulators back or load rows (see Roles), and the one that multiplies.
+constexpr int kMmaWarp = 12;
 constexpr int kFwdThreads = (kMmaWarp + 1) * 32;
-constexpr int kLoaders = kLoadWarps * 16;   // threads of a load group: the two groups take rows in turn
+constexpr int kGroup = 128;                 // threads that load a row, or that read one back
 constexpr int kSlots = 8;                   // halo rows in the ring
-constexpr int kAccs = 4;                    // TMEM accumulators of 32 columns
+constexpr int kAhead = 3;                   // rows copied behind the one announced next
+constexpr int kAccs = 8;                    // TMEM accumulators of Cout columns
 
 // Dynamic shared memory of the forward kernel: the halo rows and the weight image.
 __host__ __device__ constexpr int fwd_smem_bytes(int cin, int cout) {
@@ -60,7 +63,8 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t 
                  : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void cp_async_wait_but() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Wait for phase `phase` of a barrier, suspended for up to a microsecond between tests; false after a second or so.
@@ -144,41 +148,54 @@ struct ConvRuns {
     }
 };
 
+// Load mode 1 adds two tensors on the way in, through registers: two groups of
+// loading threads take rows in turn and one group runs the epilogues.  Load
+// mode 0 copies asynchronously and one group keeps four rows in flight; a layer
+// of 32 outputs then has two groups for its epilogues (rows in turn, row pairs
+// for the pooled output), one of 16 outputs one (the denoised frame's head
+// sums a tile's rows in order).
+template <int kCout, int kLoad>
+struct Roles {
+    static constexpr int kEpiGroups = kLoad == 0 && kCout == 32 ? 2 : 1;
+    static constexpr int kLoadGroups = kLoad == 0 ? 1 : 2;
+    static constexpr int kFirstLoader = kEpiGroups * kGroup;   // threads
+    static_assert(kFirstLoader + kLoadGroups * kGroup <= kMmaWarp * 32, "room for the loaders");
+};
+
 // Bound by HBM: every input row of a strip is read once (and 2 more at each
-// end of a run), every output written once in 32-byte sectors.  Before, a CTA
-// of 128 threads did copy, MMAs and epilogue of a row in turn, at ~6 us a row
-// (four CTAs an SM) for 16 KB moved; with the roles apart four rows are in flight
-// per CTA (two CTAs an SM) and the MMAs of a row overlap the epilogue of the
-// ones before.  Times before and after at launch_fwd.
-template <int kCin, int kCout, int kLoad>
+// end of a run), every output written once in 32-byte sectors.  An M = 128, K =
+// 16 MMA with both operands in shared memory takes ~50 cycles for N up to 64
+// and 59 for N = 96 (its A operand is what it reads), so one MMA for three
+// output rows takes a row 7 instead of 18 of them.  Times at launch_fwd.
+template <int kCin, int kCout, int kLoad, bool kPool>
 __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
     static_assert(kCin % 16 == 0 && (kCout == 16 || kCout == 32), "channel counts");
+    using R = Roles<kCout, kLoad>;
     constexpr int kG = kCin / 8;                         // 16-byte columns per pixel
     constexpr int kColBytes = col_bytes(kCin);
     constexpr int kSlot = kG * kColBytes;                // one halo row
     constexpr int kW = wimage_bytes(kCin, kCout);
-    constexpr uint32_t kIdesc = umma::idesc_bf16(128, kCout, 0, 0);
+    constexpr int kN = 3 * kCout;                        // columns of the weight image
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* s_w = smem + kSlots * kSlot;
     __shared__ __align__(8) uint64_t s_full[kSlots], s_empty[kSlots];        // a row has landed; its MMAs are done
     __shared__ __align__(8) uint64_t s_afull[kAccs], s_aempty[kAccs];        // an accumulator is done; it was read
     __shared__ uint32_t s_taddr;
     __shared__ float s_bias[kCout];
-    constexpr bool kPool = kCin == 16 && kCout == 32;   // the pooled output (conv1 of the denoiser)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     if (tid == 0) {
         for (int k = 0; k < kSlots; ++k) {
-            mbar_init(&s_full[k], kLoaders);
+            mbar_init(&s_full[k], kGroup);
             mbar_init(&s_empty[k], 1);
         }
         for (int k = 0; k < kAccs; ++k) {
             mbar_init(&s_afull[k], 1);
-            mbar_init(&s_aempty[k], kEpiWarps * 32);
+            mbar_init(&s_aempty[k], kGroup);
         }
         mbar_fence_init();
     }
-    if (warp == kMmaWarp) umma::tmem_alloc(&s_taddr, kAccs * 32);
+    if (warp == kMmaWarp) umma::tmem_alloc(&s_taddr, kAccs * kCout);
     pdl_wait();   // launched as a programmatic dependent: nothing above touches global memory
     // weights: the packed image, copied verbatim; the bias
     for (int i = tid; i < kW / 16; i += kFwdThreads)
@@ -193,16 +210,16 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
     ConvRun r;
     bool failed = false;
 
-    if (warp >= kEpiWarps && warp < kMmaWarp) {
-        // ---- load: entry e of the ring (the run's rows y0 - 1 .. y1, then the next run's) by group e & 1
-        const int lt = (tid - kEpiWarps * 32) % kLoaders;
-        const uint32_t group = (uint32_t)((tid - kEpiWarps * 32) / kLoaders);
+    if (tid >= R::kFirstLoader && tid < R::kFirstLoader + R::kLoadGroups * kGroup) {
+        // ---- load: entries of the ring are the run's rows y0 - 1 .. y1, then the next run's; entry e by
+        // group e % kLoadGroups
+        const int lt = (tid - R::kFirstLoader) % kGroup;
+        const uint32_t group = (uint32_t)((tid - R::kFirstLoader) / kGroup);
         uint32_t e = 0;
-        int pending = -1;   // slot of this group's copied row that is not announced yet
         while (!failed && runs.next(r)) {
-            for (int yy = r.y0 - 1; yy <= r.y1 && !failed; ++yy, ++e) {
-                if ((e & 1u) != group) continue;
-                const int slot = (int)(e % kSlots);
+            for (int yy = r.y0 - 1; yy <= r.y1; ++yy, ++e) {
+                if (R::kLoadGroups > 1 && e % R::kLoadGroups != group) continue;
+                const uint32_t slot = e % kSlots;
                 if (e >= kSlots && !mbar_wait_suspend(&s_empty[slot], (e / kSlots - 1u) & 1u)) {
                     failed = true;
                     break;
@@ -211,29 +228,28 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
                 const bool row_in = yy >= 0 && yy < a.h;
                 const __nv_bfloat16* rowp = a.x + ((size_t)r.n * a.h + (row_in ? yy : 0)) * a.w * kCin;
                 if (kLoad == 0) {
-                    // copied asynchronously; announced once the group's next row is on its way
-                    for (int q = lt; q < 130 * kG; q += kLoaders) {
+                    // copied asynchronously; announced once kAhead more rows are on their way
+                    for (int q = lt; q < 130 * kG; q += kGroup) {
                         const int hp = q / kG, g = q - hp * kG, x = r.x0 - 1 + hp;
                         const bool in = row_in && x >= 0 && x < a.w;
                         cp_async16(dst + g * kColBytes + hp * 16, in ? rowp + (size_t)x * kCin + g * 8 : a.x, in ? 16u : 0u);
                     }
                     cp_async_commit();
-                    if (pending >= 0) {
-                        cp_async_wait_all_but_one();
+                    if (e >= kAhead) {
+                        cp_async_wait_but<kAhead>();
                         umma::fence_smem_to_async();
-                        mbar_arrive(&s_full[pending]);
+                        mbar_arrive(&s_full[(e - kAhead) % kSlots]);
                     }
-                    pending = slot;
                 } else {
                     // x + the 2x nearest upsampling of xh (FP32 sum rounded to bf16): all of a
                     // thread's granules loaded before the first is stored
-                    constexpr int kPer = (130 * kG + kLoaders - 1) / kLoaders;
+                    constexpr int kPer = (130 * kG + kGroup - 1) / kGroup;
                     const int hh = a.h >> 1, hw = a.w >> 1;
                     const __nv_bfloat16* hrow = a.xh + ((size_t)r.n * hh + (row_in ? min(yy >> 1, hh - 1) : 0)) * hw * kCin;
                     uint4 v[kPer], u[kPer];
 #pragma unroll
                     for (int k = 0; k < kPer; ++k) {
-                        const int q = lt + k * kLoaders, hp = q / kG, g = q - hp * kG, x = r.x0 - 1 + hp;
+                        const int q = lt + k * kGroup, hp = q / kG, g = q - hp * kG, x = r.x0 - 1 + hp;
                         v[k] = u[k] = make_uint4(0u, 0u, 0u, 0u);
                         if (row_in && x >= 0 && x < a.w && q < 130 * kG) {
                             v[k] = __ldg(reinterpret_cast<const uint4*>(rowp + (size_t)x * kCin) + g);
@@ -242,7 +258,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
                     }
 #pragma unroll
                     for (int k = 0; k < kPer; ++k) {
-                        const int q = lt + k * kLoaders, hp = q / kG, g = q - hp * kG;
+                        const int q = lt + k * kGroup, hp = q / kG, g = q - hp * kG;
                         if (q < 130 * kG) *reinterpret_cast<uint4*>(dst + g * kColBytes + hp * 16) = bf16x8_add(v[k], u[k]);
                     }
                     umma::fence_smem_to_async();
@@ -250,81 +266,100 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
                 }
             }
         }
-        cp_async_wait_all();
-        if (pending >= 0) {
+        if (kLoad == 0) {   // the rows not announced yet
+            cp_async_wait_all();
             umma::fence_smem_to_async();
-            mbar_arrive(&s_full[pending]);
+            for (uint32_t k = e > kAhead ? e - kAhead : 0u; k < e; ++k) mbar_arrive(&s_full[k % kSlots]);
         }
     } else if (warp == kMmaWarp) {
         // ---- multiply: one thread
         if (lane == 0) {
             const uint32_t halo_base = smem_u32(smem), w_base = smem_u32(s_w);
-            uint32_t e = 0, m = 0;   // ring entry of the row above; output rows so far
+            uint32_t e = 0, m = 0;   // ring entry; output rows of earlier runs
+            // the MMA of K-step kb of tap column kx into the accumulators of output rows j .. j + c - 1
+            // (ring positions), the weights' columns starting at block nb (0: ky = 2)
+            auto mma_rows = [&](uint32_t slot, int kx, int kb, uint32_t j, uint32_t c, uint32_t nb, uint32_t accumulate) {
+                const uint64_t ad = umma::smem_desc(slot + (uint32_t)(2 * kb * kColBytes + kx * 16), (uint32_t)kColBytes, 128u);
+                const uint32_t k8 = (uint32_t)((kx * kCin + kb * 16) >> 3);
+                while (c) {
+                    const uint32_t p = j % kAccs, n = min(c, (uint32_t)kAccs - p);   // up to the ring's end
+                    const uint64_t bd = umma::smem_desc(w_base + k8 * (uint32_t)(kN * 16) + nb * (uint32_t)(kCout * 16),
+                                                        (uint32_t)(kN * 16), 128u);
+                    umma::mma_bf16(taddr + p * (uint32_t)kCout, ad, bd,
+                                   umma::idesc_bf16(128, kCout, 0, 0) + ((n - 1u) * (uint32_t)(kCout >> 3) << 17), accumulate);
+                    j += n;
+                    nb += n;
+                    c -= n;
+                }
+            };
             while (!failed && runs.next(r)) {
-                for (int y = r.y0; y < r.y1; ++y, ++e, ++m) {
-                    bool ok = true;
-                    for (uint32_t k = y == r.y0 ? 0u : 2u; k < 3u && ok; ++k)
-                        ok = mbar_wait_suspend(&s_full[(e + k) % kSlots], ((e + k) / kSlots) & 1u);
-                    const uint32_t acc = m % kAccs;
-                    if (ok && m >= kAccs) ok = mbar_wait_suspend(&s_aempty[acc], (m / kAccs - 1u) & 1u);
+                const int rows = r.y1 - r.y0;
+                for (int i = -1; i <= rows; ++i, ++e) {   // input row y0 + i: output rows i - 1, i, i + 1 of the run
+                    bool ok = mbar_wait_suspend(&s_full[e % kSlots], (e / kSlots) & 1u);
+                    const bool fresh = i + 1 < rows;      // row i + 1 gets its first terms
+                    const uint32_t mf = m + (uint32_t)(i + 1);
+                    if (ok && fresh && mf >= kAccs) ok = mbar_wait_suspend(&s_aempty[mf % kAccs], (mf / kAccs - 1u) & 1u);
                     if (!ok) {
                         failed = true;
                         break;
                     }
                     umma::fence_after_sync();
-                    uint32_t accumulate = 0;
-#pragma unroll
-                    for (int ky = 0; ky < 3; ++ky) {
-                        const uint32_t slot = halo_base + ((e + (uint32_t)ky) % kSlots) * (uint32_t)kSlot;
-#pragma unroll
-                        for (int kx = 0; kx < 3; ++kx) {
-#pragma unroll
-                            for (int kb = 0; kb < kCin / 16; ++kb) {
-                                const uint64_t ad = umma::smem_desc(slot + (uint32_t)(2 * kb * kColBytes + kx * 16),
-                                                                    (uint32_t)kColBytes, 128u);
-                                const int k0 = (ky * 3 + kx) * kCin + kb * 16;
-                                const uint64_t bd = umma::smem_desc(w_base + (uint32_t)((k0 >> 3) * kCout * 16),
-                                                                    (uint32_t)(kCout * 16), 128u);
-                                umma::mma_bf16(taddr + acc * 32u, ad, bd, kIdesc, accumulate);
-                                accumulate = 1;
-                            }
-                        }
+                    const int lo = max(i - 1, 0), hi = min(i + 1, rows - 1);
+                    const uint32_t slot = halo_base + (e % kSlots) * (uint32_t)kSlot;
+                    const uint32_t j0 = m + (uint32_t)lo, c = (uint32_t)(hi - lo + 1), nb = (uint32_t)(lo - (i - 1));
+                    if (fresh) {
+                        mma_rows(slot, 0, 0, j0, c - 1u, nb, 1u);
+                        mma_rows(slot, 0, 0, mf, 1u, 2u, 0u);
+                    } else {
+                        mma_rows(slot, 0, 0, j0, c, nb, 1u);
                     }
-                    umma::commit(&s_empty[e % kSlots]);   // this row was the last to read the row above it
-                    umma::commit(&s_afull[acc]);
-                }
-                if (!failed) {   // the run's last two halo rows
+#pragma unroll
+                    for (int k = 1; k < 3 * (kCin / 16); ++k) mma_rows(slot, k / (kCin / 16), k % (kCin / 16), j0, c, nb, 1u);
                     umma::commit(&s_empty[e % kSlots]);
-                    umma::commit(&s_empty[(e + 1u) % kSlots]);
-                    e += 2u;
+                    if (i >= 1) umma::commit(&s_afull[(m + (uint32_t)(i - 1)) % kAccs]);
                 }
+                m += (uint32_t)rows;
             }
             // every MMA of this CTA, and the last commit's arrival, is done before its shared memory and TMEM go
-            if (!failed && m > 0 && !mbar_wait_suspend(&s_empty[(e - 1u) % kSlots], ((e - 1u) / kSlots) & 1u)) failed = true;
+            if (!failed && m > 0) {
+                if (!mbar_wait_suspend(&s_empty[(e - 1u) % kSlots], ((e - 1u) / kSlots) & 1u)) failed = true;
+                if (!mbar_wait_suspend(&s_afull[(m - 1u) % kAccs], ((m - 1u) / kAccs) & 1u)) failed = true;
+            }
         }
         __syncwarp();
-    } else {
-        // ---- epilogue: thread t holds pixel x0 + t of a row
+    } else if (tid < R::kFirstLoader) {
+        // ---- epilogue: thread t of a group holds pixel x0 + t of a row (its TMEM lane: warp % 4)
+        const uint32_t group = (uint32_t)(tid / kGroup);
+        const int t = tid % kGroup;
         uint32_t m = 0;
         float err_sum = 0.0f, err_cnt = 0.0f;   // head mode: this thread's column of the band, in row order
         uint32_t even[kPool ? 16 : 1];          // the bf16 outputs of the even row above (pooled output)
         while (!failed && runs.next(r)) {
-            const int x = r.x0 + tid;
+            const int x = r.x0 + t;
+            const bool in = x < a.w;
             for (int y = r.y0; y < r.y1; ++y, ++m) {
+                if (R::kEpiGroups > 1 && ((m >> (kPool ? 1 : 0)) & 1u) != group) continue;
                 const uint32_t acc = m % kAccs;
                 const size_t o = ((size_t)r.n * a.h + y) * a.w + x;
+                // what the epilogue reads from memory comes while the row is multiplied
+                constexpr int kMaskQ = kPool ? 1 : kCout / 8;
+                uint4 mask[kMaskQ], xv = make_uint4(0u, 0u, 0u, 0u);
+                if (!kPool && a.mask && in) {
+#pragma unroll
+                    for (int q = 0; q < kMaskQ; ++q) mask[q] = __ldg(reinterpret_cast<const uint4*>(a.mask + o * kCout) + q);
+                }
+                if (kCout == 16 && a.head_x && in) xv = __ldg(reinterpret_cast<const uint4*>(a.head_x + o * 16));
                 if (!mbar_wait_suspend(&s_afull[acc], (m / kAccs) & 1u)) {
                     failed = true;
                     break;
                 }
                 umma::fence_after_sync();
-                const uint32_t acc_addr = taddr + acc * 32u + ((uint32_t)(warp * 32) << 16);
+                const uint32_t acc_addr = taddr + acc * (uint32_t)kCout + ((uint32_t)((warp & 3) * 32) << 16);
                 float v[32];
                 if (kCout == 32) umma::tmem_ld32(acc_addr, *reinterpret_cast<float(*)[32]>(v));
                 else umma::tmem_ld16(acc_addr, *reinterpret_cast<float(*)[16]>(v));
                 umma::fence_before_sync();
                 mbar_arrive(&s_aempty[acc]);
-                uint32_t pk[kCout / 2];
                 if (a.bias) {
 #pragma unroll
                     for (int c = 0; c < kCout; ++c) v[c] += s_bias[c];
@@ -333,87 +368,85 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
 #pragma unroll
                     for (int c = 0; c < kCout; ++c) v[c] = fmaxf(v[c], 0.0f);
                 }
-                if (x < a.w) {
-                    if (a.mask) {
-                        const uint4* mp = reinterpret_cast<const uint4*>(a.mask + o * kCout);
+                if (!kPool && a.mask && in) {
 #pragma unroll
-                        for (int q = 0; q < kCout / 8; ++q) {
-                            const uint4 mv = __ldg(mp + q);
-                            const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(&mv);
+                    for (int q = 0; q < kMaskQ; ++q) {
+                        const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(&mask[q]);
 #pragma unroll
-                            for (int i = 0; i < 8; ++i)
-                                if (!(__bfloat162float(mb[i]) > 0.0f)) v[q * 8 + i] = 0.0f;
-                        }
-                    }
-                    if (kCout == 16 && a.head_x) {
-                        // the denoised frame's pixel (head_rgba of the output step) and its error estimate
-                        const uint4 xv = __ldg(reinterpret_cast<const uint4*>(a.head_x + o * 16));
-                        const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(&xv);
-                        const float4 px = make_float4(__bfloat162float(xb[5]) + v[0], __bfloat162float(xb[6]) + v[1],
-                                                      __bfloat162float(xb[7]) + v[2], __bfloat162float(xb[3]) + v[3]);
-                        __half2 h01 = __floats2half2_rn(px.x, px.y), h23 = __floats2half2_rn(px.z, px.w);
-                        uint2 pk2;
-                        pk2.x = *reinterpret_cast<uint32_t*>(&h01);
-                        pk2.y = *reinterpret_cast<uint32_t*>(&h23);
-                        reinterpret_cast<uint2*>(a.head_out16)[o] = pk2;
-                        err_sum += fmaxf(v[4], 0.0f);
-                        err_cnt += 1.0f;
+                        for (int i = 0; i < 8; ++i)
+                            if (!(__bfloat162float(mb[i]) > 0.0f)) v[q * 8 + i] = 0.0f;
                     }
                 }
-#pragma unroll
-                for (int i = 0; i < kCout / 2; ++i) {
-                    __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-                    pk[i] = *reinterpret_cast<uint32_t*>(&b2);
+                if (kCout == 16 && a.head_x && in) {
+                    // the denoised frame's pixel (head_rgba of the output step) and its error estimate
+                    const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(&xv);
+                    const float4 px = make_float4(__bfloat162float(xb[5]) + v[0], __bfloat162float(xb[6]) + v[1],
+                                                  __bfloat162float(xb[7]) + v[2], __bfloat162float(xb[3]) + v[3]);
+                    __half2 h01 = __floats2half2_rn(px.x, px.y), h23 = __floats2half2_rn(px.z, px.w);
+                    uint2 pk2;
+                    pk2.x = *reinterpret_cast<uint32_t*>(&h01);
+                    pk2.y = *reinterpret_cast<uint32_t*>(&h23);
+                    reinterpret_cast<uint2*>(a.head_out16)[o] = pk2;
+                    err_sum += fmaxf(v[4], 0.0f);
+                    err_cnt += 1.0f;
                 }
-                if (a.out_bf16 && x < a.w) {
-                    uint4* op = reinterpret_cast<uint4*>(a.out_bf16 + o * kCout);
-#pragma unroll
-                    for (int q = 0; q < kCout / 16; ++q) {
-                        const uint4 lo = make_uint4(pk[8 * q], pk[8 * q + 1], pk[8 * q + 2], pk[8 * q + 3]);
-                        const uint4 hi = make_uint4(pk[8 * q + 4], pk[8 * q + 5], pk[8 * q + 6], pk[8 * q + 7]);
-                        if (a.out_wide) {
-                            st_global32(op + 2 * q, lo, hi);
-                        } else {
-                            op[2 * q] = lo;
-                            op[2 * q + 1] = hi;
-                        }
-                    }
-                }
-                if (a.out_f32 && x < a.w) {
+                if (a.out_f32 && in) {
                     float4* op = reinterpret_cast<float4*>(a.out_f32 + o * kCout);
 #pragma unroll
                     for (int q = 0; q < kCout / 4; ++q)
                         op[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                 }
-                if (kPool && a.pool_out) {
-                    // 2x2 average of the bf16 outputs: (0 + (y, x) + (y, x + 1) + (y + 1, x) + (y + 1, x + 1)) * 0.25,
-                    // the right neighbour's by lane shuffles (runs hold whole row pairs)
-                    if ((y & 1) == 0) {
+                if (a.out_bf16 || kPool) {
+                    uint32_t pk[kCout / 2];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) even[i] = pk[i];
-                    } else {
-                        const bool write = (x & 1) == 0 && x < a.w;
-                        uint4* dp = reinterpret_cast<uint4*>(
-                            a.pool_out + (((size_t)r.n * (a.h >> 1) + (y >> 1)) * (a.w >> 1) + (x >> 1)) * kCout);
+                    for (int i = 0; i < kCout / 2; ++i) {
+                        __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                        pk[i] = *reinterpret_cast<uint32_t*>(&b2);
+                    }
+                    if (in) {
+                        uint4* op = reinterpret_cast<uint4*>(a.out_bf16 + o * kCout);
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            uint32_t res[4];
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const uint32_t up = even[4 * q + i], down = pk[4 * q + i];
-                                const uint32_t t4[4] = {up, __shfl_xor_sync(0xffffffffu, up, 1), down,
-                                                        __shfl_xor_sync(0xffffffffu, down, 1)};
-                                float acc0 = 0.0f, acc1 = 0.0f;
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) {
-                                    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&t4[k]));
-                                    acc0 += f.x;
-                                    acc1 += f.y;
-                                }
-                                __nv_bfloat162 r2 = __floats2bfloat162_rn(0.25f * acc0, 0.25f * acc1);
-                                res[i] = *reinterpret_cast<uint32_t*>(&r2);
+                        for (int q = 0; q < kCout / 16; ++q) {
+                            const uint4 lo = make_uint4(pk[8 * q], pk[8 * q + 1], pk[8 * q + 2], pk[8 * q + 3]);
+                            const uint4 hi = make_uint4(pk[8 * q + 4], pk[8 * q + 5], pk[8 * q + 6], pk[8 * q + 7]);
+                            if (a.out_wide) {
+                                st_global32(op + 2 * q, lo, hi);
+                            } else {
+                                op[2 * q] = lo;
+                                op[2 * q + 1] = hi;
                             }
-                            if (write) dp[q] = make_uint4(res[0], res[1], res[2], res[3]);
+                        }
+                    }
+                    if constexpr (kPool) {
+                        // 2x2 average of the bf16 outputs: (0 + (y, x) + (y, x + 1) + (y + 1, x) + (y + 1, x + 1)) * 0.25,
+                        // the right neighbour's by lane shuffles (runs hold whole row pairs)
+                        if ((y & 1) == 0) {
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) even[i] = pk[i];
+                        } else {
+                            const bool write = (x & 1) == 0 && in;
+                            uint4* dp = reinterpret_cast<uint4*>(
+                                a.pool_out + (((size_t)r.n * (a.h >> 1) + (y >> 1)) * (a.w >> 1) + (x >> 1)) * kCout);
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                uint32_t res[4];
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    const uint32_t up = even[4 * q + i], down = pk[4 * q + i];
+                                    const uint32_t t4[4] = {up, __shfl_xor_sync(0xffffffffu, up, 1), down,
+                                                            __shfl_xor_sync(0xffffffffu, down, 1)};
+                                    float acc0 = 0.0f, acc1 = 0.0f;
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k) {
+                                        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&t4[k]));
+                                        acc0 += f.x;
+                                        acc1 += f.y;
+                                    }
+                                    __nv_bfloat162 r2 = __floats2bfloat162_rn(0.25f * acc0, 0.25f * acc1);
+                                    res[i] = *reinterpret_cast<uint32_t*>(&r2);
+                                }
+                                if (write) dp[q] = make_uint4(res[0], res[1], res[2], res[3]);
+                            }
                         }
                     }
                 }
@@ -425,8 +458,8 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
                         err_sum += __shfl_xor_sync(0xffffffffu, err_sum, off);
                         err_cnt += __shfl_xor_sync(0xffffffffu, err_cnt, off);
                     }
-                    const int tx = (r.x0 >> 4) + (tid >> 4);
-                    if ((tid & 15) == 0 && tx < a.tiles_x && err_cnt > 0.0f) {
+                    const int tx = (r.x0 >> 4) + (t >> 4);
+                    if ((t & 15) == 0 && tx < a.tiles_x && err_cnt > 0.0f) {
                         const int band = (y + a.row_offset) / 16;
                         const int ty = (a.h + a.row_offset) / 16 - 1 - band;   // GL tile row of this band
                         const uint32_t tile = (uint32_t)(ty * a.tiles_x + tx);
@@ -439,12 +472,12 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
             }
         }
     }
-    if (failed && (lane == 0 || warp != kMmaWarp)) atomicOr(a.err, 1u);
+    if (failed) atomicOr(a.err, 1u);
     umma::fence_before_sync();
     __syncthreads();
     if (warp == kMmaWarp) {
         umma::fence_after_sync();
-        umma::tmem_dealloc(taddr, kAccs * 32);
+        umma::tmem_dealloc(taddr, kAccs * kCout);
     }
 }
 
@@ -674,22 +707,12 @@ __global__ void pack_weights_kernel(const float* __restrict__ w, int cin, int co
     const int total = 9 * cin * cout;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int co = i % cout, ci = (i / cout) % cin, tap = i / (cin * cout);
-        const float v = w[i];
-        int k, nn, cdim;
-        if (!transposed) {
-            k = tap * cin + ci;
-            nn = co;
-            cdim = cout;
-        } else {
-            k = (8 - tap) * cout + co;
-            nn = ci;
-            cdim = cin;
-        }
-        *reinterpret_cast<__nv_bfloat16*>(image + wimage_offset(k, nn, cdim)) = __float2bfloat16_rn(v);
+        const int at = transposed ? wimage_offset(8 - tap, co, ci, cout, cin) : wimage_offset(tap, ci, co, cin, cout);
+        *reinterpret_cast<__nv_bfloat16*>(image + at) = __float2bfloat16_rn(w[i]);
     }
 }
 
-template <int kCin, int kCout, int kLoad>
+template <int kCin, int kCout, int kLoad, bool kPool = false>
 static int launch_fwd_t(ConvArgs a, cudaStream_t s) {
     const long strips = (long)a.n * ((a.w + 127) / 128);
     const long units = strips * ((a.h + a.row_offset + a.unit_rows - 1) / a.unit_rows);
@@ -697,13 +720,13 @@ static int launch_fwd_t(ConvArgs a, cudaStream_t s) {
     a.out_wide = (reinterpret_cast<uintptr_t>(a.out_bf16) & 31u) == 0u ? 1 : 0;
     static bool attr = false;
     if (!attr) {
-        cudaFuncSetAttribute(conv_fwd_kernel<kCin, kCout, kLoad>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(conv_fwd_kernel<kCin, kCout, kLoad, kPool>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
         attr = true;
     }
     // two CTAs an SM; on small images one unit each at most
     const long ctas = 2L * a.max_sms;
-    launch_pdl(conv_fwd_kernel<kCin, kCout, kLoad>, dim3((unsigned)(units < ctas ? units : ctas)), dim3(kFwdThreads), smem,
+    launch_pdl(conv_fwd_kernel<kCin, kCout, kLoad, kPool>, dim3((unsigned)(units < ctas ? units : ctas)), dim3(kFwdThreads), smem,
                s, a);
     return 1;
 }
@@ -730,6 +753,7 @@ static int launch_wgrad_t(const WgradArgs& a, int max_ctas, cudaStream_t s) {
 int launch_fwd(int cin, int cout, int load_mode, const ConvArgs& a, cudaStream_t s) {
     if (a.n <= 0 || a.h <= 0 || a.w <= 0) return 0;
     if (load_mode == 0) {
+        if (cin == 16 && cout == 32 && a.pool_out) return launch_fwd_t<16, 32, 0, true>(a, s);
         if (cin == 16 && cout == 32) return launch_fwd_t<16, 32, 0>(a, s);
         if (cin == 32 && cout == 32) return launch_fwd_t<32, 32, 0>(a, s);
         if (cin == 32 && cout == 16) return launch_fwd_t<32, 16, 0>(a, s);

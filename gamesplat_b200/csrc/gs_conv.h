@@ -60,9 +60,11 @@ int launch_fwd(int cin, int cout, int load_mode, const ConvArgs& a, cudaStream_t
 int launch_wgrad(int cin, int cout, int load_mode, const WgradArgs& a, int max_ctas, cudaStream_t s);
 // transposed: the image of the layer's input gradient
 int launch_pack_weights(const float* w, int cin, int cout, int transposed, uint8_t* image, cudaStream_t s);
-// Byte offset of weight (k = tap * cin + ci, n = co) in the K-major B image.
-__host__ __device__ constexpr int wimage_offset(int k, int n, int cout) {
-    return (k >> 3) * (cout * 16) + (n >> 3) * 128 + (n & 7) * 16 + (k & 7) * 2;
+// Byte offset of weight (tap = 3 ky + kx, ci, co) in the K-major B image: K = 3 kx x cin, N = 3 x cout with the
+// columns of ky = 2, 1, 0 side by side.
+__host__ __device__ constexpr int wimage_offset(int tap, int ci, int co, int cin, int cout) {
+    const int k = (tap % 3) * cin + ci, n = (2 - tap / 3) * cout + co;
+    return (k >> 3) * (3 * cout * 16) + (n >> 3) * 128 + (n & 7) * 16 + (k & 7) * 2;
 }
 size_t weight_image_bytes(int cin, int cout);
 

@@ -383,9 +383,9 @@ __global__ void update_pack_kernel(ParamImages im, float* __restrict__ w, const 
         if (k >= 9 * L.cin * L.cout) continue;   // a bias
         const int co = k % L.cout, ci = (k / L.cout) % L.cin, tap = k / (L.cin * L.cout);
         const __nv_bfloat16 h = __float2bfloat16_rn(wi);
-        *reinterpret_cast<__nv_bfloat16*>(L.image + conv::wimage_offset(tap * L.cin + ci, co, L.cout)) = h;
+        *reinterpret_cast<__nv_bfloat16*>(L.image + conv::wimage_offset(tap, ci, co, L.cin, L.cout)) = h;
         // cut_cout: the output channel whose gradient stops at this layer
-        *reinterpret_cast<__nv_bfloat16*>(L.image_t + conv::wimage_offset((8 - tap) * L.cout + co, ci, L.cin)) =
+        *reinterpret_cast<__nv_bfloat16*>(L.image_t + conv::wimage_offset(8 - tap, co, ci, L.cout, L.cin)) =
             co == L.cut_cout ? __float2bfloat16_rn(0.0f) : h;
     }
 }

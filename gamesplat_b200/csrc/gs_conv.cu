@@ -50,7 +50,9 @@ constexpr int kFwdThreads = (kMmaWarp + 1) * 32;
 constexpr int kGroup = 128;                 // threads that load a row, or that read one back
 constexpr int kSlots = 8;                   // halo rows in the ring
 constexpr int kAhead = 3;                   // rows copied behind the one announced next
-constexpr int kAccs = 8;                    // TMEM accumulators of Cout columns
+constexpr uint32_t kAccs = 8;               // TMEM accumulators of Cout columns
+constexpr uint32_t kDone = 16;              // barriers of finished rows: a reader of accumulators is at most kAccs
+                                            // output rows, so kAccs + 2 ring entries, behind the MMAs
 
 // Dynamic shared memory of the forward kernel: the halo rows and the weight image.
 __host__ __device__ constexpr int fwd_smem_bytes(int cin, int cout) {
@@ -82,8 +84,10 @@ __device__ __forceinline__ bool mbar_wait_suspend(uint64_t* bar, uint32_t phase)
     }
     return false;
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+// One arrival for a warp, behind what all its lanes did before.
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t* bar) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 // 32 bytes to global memory (32-byte aligned).
 __device__ __forceinline__ void st_global32(void* p, const uint4& a, const uint4& b) {
@@ -178,21 +182,19 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
     constexpr int kN = 3 * kCout;                        // columns of the weight image
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* s_w = smem + kSlots * kSlot;
-    __shared__ __align__(8) uint64_t s_full[kSlots], s_empty[kSlots];        // a row has landed; its MMAs are done
-    __shared__ __align__(8) uint64_t s_afull[kAccs], s_aempty[kAccs];        // an accumulator is done; it was read
+    // a row has landed; its MMAs are done (its slot is free and the output row above it complete: one commit, which
+    // takes the tensor core ~70 cycles, says both); an accumulator was read
+    __shared__ __align__(8) uint64_t s_full[kSlots], s_done[kDone], s_aempty[kAccs];
     __shared__ uint32_t s_taddr;
-    __shared__ float s_bias[kCout];
+    __shared__ __align__(16) float s_bias[kCout];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     if (tid == 0) {
         for (int k = 0; k < kSlots; ++k) {
-            mbar_init(&s_full[k], kGroup);
-            mbar_init(&s_empty[k], 1);
+            mbar_init(&s_full[k], kGroup / 32);
         }
-        for (int k = 0; k < kAccs; ++k) {
-            mbar_init(&s_afull[k], 1);
-            mbar_init(&s_aempty[k], kGroup);
-        }
+        for (uint32_t k = 0; k < kDone; ++k) mbar_init(&s_done[k], 1);
+        for (uint32_t k = 0; k < kAccs; ++k) mbar_init(&s_aempty[k], kGroup / 32);
         mbar_fence_init();
     }
     if (warp == kMmaWarp) umma::tmem_alloc(&s_taddr, kAccs * kCout);
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
             for (int yy = r.y0 - 1; yy <= r.y1; ++yy, ++e) {
                 if (R::kLoadGroups > 1 && e % R::kLoadGroups != group) continue;
                 const uint32_t slot = e % kSlots;
-                if (e >= kSlots && !mbar_wait_suspend(&s_empty[slot], (e / kSlots - 1u) & 1u)) {
+                if (e >= kSlots && !mbar_wait_suspend(&s_done[(e - kSlots) % kDone], ((e - kSlots) / kDone) & 1u)) {
                     failed = true;
                     break;
                 }
@@ -238,7 +240,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
                     if (e >= kAhead) {
                         cp_async_wait_but<kAhead>();
                         umma::fence_smem_to_async();
-                        mbar_arrive(&s_full[(e - kAhead) % kSlots]);
+                        mbar_arrive_warp(&s_full[(e - kAhead) % kSlots]);
                     }
                 } else {
                     // x + the 2x nearest upsampling of xh (FP32 sum rounded to bf16): all of a
@@ -262,94 +264,95 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
                         if (q < 130 * kG) *reinterpret_cast<uint4*>(dst + g * kColBytes + hp * 16) = bf16x8_add(v[k], u[k]);
                     }
                     umma::fence_smem_to_async();
-                    mbar_arrive(&s_full[slot]);
+                    mbar_arrive_warp(&s_full[slot]);
                 }
             }
         }
         if (kLoad == 0) {   // the rows not announced yet
             cp_async_wait_all();
             umma::fence_smem_to_async();
-            for (uint32_t k = e > kAhead ? e - kAhead : 0u; k < e; ++k) mbar_arrive(&s_full[k % kSlots]);
+            for (uint32_t k = e > kAhead ? e - kAhead : 0u; k < e; ++k) mbar_arrive_warp(&s_full[k % kSlots]);
         }
     } else if (warp == kMmaWarp) {
-        // ---- multiply: one thread
-        if (lane == 0) {
-            const uint32_t halo_base = smem_u32(smem), w_base = smem_u32(s_w);
-            uint32_t e = 0, m = 0;   // ring entry; output rows of earlier runs
-            // the MMA of K-step kb of tap column kx into the accumulators of output rows j .. j + c - 1
-            // (ring positions), the weights' columns starting at block nb (0: ky = 2)
-            auto mma_rows = [&](uint32_t slot, int kx, int kb, uint32_t j, uint32_t c, uint32_t nb, uint32_t accumulate) {
-                const uint64_t ad = umma::smem_desc(slot + (uint32_t)(2 * kb * kColBytes + kx * 16), (uint32_t)kColBytes, 128u);
-                const uint32_t k8 = (uint32_t)((kx * kCin + kb * 16) >> 3);
-                while (c) {
-                    const uint32_t p = j % kAccs, n = min(c, (uint32_t)kAccs - p);   // up to the ring's end
-                    const uint64_t bd = umma::smem_desc(w_base + k8 * (uint32_t)(kN * 16) + nb * (uint32_t)(kCout * 16),
-                                                        (uint32_t)(kN * 16), 128u);
-                    umma::mma_bf16(taddr + p * (uint32_t)kCout, ad, bd,
-                                   umma::idesc_bf16(128, kCout, 0, 0) + ((n - 1u) * (uint32_t)(kCout >> 3) << 17), accumulate);
-                    j += n;
-                    nb += n;
-                    c -= n;
+        // ---- multiply: the warp in step, one lane issuing
+        const uint32_t elected = lane == 0 ? 1u : 0u;
+        const uint64_t ad0 = umma::smem_desc(smem_u32(smem), (uint32_t)kColBytes, 128u);
+        const uint64_t bd0 = umma::smem_desc(smem_u32(s_w), (uint32_t)(kN * 16), 128u);
+        uint32_t e = 0, m = 0;   // ring entry; output rows of earlier runs
+        while (!failed && runs.next(r)) {
+            const int rows = r.y1 - r.y0;
+            for (int i = -1; i <= rows; ++i, ++e) {   // input row y0 + i: output rows i - 1, i, i + 1 of the run
+                bool ok = mbar_wait_suspend(&s_full[e % kSlots], (e / kSlots) & 1u);
+                const bool fresh = i + 1 < rows;      // row i + 1 gets its first terms
+                const uint32_t mf = m + (uint32_t)(i + 1);
+                if (ok && fresh && mf >= kAccs) ok = mbar_wait_suspend(&s_aempty[mf % kAccs], (mf / kAccs - 1u) & 1u);
+                if (__any_sync(0xffffffffu, !ok)) {
+                    failed = true;
+                    break;
                 }
-            };
-            while (!failed && runs.next(r)) {
-                const int rows = r.y1 - r.y0;
-                for (int i = -1; i <= rows; ++i, ++e) {   // input row y0 + i: output rows i - 1, i, i + 1 of the run
-                    bool ok = mbar_wait_suspend(&s_full[e % kSlots], (e / kSlots) & 1u);
-                    const bool fresh = i + 1 < rows;      // row i + 1 gets its first terms
-                    const uint32_t mf = m + (uint32_t)(i + 1);
-                    if (ok && fresh && mf >= kAccs) ok = mbar_wait_suspend(&s_aempty[mf % kAccs], (mf / kAccs - 1u) & 1u);
-                    if (!ok) {
-                        failed = true;
-                        break;
-                    }
-                    umma::fence_after_sync();
-                    const int lo = max(i - 1, 0), hi = min(i + 1, rows - 1);
-                    const uint32_t slot = halo_base + (e % kSlots) * (uint32_t)kSlot;
-                    const uint32_t j0 = m + (uint32_t)lo, c = (uint32_t)(hi - lo + 1), nb = (uint32_t)(lo - (i - 1));
-                    if (fresh) {
-                        mma_rows(slot, 0, 0, j0, c - 1u, nb, 1u);
-                        mma_rows(slot, 0, 0, mf, 1u, 2u, 0u);
-                    } else {
-                        mma_rows(slot, 0, 0, j0, c, nb, 1u);
-                    }
+                umma::fence_after_sync();
+                const int lo = max(i - 1, 0), hi = min(i + 1, rows - 1);
+                // accumulators p0 .. of the ring for output rows lo .. hi, the weights' columns from block nb
+                // (0: ky = 2); the rows past the ring's end are a second MMA
+                const uint32_t p0 = (m + (uint32_t)lo) % kAccs, c = (uint32_t)(hi - lo + 1), nb = (uint32_t)(lo - (i - 1));
+                const uint64_t ad = ad0 + (uint64_t)((e % kSlots) * (uint32_t)(kSlot >> 4));
+                auto mma_rows = [&](int k, uint32_t p, uint32_t rows_n, uint32_t block, uint32_t accumulate) {
+                    const int kx = k / (kCin / 16), kb = k % (kCin / 16);
+                    umma::mma_bf16_elect(taddr + p * (uint32_t)kCout,
+                                         ad + (uint64_t)((2 * kb * kColBytes + kx * 16) >> 4),
+                                         bd0 + (uint64_t)(((kx * kCin + kb * 16) >> 3) * kN) + block * (uint32_t)kCout,
+                                         umma::idesc_bf16(128, kCout, 0, 0) + ((rows_n - 1u) * (uint32_t)(kCout >> 3) << 17),
+                                         accumulate, elected);
+                };
+                {   // K-step 0: the fresh row's accumulator is written, the others are added to
+                    const uint32_t old = fresh ? c - 1u : c, c1 = min(old, kAccs - p0), c2 = old - c1;
+                    if (c1) mma_rows(0, p0, c1, nb, 1u);
+                    if (c2) mma_rows(0, 0u, c2, nb + c1, 1u);
+                    if (fresh) mma_rows(0, mf % kAccs, 1u, 2u, 0u);
+                }
+                const uint32_t c1 = min(c, kAccs - p0), c2 = c - c1;
 #pragma unroll
-                    for (int k = 1; k < 3 * (kCin / 16); ++k) mma_rows(slot, k / (kCin / 16), k % (kCin / 16), j0, c, nb, 1u);
-                    umma::commit(&s_empty[e % kSlots]);
-                    if (i >= 1) umma::commit(&s_afull[(m + (uint32_t)(i - 1)) % kAccs]);
+                for (int k = 1; k < 3 * (kCin / 16); ++k) mma_rows(k, p0, c1, nb, 1u);
+                if (c2) {
+#pragma unroll
+                    for (int k = 1; k < 3 * (kCin / 16); ++k) mma_rows(k, 0u, c2, nb + c1, 1u);
                 }
-                m += (uint32_t)rows;
+                umma::commit_elect(&s_done[e % kDone], elected);
             }
-            // every MMA of this CTA, and the last commit's arrival, is done before its shared memory and TMEM go
-            if (!failed && m > 0) {
-                if (!mbar_wait_suspend(&s_empty[(e - 1u) % kSlots], ((e - 1u) / kSlots) & 1u)) failed = true;
-                if (!mbar_wait_suspend(&s_afull[(m - 1u) % kAccs], ((m - 1u) / kAccs) & 1u)) failed = true;
-            }
+            m += (uint32_t)rows;
         }
+        // every MMA of this CTA, and the last commit's arrival, is done before its shared memory and TMEM go
+        if (!failed && e > 0 && !mbar_wait_suspend(&s_done[(e - 1u) % kDone], ((e - 1u) / kDone) & 1u)) failed = true;
         __syncwarp();
     } else if (tid < R::kFirstLoader) {
         // ---- epilogue: thread t of a group holds pixel x0 + t of a row (its TMEM lane: warp % 4)
         const uint32_t group = (uint32_t)(tid / kGroup);
         const int t = tid % kGroup;
-        uint32_t m = 0;
+        uint32_t m = 0, e = 2;   // output rows; the ring entry whose MMAs complete row m
         float err_sum = 0.0f, err_cnt = 0.0f;   // head mode: this thread's column of the band, in row order
         uint32_t even[kPool ? 16 : 1];          // the bf16 outputs of the even row above (pooled output)
         while (!failed && runs.next(r)) {
             const int x = r.x0 + t;
             const bool in = x < a.w;
-            for (int y = r.y0; y < r.y1; ++y, ++m) {
+            uint4 x_next = make_uint4(0u, 0u, 0u, 0u);
+            if (kCout == 16 && a.head_x && in)
+                x_next = __ldg(reinterpret_cast<const uint4*>(a.head_x + (((size_t)r.n * a.h + r.y0) * a.w + x) * 16));
+            for (int y = r.y0; y < r.y1; ++y, ++m, ++e) {
                 if (R::kEpiGroups > 1 && ((m >> (kPool ? 1 : 0)) & 1u) != group) continue;
                 const uint32_t acc = m % kAccs;
                 const size_t o = ((size_t)r.n * a.h + y) * a.w + x;
                 // what the epilogue reads from memory comes while the row is multiplied
                 constexpr int kMaskQ = kPool ? 1 : kCout / 8;
-                uint4 mask[kMaskQ], xv = make_uint4(0u, 0u, 0u, 0u);
+                uint4 mask[kMaskQ];
                 if (!kPool && a.mask && in) {
 #pragma unroll
                     for (int q = 0; q < kMaskQ; ++q) mask[q] = __ldg(reinterpret_cast<const uint4*>(a.mask + o * kCout) + q);
                 }
-                if (kCout == 16 && a.head_x && in) xv = __ldg(reinterpret_cast<const uint4*>(a.head_x + o * 16));
-                if (!mbar_wait_suspend(&s_afull[acc], (m / kAccs) & 1u)) {
+                // (the head's features a row ahead: its rows take the group one after another)
+                const uint4 xv = x_next;
+                if (kCout == 16 && a.head_x && in && y + 1 < r.y1)
+                    x_next = __ldg(reinterpret_cast<const uint4*>(a.head_x + (o + a.w) * 16));
+                if (!mbar_wait_suspend(&s_done[e % kDone], (e / kDone) & 1u)) {
                     failed = true;
                     break;
                 }
@@ -359,22 +362,18 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
                 if (kCout == 32) umma::tmem_ld32(acc_addr, *reinterpret_cast<float(*)[32]>(v));
                 else umma::tmem_ld16(acc_addr, *reinterpret_cast<float(*)[16]>(v));
                 umma::fence_before_sync();
-                mbar_arrive(&s_aempty[acc]);
+                mbar_arrive_warp(&s_aempty[acc]);
                 if (a.bias) {
+                    const float4* sb = reinterpret_cast<const float4*>(s_bias);
 #pragma unroll
-                    for (int c = 0; c < kCout; ++c) v[c] += s_bias[c];
-                }
-                if (a.relu) {
-#pragma unroll
-                    for (int c = 0; c < kCout; ++c) v[c] = fmaxf(v[c], 0.0f);
-                }
-                if (!kPool && a.mask && in) {
-#pragma unroll
-                    for (int q = 0; q < kMaskQ; ++q) {
-                        const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(&mask[q]);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            if (!(__bfloat162float(mb[i]) > 0.0f)) v[q * 8 + i] = 0.0f;
+                    for (int q = 0; q < kCout / 4; ++q) {
+                        const float4 b4 = sb[q];
+                        const float2 lo = __fadd2_rn(make_float2(v[4 * q], v[4 * q + 1]), make_float2(b4.x, b4.y));
+                        const float2 hi = __fadd2_rn(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(b4.z, b4.w));
+                        v[4 * q] = lo.x;
+                        v[4 * q + 1] = lo.y;
+                        v[4 * q + 2] = hi.x;
+                        v[4 * q + 3] = hi.y;
                     }
                 }
                 if (kCout == 16 && a.head_x && in) {
@@ -390,18 +389,33 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
                     err_sum += fmaxf(v[4], 0.0f);
                     err_cnt += 1.0f;
                 }
-                if (a.out_f32 && in) {
+                if (!kPool && a.out_f32 && in) {
                     float4* op = reinterpret_cast<float4*>(a.out_f32 + o * kCout);
 #pragma unroll
-                    for (int q = 0; q < kCout / 4; ++q)
-                        op[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                    for (int q = 0; q < kCout / 4; ++q) {
+                        float f[4] = {v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            if (a.relu) f[i] = fmaxf(f[i], 0.0f);
+                            if (a.mask) {
+                                const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(&mask[q >> 1]);
+                                if (!(__bfloat162float(mb[4 * (q & 1) + i]) > 0.0f)) f[i] = 0.0f;
+                            }
+                        }
+                        op[q] = make_float4(f[0], f[1], f[2], f[3]);
+                    }
                 }
                 if (a.out_bf16 || kPool) {
                     uint32_t pk[kCout / 2];
 #pragma unroll
                     for (int i = 0; i < kCout / 2; ++i) {
+                        // ReLU and mask on the rounded pairs: rounding keeps the sign and zero
                         __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                        if (a.relu) b2 = __hmax2(b2, __floats2bfloat162_rn(0.0f, 0.0f));
                         pk[i] = *reinterpret_cast<uint32_t*>(&b2);
+                        if (!kPool && a.mask)
+                            pk[i] &= __hgt2_mask(reinterpret_cast<const __nv_bfloat162*>(&mask[i >> 2])[i & 3],
+                                                 __floats2bfloat162_rn(0.0f, 0.0f));
                     }
                     if (in) {
                         uint4* op = reinterpret_cast<uint4*>(a.out_bf16 + o * kCout);
@@ -470,6 +484,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
                     err_sum = err_cnt = 0.0f;
                 }
             }
+            e += 2u;
         }
     }
     if (failed) atomicOr(a.err, 1u);

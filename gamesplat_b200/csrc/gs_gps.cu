@@ -39,51 +39,107 @@ __global__ void gps_clear_kernel(unsigned long long* packed, size_t count) {
         packed[i] = 0xFFFFFFFF00000000ull;
 }
 
-__global__ void gps_expand_kernel(GpsParams p, float4* __restrict__ prepared, uint2* __restrict__ work) {
+// A warp takes 32 visible Gaussians: one reservation for all their work items
+// (one atomic a warp: one a Gaussian on the same word was the bound, 363 of the
+// 857 us of a frame of 1M Gaussians at 1280x720), then the warp writes the
+// items together, 32 consecutive ones at a time, their owners found in the
+// prefix sums of the counts.
+__global__ void __launch_bounds__(256) gps_expand_kernel(GpsParams p, float4* __restrict__ prepared,
+                                                         uint2* __restrict__ work) {
     pdl_wait();   // launched as a programmatic dependent of the frame's previous kernel
+    __shared__ uint32_t s_end[8][32];   // per warp: inclusive prefix sums of the items written
     const uint32_t n_vis = p.fc->visible_count;
     const float ss = (float)p.supersample;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n_vis; v += gridDim.x * blockDim.x) {
-        const uint32_t splat_id = p.vis_ids[v];
-        const float4* P = p.projected + (size_t)splat_id * 4;
-        const float4 co = P[0], cr = P[1], cd = P[2], cv = P[3];
-        const float ssf = g_max(ss, 1.0f);
-        const float cov_a = add(cv.x, 0.3f), cov_b = cv.y, cov_c = add(cv.z, 0.3f);
-        const float det = sub(mul(cov_a, cov_c), mul(cov_b, cov_b));
-        const float expected = mul(mul(mul(mul(ssf, ssf), 6.28318530718f), __fsqrt_rn(g_max(det, 0.0f))),
-                                   det_dilog(g_clamp(co.w, 0.0f, 1.0f)));
-        const float ppw = g_max(mul(ssf, ssf), 1.0f);
-        const float scaled = g_max(dv(expected, ppw), 0.0f);
-        uint32_t wic = g_f2u_sat(g_clamp(floorf(scaled), 0.0f, 4294967295.0f));
-        if (hash01(splat_id + 0x9e3779b9u) < g_fract(scaled) && wic < 0xFFFFFFFFu) wic += 1u;
-        if (wic == 0u) continue;
-        const uint32_t base = atomicAdd(&p.fc->gps_work[0], wic);
-        const uint32_t cap = p.max_work_items;
-        if (base >= cap || wic > cap - base) atomicOr(&p.fc->gps_work[1], 1u);
-        if (base >= cap) continue;
-        const uint32_t write_count = min(wic, cap - base);
-        const float l00 = __fsqrt_rn(g_max(cov_a, 1.0e-5f));
-        const float l10 = dv(cov_b, l00);
-        const float l11 = __fsqrt_rn(g_max(sub(cov_c, mul(l10, l10)), 1.0e-5f));
-        const float alpha = g_clamp(co.w, 1.0e-6f, 1.0f);
-        const float dilog_alpha = det_dilog(alpha);
-        const float ndc = cd.w;
-        const float z = g_mix(add(mul(ndc, 0.5f), 0.5f), ndc, p.clip_z_01);
-        const uint32_t depth_key = g_f2u_sat(mul(g_clamp(z, 0.0f, 1.0f), 4294967294.0f));
-        uint32_t color;
-        if (p.linear_color) {
-            color = splat_id;
-        } else {
-            uint32_t r = __float2uint_rn(mul(g_clamp(co.x, 0.0f, 1.0f), 255.0f));
-            uint32_t g = __float2uint_rn(mul(g_clamp(co.y, 0.0f, 1.0f), 255.0f));
-            uint32_t b = __float2uint_rn(mul(g_clamp(co.z, 0.0f, 1.0f), 255.0f));
-            color = r | (g << 8u) | (b << 16u) | 0xFF000000u;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t groups = (n_vis + 31u) / 32u;
+    for (uint32_t grp = blockIdx.x * 8u + (uint32_t)warp; grp < groups; grp += gridDim.x * 8u) {
+        const uint32_t v = grp * 32u + (uint32_t)lane;
+        uint32_t wic = 0u, splat_id = 0u;
+        float4 co, cr, cd;
+        float cov_a = 0.0f, cov_b = 0.0f, cov_c = 0.0f;
+        if (v < n_vis) {
+            splat_id = p.vis_ids[v];
+            const float4* P = p.projected + (size_t)splat_id * 4;
+            co = P[0];
+            cr = P[1];
+            cd = P[2];
+            const float4 cv = P[3];
+            const float ssf = g_max(ss, 1.0f);
+            cov_a = add(cv.x, 0.3f);
+            cov_b = cv.y;
+            cov_c = add(cv.z, 0.3f);
+            const float det = sub(mul(cov_a, cov_c), mul(cov_b, cov_b));
+            const float expected = mul(mul(mul(mul(ssf, ssf), 6.28318530718f), __fsqrt_rn(g_max(det, 0.0f))),
+                                       det_dilog(g_clamp(co.w, 0.0f, 1.0f)));
+            const float ppw = g_max(mul(ssf, ssf), 1.0f);
+            const float scaled = g_max(dv(expected, ppw), 0.0f);
+            wic = g_f2u_sat(g_clamp(floorf(scaled), 0.0f, 4294967295.0f));
+            if (hash01(splat_id + 0x9e3779b9u) < g_fract(scaled) && wic < 0xFFFFFFFFu) wic += 1u;
         }
-        float4* pr = prepared + (size_t)v * 3;
-        pr[0] = make_float4(cr.x, cr.y, l00, l10);
-        pr[1] = make_float4(l11, alpha, dilog_alpha, 0.0f);
-        pr[2] = make_float4(__uint_as_float(depth_key), __uint_as_float(color), __uint_as_float(splat_id), 0.0f);
-        for (uint32_t i = 0; i < write_count; ++i) work[base + i] = make_uint2(v, i);
+        // reservation: the counter counts every requested item modulo 2^32, as one addition a Gaussian would
+        uint32_t incl = wic;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        if (!__any_sync(0xffffffffu, wic != 0u)) continue;
+        uint32_t first = 0u;
+        if (lane == 0) first = atomicAdd(&p.fc->gps_work[0], total);
+        first = __shfl_sync(0xffffffffu, first, 0);
+        const uint32_t cap = p.max_work_items;
+        const uint32_t base = first + incl - wic;
+        const bool over = wic != 0u && (base >= cap || wic > cap - base);
+        if (__any_sync(0xffffffffu, over) && lane == 0) atomicOr(&p.fc->gps_work[1], 1u);
+        const uint32_t write_count = wic == 0u || base >= cap ? 0u : min(wic, cap - base);
+        if (write_count) {
+            const float l00 = __fsqrt_rn(g_max(cov_a, 1.0e-5f));
+            const float l10 = dv(cov_b, l00);
+            const float l11 = __fsqrt_rn(g_max(sub(cov_c, mul(l10, l10)), 1.0e-5f));
+            const float alpha = g_clamp(co.w, 1.0e-6f, 1.0f);
+            const float dilog_alpha = det_dilog(alpha);
+            const float ndc = cd.w;
+            const float z = g_mix(add(mul(ndc, 0.5f), 0.5f), ndc, p.clip_z_01);
+            const uint32_t depth_key = g_f2u_sat(mul(g_clamp(z, 0.0f, 1.0f), 4294967294.0f));
+            uint32_t color;
+            if (p.linear_color) {
+                color = splat_id;
+            } else {
+                uint32_t r = __float2uint_rn(mul(g_clamp(co.x, 0.0f, 1.0f), 255.0f));
+                uint32_t g = __float2uint_rn(mul(g_clamp(co.y, 0.0f, 1.0f), 255.0f));
+                uint32_t b = __float2uint_rn(mul(g_clamp(co.z, 0.0f, 1.0f), 255.0f));
+                color = r | (g << 8u) | (b << 16u) | 0xFF000000u;
+            }
+            float4* pr = prepared + (size_t)v * 3;
+            pr[0] = make_float4(cr.x, cr.y, l00, l10);
+            pr[1] = make_float4(l11, alpha, dilog_alpha, 0.0f);
+            pr[2] = make_float4(__uint_as_float(depth_key), __uint_as_float(color), __uint_as_float(splat_id), 0.0f);
+        }
+        // The items of lane l are work[base_l .. base_l + write_count_l).  Without an overflow inside the warp these
+        // ranges follow one another from `first`; an overflowing warp (the budget ends in it, or the counter wraps)
+        // lets every lane write its own.
+        const uint32_t written = write_count;
+        const uint64_t sum64 = (uint64_t)first + (uint64_t)total;   // total < 2^32 only if no prefix wrapped
+        const bool plain = !__any_sync(0xffffffffu, over) && sum64 <= (uint64_t)cap &&
+                           __all_sync(0xffffffffu, incl >= wic && incl <= total);
+        if (plain) {
+            s_end[warp][lane] = incl;
+            __syncwarp();
+            for (uint32_t k = (uint32_t)lane; k < total; k += 32u) {
+                int lo = 0, hi = 31;   // the first lane whose prefix sum exceeds k
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (s_end[warp][mid] > k) hi = mid;
+                    else lo = mid + 1;
+                }
+                const uint32_t start = lo ? s_end[warp][lo - 1] : 0u;
+                work[first + k] = make_uint2(grp * 32u + (uint32_t)lo, k - start);
+            }
+            __syncwarp();
+        } else {
+            for (uint32_t i = 0; i < written; ++i) work[base + i] = make_uint2(v, i);
+        }
     }
 }
 

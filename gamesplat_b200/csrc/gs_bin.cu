@@ -17,8 +17,10 @@
 // map: marks at each splat's first entry, then a block prefix maximum), so
 // the work is balanced however many tiles one splat covers and the stores are
 // coalesced; the tile ids' digit histograms for the tile sort are accumulated
-// on the way.  Two more small kernels follow the tile sort: the [start, end)
-// range of each tile, and the rasterization order (heaviest tiles first).
+// on the way.  After the tile sort, which marks the [start, end) range of each
+// tile, comes the rasterization order (heaviest tiles first).  Frames whose
+// tile ids and positions do not fit the packed entries (tile_pass_kernel) sort
+// (id, position) pairs and find the ranges in a pass of their own.
 //
 // Tile selection is conservative: the covered rectangle is intersected with
 // the bounding box of the ellipse where the Gaussian's alpha reaches 1/255
@@ -39,7 +41,9 @@ __device__ __forceinline__ BinItem bin_one(const BinParams& p, uint32_t s, uint3
                                            float ysign) {
     BinItem it = {0u, 0, -1, 0, -1};
     const float4* P = p.projected + (size_t)id * 4;
-    const float4 co = P[0], cr = P[1], cd = P[2];
+    float4 co, cr;
+    ld_global32(P, co, cr);
+    const float4 cd = P[2];
     PixelRect q;
     const float cutoff = alpha_cutoff(co.w);
     bool ok;
@@ -115,10 +119,8 @@ __device__ __forceinline__ BinItem bin_one(const BinParams& p, uint32_t s, uint3
     }
     float4* dst = reinterpret_cast<float4*>(p.records + s);
     const float4* src = reinterpret_cast<const float4*>(&rec);
-    dst[0] = src[0];
-    dst[1] = src[1];
-    dst[2] = src[2];
-    dst[3] = src[3];
+    st_global32(dst, src[0], src[1]);
+    st_global32(dst + 2, src[2], src[3]);
     return it;
 }
 
@@ -241,6 +243,8 @@ __global__ void __launch_bounds__(kBinThreads) bin_kernel(BinParams p) {
 // written in the order the binning defined, so the result is the same
 // whichever CTA expands a chunk; the tile ids' digit histograms for the tile
 // sort are accumulated here.
+// kPacked: entries as tile_pass_kernel sorts them (a byte and a word).
+template <bool kPacked>
 __global__ void __launch_bounds__(kBinThreads) expand_kernel(BinParams p) {
     pdl_wait();
     __shared__ uint32_t scan_tmp[33];
@@ -297,11 +301,16 @@ __global__ void __launch_bounds__(kBinThreads) expand_kernel(BinParams p) {
             const uint32_t w = max(inf.z, 1u);
             const uint32_t ty = (inf.y >> 16) + k / w, tx = (inf.y & 0xFFFFu) + k % w;
             const uint32_t tid = ty * (uint32_t)p.tiles_x + tx;
-            p.entry_keys[e0 + i] = tid;
-            p.entry_vals[e0 + i] = n_vis - 1u - q;
+            if (kPacked) {
+                reinterpret_cast<uint8_t*>(p.entry_keys)[e0 + i] = (uint8_t)tid;
+                p.entry_vals[e0 + i] = (n_vis - 1u - q) | (tid >> 8 ? (tid >> 8) << p.entry_vbits : 0u);
+            } else {
+                p.entry_keys[e0 + i] = tid;
+                p.entry_vals[e0 + i] = n_vis - 1u - q;
+                atomicAdd(&s_hist[2][(tid >> 16) & 255u], 1u);
+            }
             atomicAdd(&s_hist[0][tid & 255u], 1u);
             atomicAdd(&s_hist[1][(tid >> 8) & 255u], 1u);
-            atomicAdd(&s_hist[2][(tid >> 16) & 255u], 1u);
         }
         __syncthreads();
     }
@@ -349,8 +358,8 @@ __global__ void tile_ranges_kernel(const SortPlan* plan, const FrameCounters* fc
 // classes), so the heaviest tiles start in the first wave instead of
 // stretching the last one.  One CTA; the order within a class is immaterial
 // (each tile's CTA writes only its own pixels).
-__global__ void __launch_bounds__(1024) tile_order_kernel(const uint2* __restrict__ ranges, uint32_t num_tiles,
-                                                          uint32_t* __restrict__ order) {
+__global__ void __launch_bounds__(1024) tile_order_kernel(uint2* __restrict__ ranges, uint32_t num_tiles,
+                                                          uint32_t* __restrict__ order, bool turned) {
     pdl_wait();
     pdl_trigger();
     __shared__ uint32_t s_cnt[129], s_start[129];
@@ -365,7 +374,13 @@ __global__ void __launch_bounds__(1024) tile_order_kernel(const uint2* __restric
         const uint32_t frac = lz >= 30 ? 0u : (w << (lz + 1)) >> 30;   // two bits after the leading one
         return lz * 4u + (3u - frac);
     };
-    for (uint32_t tl = t; tl < num_tiles; tl += blockDim.x) atomicAdd(&s_cnt[cls(tl)], 1u);
+    for (uint32_t tl = t; tl < num_tiles; tl += blockDim.x) {
+        if (turned) {   // (~start, end), zero without entries: see tile_pass_kernel
+            const uint2 r = ranges[tl];
+            ranges[tl] = r.y ? make_uint2(~r.x, r.y) : make_uint2(0u, 0u);
+        }
+        atomicAdd(&s_cnt[cls(tl)], 1u);
+    }
     __syncthreads();
     if (t == 0) {
         uint32_t run = 0;
@@ -378,11 +393,11 @@ __global__ void __launch_bounds__(1024) tile_order_kernel(const uint2* __restric
     for (uint32_t tl = t; tl < num_tiles; tl += blockDim.x) order[atomicAdd(&s_start[cls(tl)], 1u)] = tl;
 }
 
-int launch_tile_order(const uint2* ranges, uint32_t num_tiles, uint32_t* order, cudaStream_t s) {
+int launch_tile_order(uint2* ranges, uint32_t num_tiles, uint32_t* order, bool turned, cudaStream_t s) {
     if (num_tiles == 0) return 0;
     // programmatic dependent launch (as the ranges and the raster after it): the kernel is scheduled while its
     // predecessor drains and waits for it (griddepcontrol.wait) before it reads anything
-    launch_pdl(tile_order_kernel, dim3(1), dim3(1024), 0, s, ranges, num_tiles, order);
+    launch_pdl(tile_order_kernel, dim3(1), dim3(1024), 0, s, ranges, num_tiles, order, turned);
     return 1;
 }
 
@@ -392,7 +407,9 @@ int launch_bin(const BinParams& p, uint32_t n_cap, uint32_t num_sms, cudaStream_
     if (grid > tiles) grid = tiles;
     if (grid == 0) grid = 1;
     launch_pdl(bin_kernel, dim3(grid), dim3(kBinThreads), 0, s, p);
-    launch_pdl(expand_kernel, dim3(num_sms * (1024 / kBinThreads)), dim3(kBinThreads), 0, s, p);
+    const dim3 egrid(num_sms * (1024 / kBinThreads));
+    if (p.entry_vbits >= 0) launch_pdl(expand_kernel<true>, egrid, dim3(kBinThreads), 0, s, p);
+    else launch_pdl(expand_kernel<false>, egrid, dim3(kBinThreads), 0, s, p);
     return 2;
 }
 

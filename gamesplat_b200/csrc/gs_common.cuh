@@ -155,6 +155,18 @@ __device__ __forceinline__ float alpha_cutoff(float opacity) {
     return det_logf(dv(1.0f / 255.0f, g_max(opacity, 1.0e-8f)));
 }
 
+// 32 bytes in one access (32-byte aligned): a whole sector whatever the L1 holds.
+__device__ __forceinline__ void ld_global32(const void* p, float4& a, float4& b) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p));
+}
+__device__ __forceinline__ void st_global32(void* p, const float4& a, const float4& b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+
 // ---------------------------------------------------------------------------
 // Quad coverage of one splat (shaders/splat.glsl:61-67): corners centre ±
 // radius (+ jitter), NDC, viewport transform x_w = ndc * (w/2) + w/2, 8-bit

@@ -339,7 +339,8 @@ int launch_pack_half_rows(const float4* rows, float4* half_rows, uint32_t n, uin
 // (shaders/cull.glsl:209-220), computes the depth keys (:230-232) and places
 // the tile's visible (key, id) pairs in index order: a block scan of the
 // per-(row group, warp) counts, then one warp-level decoupled look-back per
-// tile.  The 4 x 256 key-digit histograms of the depth sort are accumulated in
+// tile.  The key-digit histograms of the depth sort (9-bit digits of the biased
+// key, see kDepthKeyBias) are accumulated in
 // shared memory; the top digit (sign and high exponent bits, a handful of
 // values in a scene) is aggregated per warp first, since 32 lanes adding to
 // one shared word would serialize.
@@ -347,12 +348,12 @@ __global__ void __launch_bounds__(kCullVisThreads) cull_visible_kernel(CullParam
     pdl_wait();
     constexpr int kWarps = kCullVisThreads / 32;
     static_assert(kCullVisItems * kWarps == 64, "the count scan gives each lane two (row group, warp) counts");
-    __shared__ uint32_t s_hist[4][256];
+    __shared__ uint32_t s_hist[4][kDepthRadix];
     __shared__ uint32_t s_cnt[kCullVisItems * kWarps];   // (row group, warp) order = index order
     __shared__ uint32_t s_tile, s_excl;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t lt = (1u << lane) - 1u;
-    for (int i = t; i < 4 * 256; i += kCullVisThreads) (&s_hist[0][0])[i] = 0u;
+    for (int i = t; i < 4 * kDepthRadix; i += kCullVisThreads) (&s_hist[0][0])[i] = 0u;
     if (t == 0) s_tile = atomicAdd(&p.fc->cull_ticket, 1u);
     __syncthreads();
     const uint32_t tile = s_tile;
@@ -432,17 +433,18 @@ __global__ void __launch_bounds__(kCullVisThreads) cull_visible_kernel(CullParam
             const uint32_t o = excl + s_cnt[k * kWarps + warp] + (uint32_t)__popc(mask[k] & lt);
             p.keys_out[o] = kk;
             p.ids_out[o] = base + k * kCullVisThreads + t;
-            atomicAdd(&s_hist[0][kk & 255u], 1u);
-            atomicAdd(&s_hist[1][(kk >> 8) & 255u], 1u);
-            atomicAdd(&s_hist[2][(kk >> 16) & 255u], 1u);
+            const uint32_t b = kk + kDepthKeyBias;
+            atomicAdd(&s_hist[0][b & 511u], 1u);
+            atomicAdd(&s_hist[1][(b >> 9) & 511u], 1u);
+            atomicAdd(&s_hist[2][(b >> 18) & 511u], 1u);
         }
         // invisible lanes match among themselves (256 is no digit) and add nothing
-        const uint32_t d3 = v ? (kk >> 24) : 256u;
+        const uint32_t d3 = v ? (kk + kDepthKeyBias) >> 27 : 256u;
         const uint32_t peers = __match_any_sync(0xffffffffu, d3);
         if (v && lane == __ffs(peers) - 1) atomicAdd(&s_hist[3][d3], (uint32_t)__popc(peers));
     }
     __syncthreads();
-    for (int i = t; i < 4 * 256; i += kCullVisThreads) {
+    for (int i = t; i < 4 * kDepthRadix; i += kCullVisThreads) {
         const uint32_t c = (&s_hist[0][0])[i];
         if (c) atomicAdd(p.key_hist + i, c);
     }

@@ -67,7 +67,6 @@ struct FrameSlot {
     uint32_t* chunk_first = nullptr;
     uint32_t chunk_cap = 0;
     unsigned long long* tsort_status = nullptr;
-    size_t tsort_status_stride = 0;
     uint32_t record_cap = 0;
 };
 
@@ -101,14 +100,12 @@ struct gs_ctx {
     unsigned long long* cull_status = nullptr;
     unsigned long long* sort_status = nullptr;
     unsigned long long* bin_status = nullptr;
-    size_t sort_status_stride = 0;
 
     // tile entries
     uint32_t entry_cap = 0;
     uint32_t* ekeys[2] = {nullptr, nullptr};
     uint32_t* evals[2] = {nullptr, nullptr};
     unsigned long long* tsort_status = nullptr;
-    size_t tsort_status_stride = 0;
 
     // per-frame control block (zeroed each frame)
     void* ctrl = nullptr;
@@ -344,7 +341,6 @@ void swap_slot(gs_ctx* c, FrameSlot& f) {
     std::swap(c->chunk_first, f.chunk_first);
     std::swap(c->chunk_cap, f.chunk_cap);
     std::swap(c->tsort_status, f.tsort_status);
-    std::swap(c->tsort_status_stride, f.tsort_status_stride);
 }
 
 void release_scene(gs_ctx* c) {
@@ -501,17 +497,17 @@ int ensure_entries(gs_ctx* c, uint32_t cap) {
     const uint32_t chunks = cap / (uint32_t)gs::kBinChunk + 2u;
     GS_CUDA(c, dalloc(&c->chunk_first, (size_t)chunks * 4));
     c->chunk_cap = chunks;
-    c->tsort_status_stride = gs::sort_status_words(cap);
-    GS_CUDA(c, dalloc(&c->tsort_status, c->tsort_status_stride * 4 * sizeof(unsigned long long)));
-    GS_CUDA(c, cudaMemsetAsync(c->tsort_status, 0, c->tsort_status_stride * 4 * sizeof(unsigned long long), c->stream));
+    const size_t status_bytes = gs::sort_status_words(cap) * 4 * sizeof(unsigned long long);
+    GS_CUDA(c, dalloc(&c->tsort_status, status_bytes));
+    GS_CUDA(c, cudaMemsetAsync(c->tsort_status, 0, status_bytes, c->stream));
     c->entry_cap = cap;
     return GS_OK;
 }
 
 // The per-frame control block of a w x h frame in the context's fields:
 // FrameCounters | SortPlan x2 | hist x2 (4x256) | tile ranges, and the tile order.
-// Control block layout: FrameCounters | SortPlan x2 | hist x2 (4x256) | tile
-// ranges; each part 256-byte aligned.
+// Control block layout: FrameCounters | SortPlan x2 | depth and tile digit
+// histograms | tile ranges; each part 256-byte aligned.
 struct CtrlLayout {
     size_t fc, dp, tp, dh, th, tr, bytes;
 };
@@ -527,7 +523,7 @@ CtrlLayout ctrl_layout(uint32_t tiles) {
     L.fc = place(sizeof(FrameCounters));
     L.dp = place(sizeof(SortPlan));
     L.tp = place(sizeof(SortPlan));
-    L.dh = place(4 * 256 * 4);
+    L.dh = place(4 * gs::kDepthRadix * 4);
     L.th = place(4 * 256 * 4);
     L.tr = place((size_t)tiles * sizeof(uint2));
     L.bytes = off;
@@ -738,17 +734,28 @@ void run_depth_sort(gs_ctx* c) {
     p.hist_ready = 1;
     p.plan = c->depth_plan;
     p.status = c->sort_status;
-    p.status_stride = c->sort_status_stride;
     p.epoch = c->epoch;
     p.error_flags = &c->fc->error_flags;
+    p.key_bias = gs::kDepthKeyBias;
     p.first_pdl = 1;
-    sc.add(gs::launch_sort(p, c->num_sms, c->stream));
+    sc.add(gs::launch_depth_sort(p, c->num_sms, c->stream));
+}
+
+// Bits of a sorted position when the tile entries can be packed into a byte and
+// a word (tile_pass_kernel), -1 when they cannot and are sorted as (id,
+// position) pairs.  Both limits are the layout's: ids of 16 bits (65 536 tiles,
+// 4096 x 4096 pixels) and, above a position, the id bits past the lower 8 in
+// 32 bits (2^24 Gaussians at that size, 2^27 at 1080p).
+int packed_entry_bits(const gs_ctx* c) {
+    const int idbits = entry_bits(c->tiles_cap), vbits = entry_bits(c->n);
+    return idbits <= 16 && vbits + std::max(idbits - 8, 0) <= 32 ? vbits : -1;
 }
 
 // Binning, tile sort and tile ranges for one raster pass.
 // readback: copy the counters to h_bin_fc on fc_stream once the tile sort has
 // run (the entry count is final after the expansion).
 void run_binning(gs_ctx* c, float jx, float jy, float seed, bool envelope = false, bool readback = true) {
+    const int vbits = packed_entry_bits(c);
     {
         StageScope sc(c, ST_BIN);
         gs::BinParams p{};
@@ -769,6 +776,7 @@ void run_binning(gs_ctx* c, float jx, float jy, float seed, bool envelope = fals
         p.records = c->records;
         p.entry_keys = c->ekeys[1];
         p.entry_vals = c->evals[1];
+        p.entry_vbits = vbits;
         p.entry_cap = c->entry_cap;
         p.item_info = c->item_info;
         p.chunk_first = c->chunk_first;
@@ -782,27 +790,46 @@ void run_binning(gs_ctx* c, float jx, float jy, float seed, bool envelope = fals
     }
     {
         StageScope sc(c, ST_TILE_SORT);
-        gs::SortParams p{};
-        p.keys_in = c->ekeys[1];
-        p.vals_in = c->evals[1];
-        p.keys_buf[0] = c->ekeys[0];
-        p.keys_buf[1] = c->ekeys[1];
-        p.vals_buf[0] = c->evals[0];
-        p.vals_buf[1] = c->evals[1];
-        p.land_in_buf0 = 0;
-        p.count_ptr = &c->fc->tile_entries;
-        p.count_cap = c->entry_cap;
-        p.begin_bit = 0;
-        p.end_bit = entry_bits(c->tiles_cap);
-        p.hist = c->tile_hist;    // accumulated by the bin kernel
-        p.hist_ready = 1;
-        p.plan = c->tile_plan;
-        p.status = c->tsort_status;
-        p.status_stride = c->tsort_status_stride;
-        p.epoch = c->epoch;
-        p.error_flags = &c->fc->error_flags;
-        p.first_pdl = 1;
-        sc.add(gs::launch_sort(p, c->num_sms, c->stream));
+        if (vbits >= 0) {
+            gs::TileSortParams p{};
+            p.low = reinterpret_cast<const uint8_t*>(c->ekeys[1]);
+            p.words[0] = c->evals[1];
+            p.words[1] = c->evals[0];
+            p.words[2] = c->evals[1];
+            p.vbits = vbits;
+            p.last_pass = c->tiles_cap > 256u ? 1 : 0;
+            p.count_ptr = &c->fc->tile_entries;
+            p.count_cap = c->entry_cap;
+            p.hist = c->tile_hist;    // accumulated by the expansion
+            p.plan = c->tile_plan;
+            p.status = c->tsort_status;
+            p.epoch = c->epoch;
+            p.error_flags = &c->fc->error_flags;
+            p.ranges = c->tile_ranges;
+            p.num_tiles = c->tiles_cap;
+            sc.add(gs::launch_tile_sort(p, c->num_sms, c->stream));
+        } else {
+            gs::SortParams p{};
+            p.keys_in = c->ekeys[1];
+            p.vals_in = c->evals[1];
+            p.keys_buf[0] = c->ekeys[0];
+            p.keys_buf[1] = c->ekeys[1];
+            p.vals_buf[0] = c->evals[0];
+            p.vals_buf[1] = c->evals[1];
+            p.land_in_buf0 = 0;
+            p.count_ptr = &c->fc->tile_entries;
+            p.count_cap = c->entry_cap;
+            p.begin_bit = 0;
+            p.end_bit = entry_bits(c->tiles_cap);
+            p.hist = c->tile_hist;    // accumulated by the expansion
+            p.hist_ready = 1;
+            p.plan = c->tile_plan;
+            p.status = c->tsort_status;
+            p.epoch = c->epoch;
+            p.error_flags = &c->fc->error_flags;
+            p.first_pdl = 1;
+            sc.add(gs::launch_sort(p, c->num_sms, c->stream));
+        }
         // The entry count is final once the expansion ran; the readback is
         // queued behind the tile sort so that the expansion and the sort's
         // first pass stay adjacent (programmatic dependent launch between them).
@@ -813,9 +840,10 @@ void run_binning(gs_ctx* c, float jx, float jy, float seed, bool envelope = fals
             cudaEventRecord(c->bin_event, c->fc_stream);
             c->bin_recorded = true;
         }
-        sc.add(gs::launch_tile_ranges(c->tile_plan, c->fc, c->entry_cap, c->tile_ranges, c->tiles_cap, c->num_sms,
-                                       c->stream));
-        sc.add(gs::launch_tile_order(c->tile_ranges, c->tiles_cap, c->tile_order, c->stream));
+        if (vbits < 0)
+            sc.add(gs::launch_tile_ranges(c->tile_plan, c->fc, c->entry_cap, c->tile_ranges, c->tiles_cap, c->num_sms,
+                                           c->stream));
+        sc.add(gs::launch_tile_order(c->tile_ranges, c->tiles_cap, c->tile_order, vbits >= 0, c->stream));
     }
 }
 
@@ -1362,12 +1390,12 @@ static int upload_common(gs_ctx* c, const float* rows, uint64_t count, cudaMemcp
     GS_CUDA(c, dalloc(&c->item_info, (size_t)n * sizeof(uint4)));
     const size_t cull_tiles = ((size_t)n + gs::kCullVisTile - 1) / gs::kCullVisTile;
     GS_CUDA(c, dalloc(&c->cull_status, cull_tiles * sizeof(unsigned long long)));
-    c->sort_status_stride = gs::sort_status_words(n);
-    GS_CUDA(c, dalloc(&c->sort_status, c->sort_status_stride * 4 * sizeof(unsigned long long)));
+    const size_t sort_words = gs::sort_status_words(n) * 4;
+    GS_CUDA(c, dalloc(&c->sort_status, sort_words * sizeof(unsigned long long)));
     const size_t bin_tiles = ((size_t)n + gs::kBinTile - 1) / gs::kBinTile;
     GS_CUDA(c, dalloc(&c->bin_status, bin_tiles * sizeof(unsigned long long)));
     GS_CUDA(c, cudaMemsetAsync(c->cull_status, 0, cull_tiles * 8, c->stream));
-    GS_CUDA(c, cudaMemsetAsync(c->sort_status, 0, c->sort_status_stride * 4 * 8, c->stream));
+    GS_CUDA(c, cudaMemsetAsync(c->sort_status, 0, sort_words * 8, c->stream));
     GS_CUDA(c, cudaMemsetAsync(c->bin_status, 0, bin_tiles * 8, c->stream));
     GS_CUDA(c, cudaMemsetAsync(c->projected, 0, (size_t)n * 64, c->stream));
     if (half) {

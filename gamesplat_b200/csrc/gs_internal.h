@@ -36,31 +36,28 @@ struct FrameCounters {
     uint32_t pad[1];
 };
 
-// Device-resident plan of one radix sort, written by its plan kernel from the
-// digit histograms: which passes do work (a pass whose digit is the same for
-// every key is the identity permutation of a stable sort and is skipped),
-// and the ping-pong buffers of each active pass.  Zeroed before each sort.
+// Device-resident state of one radix sort: the tile tickets of its passes and
+// where its result is.  Zeroed before each sort.
 struct SortPlan {
-    const uint32_t* kin[4];
-    const uint32_t* vin[4];
-    uint32_t* kout[4];
-    uint32_t* vout[4];
-    uint32_t active[4];
-    uint32_t ticket[4];
     const uint32_t* kfinal;      // where the sorted keys are
     const uint32_t* vfinal;      // where the sorted values are
-    uint32_t copy_needed;        // land_in_buf0 with no active pass
+    uint32_t ticket[4];
     uint32_t count;
-    uint32_t pad[2];
 };
 
 // Onesweep radix sort configuration.
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;  // keys per CTA tile
-constexpr int kSortLookback = 8;                       // look-back words read per step
+constexpr int kSortTile = 4096;   // pairs per 4 x kRadix look-back words (sort_status_words() * 4 words in all)
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 1 << kRadixBits;
+// Depth keys are 0xFFFFFFFF - bits(depth) with depth >= 0.2 for every visible
+// row (the near test of the cull).  Adding bits(0.2f) (modulo 2^32) keeps their
+// order and lifts the keys of depths below ~13 000 into the top 2^27 of the
+// range: their upper 5 bits are equal, so three passes of 9 bits sort them and
+// the fourth, of 5, is skipped.
+constexpr int kDepthBits = 9;
+constexpr int kDepthRadix = 1 << kDepthBits;
+constexpr uint32_t kDepthKeyBias = 0x3E4CCCCDu;   // bits of 0.2f
 
 // Cull configuration.  Visibility pass: 256-thread CTAs, 8 rows per thread;
 // its 2048-row CTA tiles are the units of the look-back.  Projection pass:
@@ -119,7 +116,7 @@ struct CullParams {
     uint32_t* ids_out;           // compacted visible ids
     unsigned long long* status;  // per-tile look-back words (epoch-tagged)
     uint32_t epoch;
-    uint32_t* key_hist;          // 4 x 256 digit histograms of the emitted keys (zeroed per frame)
+    uint32_t* key_hist;          // 4 x kDepthRadix digit histograms of key + kDepthKeyBias (zeroed per frame)
     // gsanim int8 appearance deltas (shaders/cull.glsl:125-164); null = none
     const int8_t* anim_deltas;   // [(state-1) * n + row] * 48 + j
     const float* anim_scales;    // 48 (device)
@@ -142,14 +139,31 @@ struct SortParams {
     const uint32_t* count_ptr;   // device-side element count
     uint32_t count_cap;          // capacity (grid sizing)
     int begin_bit, end_bit;
-    uint32_t* hist;              // 4 x 256 digit histograms (zeroed before the sort)
+    uint32_t* hist;              // digit histograms of the passes (zeroed before the sort)
     int hist_ready;              // 1: the producer of the keys already filled `hist`
     SortPlan* plan;              // zeroed before the sort
-    unsigned long long* status;  // per pass: tiles x 256 look-back words (epoch-tagged)
-    size_t status_stride;        // words per pass
+    unsigned long long* status;  // look-back words, tagged with the epoch and the pass
     uint32_t epoch;
     uint32_t* error_flags;
+    uint32_t key_bias = 0;       // digits are those of key + key_bias (modulo 2^32)
     int first_pdl = 0;           // 1: the first pass too is a programmatic dependent launch
+};
+
+// Tile entries whose id's upper bits and sorted position fit one word.
+struct TileSortParams {
+    const uint8_t* low;          // lower 8 id bits of every entry
+    uint32_t* words[3];          // (id >> 8) << vbits | position: input, after the first pass, after the second
+    int vbits;
+    int last_pass;               // 0: at most 256 tiles, one pass; its output and the second's are bare positions
+    const uint32_t* count_ptr;   // entries (device)
+    uint32_t count_cap;
+    const uint32_t* hist;        // 2 x 256: lower and upper digits of the ids
+    SortPlan* plan;              // zeroed before the sort; vfinal = the sorted positions
+    unsigned long long* status;
+    uint32_t epoch;
+    uint32_t* error_flags;
+    uint2* ranges;               // per tile (~start, end), zeroed before the sort
+    uint32_t num_tiles;
 };
 
 struct BinParams {
@@ -161,8 +175,9 @@ struct BinParams {
     int width, height, tiles_x, tiles_y;
     int tile_shift_x, tile_shift_y;  // log2 of the tile width and height
     RasterRecord* records;           // N_vis records (sorted order)
-    uint32_t* entry_keys;            // tile id per entry
-    uint32_t* entry_vals;            // sorted position per entry
+    uint32_t* entry_keys;            // tile id per entry (entry_vbits < 0), or its lower 8 bits, a byte per entry
+    uint32_t* entry_vals;            // sorted position per entry, with (id >> 8) << entry_vbits above it
+    int entry_vbits;
     uint32_t entry_cap;
     uint4* item_info;                // per binned item: first entry, tx0 | ty0 << 16, width in tiles (0: none)
     uint32_t* chunk_first;           // per expansion chunk: the item owning its first entry
@@ -254,11 +269,14 @@ inline size_t state_colour_floats(size_t cap, int frames) {
 }
 int launch_recolour_states(const CullParams& p, const RasterRecord* records, const StateBatch& st, int frames,
                            float* colours, uint32_t num_sms, cudaStream_t s);
-int launch_sort(const SortParams& p, uint32_t num_sms, cudaStream_t s);
+int launch_sort(const SortParams& p, uint32_t num_sms, cudaStream_t s);         // 8-bit digits, any bit range
+int launch_depth_sort(const SortParams& p, uint32_t num_sms, cudaStream_t s);   // 9-bit digits, histograms ready
+int launch_tile_sort(const TileSortParams& p, uint32_t num_sms, cudaStream_t s);
 int launch_bin(const BinParams& p, uint32_t n_cap, uint32_t num_sms, cudaStream_t s);
 int launch_tile_ranges(const SortPlan* tile_plan, const FrameCounters* fc, uint32_t entry_cap, uint2* ranges,
                        uint32_t num_tiles, uint32_t num_sms, cudaStream_t s);
-int launch_tile_order(const uint2* ranges, uint32_t num_tiles, uint32_t* order, cudaStream_t s);
+// turned: the ranges are (~start, end) (launch_tile_sort) and are turned round here
+int launch_tile_order(uint2* ranges, uint32_t num_tiles, uint32_t* order, bool turned, cudaStream_t s);
 int launch_raster_alpha(const RasterParams& p, cudaStream_t s);
 int launch_raster_stochastic(const RasterParams& p, cudaStream_t s);
 int launch_raster_stochastic2(const RasterParams& p, cudaStream_t s);
@@ -273,6 +291,6 @@ int launch_raster_states(const RasterParams& p, const StateOuts& outs, int frame
 int launch_wait_probe(const unsigned long long* status, FrameCounters* fc, uint32_t epoch, int which, uint32_t limit,
                       cudaStream_t s);
 
-size_t sort_status_words(uint32_t count_cap);   // look-back words per pass
+size_t sort_status_words(uint32_t count_cap);   // a quarter of a sort's look-back words
 int sort_passes(int begin_bit, int end_bit);
 }  // namespace gs

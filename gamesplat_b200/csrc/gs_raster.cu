@@ -44,9 +44,10 @@
 //
 // Stochastic mode: a fragment is kept iff hash13(fragcoord, id + seed) <
 // alpha; the depth test (LESS, writes on) keeps the kept fragment with the
-// smallest (D24 depth, instance index).  Walking front to back, a pixel stops
-// once a splat's D24 exceeds the kept one's by more than 8 (the float
-// depth-to-D24 mapping is monotone to within 5 units).  Deterministic exp and
+// smallest (D24 depth, instance index).  Walking front to back, a warp stops
+// once a splat's D24 exceeds the kept ones of all its pixels by more than 8 (the
+// float depth-to-D24 mapping is monotone to within 5 units, so a pixel whose
+// kept depth was exceeded by 8 keeps nothing of a later splat either).  Deterministic exp and
 // hash, so the kept set matches the oracle bit for bit.
 #include <cuda_fp16.h>
 
@@ -84,12 +85,14 @@ __device__ __forceinline__ PixelHash pixel_hash(float x, float y) {
     return h;
 }
 
-__device__ __forceinline__ float hash_z(float z) { return g_fract(mul(z, 0.1031f)); }
+// Both pixels of a thread (they share a column, hence p0): the same operations
+// in the same order, two to an instruction.
+struct PixelHash2 {
+    float p0, p0c;
+    float2 p1, t1;
+};
 
-__device__ __forceinline__ float hash13(const PixelHash& h, float p2) {
-    const float d = add(add(h.t1, mul(h.p1, add(p2, 33.33f))), mul(p2, h.p0c));
-    return g_fract(mul(add(add(h.p0, d), add(h.p1, d)), add(p2, d)));
-}
+__device__ __forceinline__ float hash_z(float z) { return g_fract(mul(z, 0.1031f)); }
 
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
@@ -99,92 +102,50 @@ __device__ __forceinline__ float ex2_approx(float x) {
 
 __device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
 
+// The multiplications stay scalar: a packed one is contracted with the packed
+// addition of its result (whatever -fmad says), which the hash does not stand.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(mul(a.x, b.x), mul(a.y, b.y)); }
+
+__device__ __forceinline__ float2 hash13(const PixelHash2& h, float p2) {
+    const float m = mul(p2, h.p0c);
+    const float2 d = __fadd2_rn(__fadd2_rn(h.t1, mul2(h.p1, f2(add(p2, 33.33f)))), f2(m));
+    const float2 x = mul2(__fadd2_rn(__fadd2_rn(f2(h.p0), d), __fadd2_rn(h.p1, d)), __fadd2_rn(f2(p2), d));
+    return make_float2(g_fract(x.x), g_fract(x.y));
+}
+
+// Fragment tests of one pixel: covered (all bits it needs are among the
+// record's) and 0 <= s <= s_max, as one unsigned comparison (a negative s has
+// the top bit set, a NaN compares above s_max).  The bounds of RasterRecord
+// also admit s = -0 and the negative subnormal of the last place; s, a sum of
+// conic_x dx^2 >= +0, a product and conic_z dy^2 >= +0, never is -0, and is that
+// subnormal only if all terms are below 2^-125, a splat of sigma above 2^38
+// pixels.  These tests are the loop's comparisons, on the ALU pipe that bounds
+// the rasterizers (see raster_kernel): 310 -> 287 us for the alpha frame there.
+template <class M>
+__device__ __forceinline__ bool frag_live(M bits, M need, float s, float s_max) {
+    return (need & ~bits) == (M)0 && __float_as_uint(s) <= __float_as_uint(s_max);
+}
+
+// The kept fragment of one (pixel, sample); best_id 0xFFFFFFFF (beyond every
+// index) and the far plane's D24 while there is none.
 struct StochState {
     uint32_t best_d24, best_id;
     float r, g, b;
 };
 
-// alpha = min(opacity * exp(power), 0.99) with power <= 0 (exp <= 1 there, also
-// for the deterministic exp) never exceeds min(opacity, 0.99): a fragment whose
-// hash is at or above that bound is rejected without evaluating exp.
-// ph: the pixel's hash terms, hz: hash_z(splat id + sample seed).
-__device__ __forceinline__ void stoch_step(StochState& S, float s, float opacity, const PixelHash& ph, float hz,
-                                           uint32_t z24, uint32_t id, float r, float g, float b) {
-    const float rnd = hash13(ph, hz);
-    if (!(rnd < g_min(opacity, 0.99f))) return;
-    const float alpha = g_min(mul(opacity, det_expf(mul(-0.5f, s))), 0.99f);
-    if (rnd < alpha) {
-        S.best_d24 = z24;
-        S.best_id = id;
-        S.r = r;
-        S.g = g;
-        S.b = b;
-    }
-}
+constexpr uint32_t kFarD24 = 16777215u;
 
-// Two samples of one pixel (denoised mode): the kept fragment of each seed.
-struct Stoch2 {
-    StochState s[2];
-    bool done[2];
-};
-
-__device__ __forceinline__ void stoch2_init(Stoch2& P, bool inside) {
-    for (int k = 0; k < 2; ++k) {
-        P.s[k] = {16777215u, 0xFFFFFFFFu, 0.0f, 0.0f, 0.0f};
-        P.done[k] = !inside;
-    }
-}
-
-// One splat into both samples of a pixel: alpha once, one hash per seed.
-__device__ __forceinline__ void stoch2_step(Stoch2& P, bool live, float sq, float opacity, const PixelHash& ph,
-                                            float hz0, float hz1, uint32_t z24, uint32_t id, float r, float g,
-                                            float b) {
-    bool want[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-        want[k] = live && !P.done[k] &&
-                  (z24 < P.s[k].best_d24 || (z24 == P.s[k].best_d24 && id < P.s[k].best_id));
-    if (!(want[0] || want[1])) return;
-    // hashes first: exp only when one of them is below alpha's bound (see stoch_step)
-    const float bound = g_min(opacity, 0.99f);
-    float rnd[2];
-    bool cand[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        rnd[k] = want[k] ? hash13(ph, k ? hz1 : hz0) : 1.0f;
-        cand[k] = want[k] && rnd[k] < bound;
-    }
-    if (!(cand[0] || cand[1])) return;
-    const float alpha = g_min(mul(opacity, det_expf(mul(-0.5f, sq))), 0.99f);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        if (cand[k] && rnd[k] < alpha) {
-            P.s[k].best_d24 = z24;
-            P.s[k].best_id = id;
-            P.s[k].r = r;
-            P.s[k].g = g;
-            P.s[k].b = b;
-        }
-    }
-}
-
-__device__ __forceinline__ void stoch2_retire(Stoch2& P, uint32_t z24, uint32_t margin) {
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-        if (P.s[k].best_id != 0xFFFFFFFFu && z24 > P.s[k].best_d24 + margin) P.done[k] = true;
-}
-
-__device__ __forceinline__ void write_pixel_stoch2(const RasterParams& p, int px, int py, const Stoch2& P) {
+__device__ __forceinline__ void write_pixel_stoch2(const RasterParams& p, int px, int py, const StochState (&S)[2]) {
     const size_t o = (size_t)(p.height - 1 - py) * p.width + px;
     float c[2][3], a[2], d[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        const bool kept = P.s[k].best_id != 0xFFFFFFFFu;
-        c[k][0] = kept ? P.s[k].r : p.bg;
-        c[k][1] = kept ? P.s[k].g : p.bg;
-        c[k][2] = kept ? P.s[k].b : p.bg;
+        const bool kept = S[k].best_id != 0xFFFFFFFFu;
+        c[k][0] = kept ? S[k].r : p.bg;
+        c[k][1] = kept ? S[k].g : p.bg;
+        c[k][2] = kept ? S[k].b : p.bg;
         a[k] = kept ? 1.0f : 0.0f;
-        d[k] = __fdiv_rn((float)P.s[k].best_d24, 16777215.0f);
+        d[k] = __fdiv_rn((float)S[k].best_d24, 16777215.0f);
     }
     p.out_rgba32f[o] = make_float4(mul(add(c[0][0], c[1][0]), 0.5f), mul(add(c[0][1], c[1][1]), 0.5f),
                                    mul(add(c[0][2], c[1][2]), 0.5f), mul(add(a[0], a[1]), 0.5f));
@@ -274,7 +235,7 @@ __device__ __forceinline__ float min_q_box(float A, float B, float C, float X0, 
 // of it: the two pixels share a column, hence dx, the column test and the
 // first term of the Gaussian exponent.
 // Shared memory of one CTA's tile: two staging buffers of records, their
-// barriers, the records' coverage bits and warp-block masks.
+// barriers, the records' warp-block masks and the warps' lists.
 // A staged record and 16 bytes of padding: at an 80-byte stride the 16-byte
 // loads of 8 consecutive records (one record per thread in the staging pass)
 // fall in distinct banks, and a 32-bit field of 32 consecutive records spreads
@@ -298,9 +259,9 @@ template <int kMode, int kTw = 16, int kTh = 16, int kStates = 0>
 struct __align__(128) RasterShared : StateColours<kStates> {
     StagedRecord rec[2][kBatch];
     uint64_t bar[2];
-    typename TileShape<kTw, kTh>::Mask bits[kBatch];
     uint8_t mask[kBatch];
-    float4 cen[kMode == 1 ? kBatch : 1];   // stochastic: jittered centre and hash z of the sample
+    // per warp the staged records it shades, as byte offsets from the first, nearest first
+    __align__(16) uint16_t list[4][kBatch];
 };
 
 // One 16x16 tile, the whole CTA (used by the per-frame kernel, one tile per
@@ -338,7 +299,14 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
     const float fcx = (float)px + 0.5f, fcy0 = (float)py0 + 0.5f, fcy1 = (float)py1 + 0.5f;
     const float2 fcy = make_float2(fcy0, fcy1);
     // the stochastic modes' hash terms of the two pixels
-    const PixelHash ph0 = pixel_hash(fcx, fcy0), ph1 = pixel_hash(fcx, fcy1);
+    PixelHash2 pixh;
+    if (kMode != 0) {
+        const PixelHash a0 = pixel_hash(fcx, fcy0), a1 = pixel_hash(fcx, fcy1);
+        pixh.p0 = a0.p0;
+        pixh.p0c = a0.p0c;
+        pixh.p1 = make_float2(a0.p1, a1.p1);
+        pixh.t1 = make_float2(a0.t1, a1.t1);
+    }
     // alpha state of the two pixels (x: pixel 0, y: pixel 1); pixels outside
     // the image start "done" (T = 0) and are never written
     float2 T = make_float2(in0 ? 1.0f : 0.0f, in1 ? 1.0f : 0.0f);
@@ -348,13 +316,16 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
     if (kStates)
 #pragma unroll
         for (int k = 0; k < 3 * (kStates ? kStates / 2 : 1); ++k) (&CS[0][0][0])[k] = (&CS[kStates ? 1 : 0][0][0])[k] = f2(0.0f);
-    StochState S0 = {16777215u, 0xFFFFFFFFu, 0.0f, 0.0f, 0.0f}, S1 = S0;
-    bool sdone0 = !in0, sdone1 = !in1;
-    Stoch2 P0, P1;
-    if (kMode == 2) {
-        stoch2_init(P0, in0);
-        stoch2_init(P1, in1);
+    // stochastic state of the pixels, per sample; pixels outside the image start
+    // with nothing left to find and are never written
+    constexpr int kSeeds = kMode == 2 ? 2 : 1;
+    StochState S0[2], S1[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        S0[k] = {in0 ? kFarD24 : 0u, 0xFFFFFFFFu, 0.0f, 0.0f, 0.0f};
+        S1[k] = {in1 ? kFarD24 : 0u, 0xFFFFFFFFu, 0.0f, 0.0f, 0.0f};
     }
+    uint32_t last_z = 0;   // D24 of the last splat this warp went through
     bool failed = false;
     const uint32_t nb = (n + kBatch - 1) / kBatch;
     uint32_t phase0 = 0, phase1 = 0;
@@ -374,8 +345,11 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
     };
     auto pixels_done = [&]() -> bool {
         if (kMode == 0) return fmaxf(T.x, T.y) < kTransmittanceMin;
-        if (kMode == 2) return P0.done[0] && P0.done[1] && P1.done[0] && P1.done[1];
-        return sdone0 && sdone1;
+        // a pixel's samples are decided once splats are beyond their kept depths
+        // (+ margin): no later one passes the depth test
+        uint32_t far = max(S0[0].best_d24, S1[0].best_d24);
+        if (kMode == 2) far = max(far, max(S0[1].best_d24, S1[1].best_d24));
+        return last_z > far + kDepthMargin;
     };
 
     if (nb > 0) issue(0);
@@ -408,17 +382,28 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
                            : (Mask)0;
                 cen_x = add(R->cx, p.jitter_x);
                 cen_y = add(R->cy, p.jitter_y);
-                sh.cen[i] = make_float4(cen_x, cen_y, add((float)R->splat_id, p.frame_seed), 0.0f);
             } else {
                 bits = rect_bits<kTw, kTh>(rr.x, rr.y, x0, y0);
                 cen_x = R->cx;
                 cen_y = R->cy;
             }
-            sh.bits[i] = bits;
-            if (kMode == 0) {
-                // coverage bits next to g, b: one 16-byte load per splat in the loop
-                const_cast<RasterRecord*>(R)->rect_x = (uint32_t)bits;
-                if (kRs == 32) const_cast<RasterRecord*>(R)->rect_y = (uint32_t)((unsigned long long)bits >> 32);
+            {
+                // what the loop wants of the record, in place: the coverage bits next to
+                // g, b and, in the stochastic modes, the sample's centre, the hash terms of
+                // the splat and the bound of alpha (once a record here, not once a warp)
+                RasterRecord* W = const_cast<RasterRecord*>(R);
+                W->rect_x = (uint32_t)bits;
+                if (kRs == 32) W->rect_y = (uint32_t)((unsigned long long)bits >> 32);
+                if (kMode == 1) {
+                    W->cx = cen_x;
+                    W->cy = cen_y;
+                }
+                if (kMode != 0) {
+                    const float id = (float)R->splat_id;
+                    W->log2_opacity = hash_z(add(id, p.frame_seed));
+                    if (kMode == 2) W->hash_z = hash_z(add(id, p.frame_seed2));
+                    W->rect_y = __float_as_uint(g_min(R->opacity, 0.99f));
+                }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             // block w = (w % kBx, w / kBx): bit w set iff its 8 columns and 8 rows are covered
@@ -450,33 +435,44 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
         __syncthreads();
         // Warp-uniform control flow only; per-pixel work is predicated.
         bool warp_done = __any_sync(0xffffffffu, failed) || __all_sync(0xffffffffu, pixels_done());
-        for (uint32_t c = 0; c < cnt && !warp_done; c += 32) {
-            const bool mine = c + lane < cnt && ((sh.mask[c + lane] >> warp) & 1u);
-            uint32_t todo = __ballot_sync(0xffffffffu, mine);
-            if (kMode == 0) {
-                // one splat of the warp's list into both pixels' state
-                auto alpha_one = [&](uint32_t j) {
-                    const float4 q0 = reinterpret_cast<const float4*>(&recs[j].r)[0];
-                    const float4 q1 = reinterpret_cast<const float4*>(&recs[j].r)[1];
-                    const uint4 q2u = reinterpret_cast<const uint4*>(&recs[j].r)[2];
-                    Mask bits;
-                    if (kRs == 32) bits = (Mask)((unsigned long long)q2u.z | ((unsigned long long)q2u.w << 32));
-                    else bits = (Mask)q2u.z;
-                    const float dx = sub(fcx, q0.x);
-                    const float t0 = mul(mul(q0.z, dx), dx);
-                    const float m = mul(q0.w, dx);
-                    const float2 dy = __fadd2_rn(fcy, f2(-q0.y));
-                    const float2 sq = __fadd2_rn(__fadd2_rn(f2(t0), __fmul2_rn(f2(m), dy)),
-                                                 __fmul2_rn(__fmul2_rn(f2(q1.x), dy), dy));
-                    const bool live0 = (bits & need0) == need0 && sq.x >= -__int_as_float(1) && sq.x <= q1.z;
-                    const bool live1 = (bits & need1) == need1 && sq.y >= -__int_as_float(1) && sq.y <= q1.z;
+        if (!warp_done) {
+            // the warp's list of the batch
+            uint16_t* list = sh.list[warp];
+            uint32_t mine_n = 0;
+            for (uint32_t c = 0; c < cnt; c += 32) {
+                const bool mine = c + lane < cnt && ((sh.mask[c + lane] >> warp) & 1u);
+                const uint32_t m = __ballot_sync(0xffffffffu, mine);
+                if (mine)
+                    list[mine_n + (uint32_t)__popc(m & ((1u << lane) - 1u))] =
+                        (uint16_t)((c + lane) * (uint32_t)sizeof(StagedRecord));
+                mine_n += (uint32_t)__popc(m);
+            }
+            __syncwarp();
+            // one splat of the list into both pixels' state
+            auto shade = [&](uint32_t off) {
+                const char* rec = reinterpret_cast<const char*>(recs) + off;
+                const float4 q0 = reinterpret_cast<const float4*>(rec)[0];
+                const float4 q1 = reinterpret_cast<const float4*>(rec)[1];
+                const uint4 q2u = reinterpret_cast<const uint4*>(rec)[2];
+                Mask bits;
+                if (kRs == 32) bits = (Mask)((unsigned long long)q2u.z | ((unsigned long long)q2u.w << 32));
+                else bits = (Mask)q2u.z;
+                const float dx = sub(fcx, q0.x);
+                const float t0 = mul(mul(q0.z, dx), dx);
+                const float m = mul(q0.w, dx);
+                const float2 dy = __fadd2_rn(fcy, f2(-q0.y));
+                const float2 sq = __fadd2_rn(__fadd2_rn(f2(t0), __fmul2_rn(f2(m), dy)),
+                                             __fmul2_rn(__fmul2_rn(f2(q1.x), dy), dy));
+                const bool live0 = frag_live(bits, need0, sq.x, q1.z);
+                const bool live1 = frag_live(bits, need1, sq.y, q1.z);
+                if constexpr (kMode == 0) {
                     const float2 q2 = make_float2(__uint_as_float(q2u.x), __uint_as_float(q2u.y));
                     const float2 arg = __ffma2_rn(sq, f2(kNegHalfLog2e), f2(q1.y));
                     const float a0 = live0 ? fminf(ex2_approx(arg.x), 0.99f) : 0.0f;
                     const float a1 = live1 ? fminf(ex2_approx(arg.y), 0.99f) : 0.0f;
                     const float2 w = __fmul2_rn(make_float2(a0, a1), T);
                     if constexpr (kStates > 0) {
-                        const float4* col = sh.col[b & 1][j];
+                        const float4* col = sh.col[b & 1][off / (uint32_t)sizeof(StagedRecord)];
                         const float2 w0 = f2(w.x), w1 = f2(w.y);
 #pragma unroll
                         for (int ch = 0; ch < 3; ++ch)
@@ -495,80 +491,70 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
                         C2 = __ffma2_rn(w, f2(q2.y), C2);
                     }
                     T = __ffma2_rn(w, f2(-1.0f), T);
-                };
-                // two splats per trip: one loop test and one warp vote per pair
-                while (todo) {
-                    const uint32_t j = c + (uint32_t)(__ffs(todo) - 1);
-                    todo &= todo - 1u;
-                    alpha_one(j);
-                    if (todo) {
-                        const uint32_t j2 = c + (uint32_t)(__ffs(todo) - 1);
-                        todo &= todo - 1u;
-                        alpha_one(j2);
-                    }
-                    if (__all_sync(0xffffffffu, pixels_done())) { warp_done = true; break; }
-                }
-                continue;
-            }
-            while (todo) {
-                const uint32_t j = c + (uint32_t)(__ffs(todo) - 1);
-                todo &= todo - 1u;
-                float4 q0 = reinterpret_cast<const float4*>(&recs[j].r)[0];
-                const float4 q1 = reinterpret_cast<const float4*>(&recs[j].r)[1];
-                const Mask bits = sh.bits[j];
-                float hz = 0.0f;
-                if (kMode == 1) {
-                    const float4 cz = sh.cen[j];
-                    q0.x = cz.x;
-                    q0.y = cz.y;
-                    hz = cz.z;
-                }
-                // splat_power()'s sum for both pixels with the shared first term
-                const float dx = sub(fcx, q0.x);
-                const float t0 = mul(mul(q0.z, dx), dx);
-                const float m = mul(q0.w, dx);
-                const float2 dy = __fadd2_rn(fcy, f2(-q0.y));
-                const float2 sq = __fadd2_rn(__fadd2_rn(f2(t0), __fmul2_rn(f2(m), dy)),
-                                             __fmul2_rn(__fmul2_rn(f2(q1.x), dy), dy));
-                const bool live0 = (bits & need0) == need0 && sq.x >= -__int_as_float(1) && sq.x <= q1.z;
-                const bool live1 = (bits & need1) == need1 && sq.y >= -__int_as_float(1) && sq.y <= q1.z;
-                if (kMode == 0) {
-                    const float2 q2 = reinterpret_cast<const float2*>(&recs[j].r)[4];
-                    const float2 arg = __ffma2_rn(sq, f2(kNegHalfLog2e), f2(q1.y));
-                    const float a0 = live0 ? fminf(ex2_approx(arg.x), 0.99f) : 0.0f;
-                    const float a1 = live1 ? fminf(ex2_approx(arg.y), 0.99f) : 0.0f;
-                    const float2 w = __fmul2_rn(make_float2(a0, a1), T);
-                    C0 = __ffma2_rn(w, f2(q1.w), C0);
-                    C1 = __ffma2_rn(w, f2(q2.x), C1);
-                    C2 = __ffma2_rn(w, f2(q2.y), C2);
-                    T = __ffma2_rn(w, f2(-1.0f), T);
-                    if (__all_sync(0xffffffffu, pixels_done())) { warp_done = true; break; }
-                } else if (kMode == 2) {
-                    const uint4 q3 = reinterpret_cast<const uint4*>(&recs[j].r)[3];
-                    const uint32_t z24 = q3.x, id = q3.y;
-                    stoch2_retire(P0, z24, kDepthMargin);
-                    stoch2_retire(P1, z24, kDepthMargin);
-                    if (__all_sync(0xffffffffu, pixels_done())) { warp_done = true; break; }
-                    const float2 q2 = reinterpret_cast<const float2*>(&recs[j].r)[4];
-                    const float op = __uint_as_float(q3.w);
-                    const float hz0 = hash_z(add((float)id, p.frame_seed)), hz1 = hash_z(add((float)id, p.frame_seed2));
-                    stoch2_step(P0, live0, sq.x, op, ph0, hz0, hz1, z24, id, q1.w, q2.x, q2.y);
-                    stoch2_step(P1, live1, sq.y, op, ph1, hz0, hz1, z24, id, q1.w, q2.x, q2.y);
                 } else {
-                    const uint4 q3 = reinterpret_cast<const uint4*>(&recs[j].r)[3];
+                    const float2 q2 = make_float2(__uint_as_float(q2u.x), __uint_as_float(q2u.y));
+                    const uint4 q3 = reinterpret_cast<const uint4*>(rec)[3];
                     const uint32_t z24 = q3.x, id = q3.y;
-                    // a pixel stops once splats are beyond its kept depth (+ margin)
-                    if (S0.best_id != 0xFFFFFFFFu && z24 > S0.best_d24 + kDepthMargin) sdone0 = true;
-                    if (S1.best_id != 0xFFFFFFFFu && z24 > S1.best_d24 + kDepthMargin) sdone1 = true;
-                    if (__all_sync(0xffffffffu, pixels_done())) { warp_done = true; break; }
-                    const bool b0 = z24 < S0.best_d24 || (z24 == S0.best_d24 && id < S0.best_id);
-                    const bool b1 = z24 < S1.best_d24 || (z24 == S1.best_d24 && id < S1.best_id);
-                    const float2 q2 = reinterpret_cast<const float2*>(&recs[j].r)[4];
-                    const float op = __uint_as_float(q3.w);
-                    const float hzf = hash_z(hz);
-                    if (live0 && !sdone0 && b0) stoch_step(S0, sq.x, op, ph0, hzf, z24, id, q1.w, q2.x, q2.y);
-                    if (live1 && !sdone1 && b1) stoch_step(S1, sq.y, op, ph1, hzf, z24, id, q1.w, q2.x, q2.y);
+                    last_z = z24;
+                    // The depth test first (the tie by index only for a fragment that is
+                    // kept), then the hashes, and the exponential for those below alpha's
+                    // bound: alpha = min(opacity * exp(power), 0.99) with power <= 0 (exp <= 1
+                    // there, also for the deterministic exp) never exceeds min(opacity, 0.99).
+                    bool want0[kSeeds], want1[kSeeds], any = false;
+#pragma unroll
+                    for (int k = 0; k < kSeeds; ++k) {
+                        want0[k] = live0 && z24 <= S0[k].best_d24;
+                        want1[k] = live1 && z24 <= S1[k].best_d24;
+                        any = any || want0[k] || want1[k];
+                    }
+                    if (any) {
+                        const float bound = __uint_as_float(q2u.w), op = __uint_as_float(q3.w);
+                        float2 rnd[kSeeds];
+                        bool any0 = false, any1 = false;
+#pragma unroll
+                        for (int k = 0; k < kSeeds; ++k) {
+                            rnd[k] = hash13(pixh, k ? __uint_as_float(q3.z) : q1.y);
+                            want0[k] = want0[k] && rnd[k].x < bound;
+                            want1[k] = want1[k] && rnd[k].y < bound;
+                            any0 = any0 || want0[k];
+                            any1 = any1 || want1[k];
+                        }
+                        auto keep = [&](StochState& S, bool want, float r, float alpha) {
+                            if (want && r < alpha && (z24 < S.best_d24 || id < S.best_id))
+                                S = {z24, id, q1.w, q2.x, q2.y};
+                        };
+                        if (any0) {
+                            const float alpha = g_min(mul(op, det_expf(mul(-0.5f, sq.x))), 0.99f);
+#pragma unroll
+                            for (int k = 0; k < kSeeds; ++k) keep(S0[k], want0[k], rnd[k].x, alpha);
+                        }
+                        if (any1) {
+                            const float alpha = g_min(mul(op, det_expf(mul(-0.5f, sq.y))), 0.99f);
+#pragma unroll
+                            for (int k = 0; k < kSeeds; ++k) keep(S1[k], want1[k], rnd[k].y, alpha);
+                        }
+                    }
                 }
+            };
+            // kTrip splats per trip: one load of their offsets, one loop test and one
+            // warp vote (trips of 2 / 4 / 8 measured at 3M room 1080p: alpha 269 / 266 /
+            // 255 us, four stochastic samples 1390 / 1357 / 1475 us; eight state frames of
+            // 1M take 1577 / 1515 / 1480 us a batch; 16 to a trip was slower again, 264 us)
+            constexpr uint32_t kTrip = kMode == 0 ? 8 : kMode == 1 ? 4 : 2;
+            struct __align__(2 * kTrip) Trip { uint32_t pair[kTrip / 2]; };
+            uint32_t k = 0;
+            for (; k + kTrip <= mine_n; k += kTrip) {
+                const Trip t = *reinterpret_cast<const Trip*>(list + k);
+#pragma unroll
+                for (uint32_t i = 0; i < kTrip / 2; ++i) {
+                    shade(t.pair[i] & 0xFFFFu);
+                    shade(t.pair[i] >> 16);
+                }
+                if (__all_sync(0xffffffffu, pixels_done())) { warp_done = true; break; }
+            }
+            if (!warp_done) {
+                for (; k < mine_n; ++k) shade(list[k]);
+                warp_done = __all_sync(0xffffffffu, pixels_done());
             }
         }
         const int all_done = __syncthreads_and(warp_done || pixels_done() || failed);
@@ -604,14 +590,22 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
         if (in0) write_rgba16f(p.out_rgba16f, o0, r.x, g.x, bb.x, 1.0f - T.x);
         if (in1) write_rgba16f(p.out_rgba16f, o1, r.y, g.y, bb.y, 1.0f - T.y);
     } else if (kMode == 2) {
-        if (in0) write_pixel_stoch2(p, px, py0, P0);
-        if (in1) write_pixel_stoch2(p, px, py1, P1);
+        if (in0) write_pixel_stoch2(p, px, py0, S0);
+        if (in1) write_pixel_stoch2(p, px, py1, S1);
     } else {
-        if (in0) write_pixel_stoch(p, px, py0, S0);
-        if (in1) write_pixel_stoch(p, px, py1, S1);
+        if (in0) write_pixel_stoch(p, px, py0, S0[0]);
+        if (in1) write_pixel_stoch(p, px, py1, S1[0]);
     }
 }
 
+// Bound by instructions issued, the ALU pipe (comparisons, selects, integers) first
+// of the pipes at 64 %: one splat into two pixels is some 40 instructions, of
+// which the fused multiply-adds, packed two pixels to one, are the smaller part.
+// What is the same for the pixels of a warp is therefore done once a record in
+// the staging pass, the warp's splats are listed before they are shaded, and the
+// stochastic modes leave a pixel's termination to the warp's vote.  3M Gaussians,
+// room, 1920x1080: alpha 310 -> 255 us, four stochastic samples 1644 -> 1357 us,
+// two samples and their fallback (denoised mode) 1057 -> 796 us.
 template <int kMode, int kTw = 16, int kTh = 16>
 __global__ void __launch_bounds__(kRasterThreads) raster_kernel(RasterParams p) {
     pdl_wait();

@@ -478,8 +478,8 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
                         const int ty = (a.h + a.row_offset) / 16 - 1 - band;   // GL tile row of this band
                         const uint32_t tile = (uint32_t)(ty * a.tiles_x + tx);
                         const float mse = err_sum / err_cnt * 0.001f;
-                        if (a.tile_err) a.tile_err[tile] = mse;
-                        if (mse >= a.err_budget) a.fallback_tiles[atomicAdd(a.fallback_count, 1u)] = tile;
+                        a.tile_err[tile] = mse;
+                        if (mse >= a.err_budget) atomicAdd(a.fallback_count, 1u);
                     }
                     err_sum = err_cnt = 0.0f;
                 }

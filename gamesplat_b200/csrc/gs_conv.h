@@ -31,12 +31,11 @@ struct ConvArgs {
     // Denoised-mode head (Cout = 16, forward, head_x set): the epilogue writes head_out16 =
     // RGBA16F (head_x[5..7] + o[0..2], head_x[3] + o[3]) instead of the outputs above and,
     // per 16x16 tile of GL rows (unit_rows = 16 and row_offset aligning the bands with
-    // them), tile_err = mean(max(o[4], 0)) * 0.001, listing tiles at or above err_budget.
+    // them), tile_err = mean(max(o[4], 0)) * 0.001, counting tiles at or above err_budget.
     const __nv_bfloat16* head_x;   // the network input (16 channels per pixel)
     uint16_t* head_out16;
     float* tile_err;
     uint32_t* fallback_count;
-    uint32_t* fallback_tiles;
     float err_budget;
     int tiles_x;
 };

@@ -210,8 +210,8 @@ int forward(gs_denoiser* d, const bf16* x, int n, int h, int w, cudaStream_t s) 
 }
 
 int forward_frame(gs_denoiser* d, const bf16* x, int h, int w, uint16_t* out16, int tiles_x, float err_budget,
-                  uint32_t* fallback_count, uint32_t* fallback_tiles, float* tile_err, cudaStream_t s) {
-    if (h <= 0 || w <= 0 || (h & 1) || (w & 1) || !out16 || !fallback_count || !fallback_tiles) return GS_ERR_BAD_ARG;
+                  uint32_t* fallback_count, float* tile_err, cudaStream_t s) {
+    if (h <= 0 || w <= 0 || (h & 1) || (w & 1) || !out16 || !fallback_count || !tile_err) return GS_ERR_BAD_ARG;
     int rc = ensure_acts(d, (size_t)h * w);
     if (rc) return rc;
     d->last_x = nullptr;   // the activations are this frame's now: no backward pass follows
@@ -240,7 +240,6 @@ int forward_frame(gs_denoiser* d, const bf16* x, int h, int w, uint16_t* out16, 
     a.head_out16 = out16;
     a.tile_err = tile_err;
     a.fallback_count = fallback_count;
-    a.fallback_tiles = fallback_tiles;
     a.err_budget = err_budget;
     a.tiles_x = tiles_x;
     return conv::launch_fwd(L.cin, L.cout, L.load, a, s) < 0 ? GS_ERR_BAD_ARG : GS_OK;

@@ -25,11 +25,10 @@ const float* output(const gs_denoiser* d);
 // layer writes the RGBA16F image out16 (the input's history RGB and alpha plus
 // the network's correction) and, per 16x16 tile (tiles_x across, GL rows from
 // the bottom), tile_err = the estimated mean squared error; tiles at or above
-// err_budget are appended to fallback_tiles (count in *fallback_count).  The
-// last layer's 16 output channels are not stored.
+// err_budget are counted in *fallback_count.  The last layer's 16 output
+// channels are not stored.
 int forward_frame(gs_denoiser* d, const __nv_bfloat16* x, int h, int w, uint16_t* out16, int tiles_x,
-                  float err_budget, uint32_t* fallback_count, uint32_t* fallback_tiles, float* tile_err,
-                  cudaStream_t s);
+                  float err_budget, uint32_t* fallback_count, float* tile_err, cudaStream_t s);
 
 }  // namespace dn
 }  // namespace gs

@@ -199,8 +199,8 @@ struct gs_ctx {
     gs_denoiser* denoiser = nullptr;
     __nv_bfloat16* features = nullptr;
     size_t features_pix = 0;
-    uint32_t* fallback_tiles = nullptr;   // tiles_cap entries
-    float* tile_error = nullptr;          // tiles_cap estimated MSE per tile
+    float* tile_error = nullptr;          // tile_error_cap estimated MSE per tile
+    uint32_t tile_error_cap = 0;
     float denoise_budget = 1.0e-4f;       // tile MSE budget: 40 dB PSNR
     int denoise_fallback = 1;
 
@@ -391,7 +391,6 @@ void release_targets(gs_ctx* c) {
     c->ctrl_read_pending = c->alt.read_pending = false;
     dfree(c->tile_order);
     dfree(c->features);
-    dfree(c->fallback_tiles);
     dfree(c->tile_error);
     c->features_pix = 0;
     c->fc = nullptr;
@@ -1039,13 +1038,15 @@ int ensure_denoise_targets(gs_ctx* c) {
     const size_t npix = (size_t)c->width * c->height;
     if (c->features_pix != npix || !c->features) {
         dfree(c->features);
-        dfree(c->fallback_tiles);
-        dfree(c->tile_error);
-        c->features_pix = 0;
+            c->features_pix = 0;
         GS_CUDA(c, dalloc(&c->features, npix * gs::dn::kInC * sizeof(__nv_bfloat16)));
-        GS_CUDA(c, dalloc(&c->fallback_tiles, (size_t)c->tiles_cap * sizeof(uint32_t)));
-        GS_CUDA(c, dalloc(&c->tile_error, (size_t)c->tiles_cap * sizeof(float)));
         c->features_pix = npix;
+    }
+    if (c->tile_error_cap < c->tiles_cap || !c->tile_error) {   // the same pixels can be more tiles
+        dfree(c->tile_error);
+        c->tile_error_cap = 0;
+        GS_CUDA(c, dalloc(&c->tile_error, (size_t)c->tiles_cap * sizeof(float)));
+        c->tile_error_cap = c->tiles_cap;
     }
     return GS_OK;
 }
@@ -1107,15 +1108,15 @@ int render_denoised(gs_ctx* c, const gs_camera* cam, uint16_t* out) {
         // the network, its last layer writing the frame and the tiles' error estimates
         rc = gs::dn::forward_frame(c->denoiser, c->features, c->height, c->width, out, c->tiles_x,
                                    c->denoise_fallback ? c->denoise_budget : 3.0e38f, &c->fc->fallback_tiles,
-                                   c->fallback_tiles, c->tile_error, c->stream);
+                                   c->tile_error, c->stream);
         if (rc) return fail(c, rc, "denoiser forward failed");
         sd.add(5);
     }
     if (c->denoise_fallback) {
         StageScope sc(c, ST_RASTER);
         gs::RasterParams r = raster_params(c, background(c));
-        r.tile_order = c->fallback_tiles;
-        r.tile_count = &c->fc->fallback_tiles;
+        r.tile_err = c->tile_error;
+        r.err_budget = c->denoise_budget;
         r.out_rgba16f = out;
         sc.add(gs::launch_raster_alpha(r, c->stream));
     }

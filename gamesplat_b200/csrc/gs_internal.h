@@ -199,7 +199,8 @@ struct RasterParams {
     const SortPlan* tile_plan;       // tile-sorted entry values at tile_plan->vfinal
     const uint2* tile_ranges;        // [start, end) per tile
     const uint32_t* tile_order;      // tiles by descending work (CTA b rasterizes tile_order[b])
-    const uint32_t* tile_count;      // optional: CTAs b >= *tile_count do nothing (a tile list of the frame)
+    const float* tile_err;           // optional: only tiles with tile_err[tile] >= err_budget are drawn
+    float err_budget;
     const float4* colours;           // state batches: per record the colours of kStates frames (StateBatch)
     int width, height, tiles_x, tiles_y;
     int tile_w, tile_h;              // tile shape: 16x16, or 32x8 / 8x32 (alpha mode)

@@ -610,8 +610,12 @@ template <int kMode, int kTw = 16, int kTh = 16>
 __global__ void __launch_bounds__(kRasterThreads) raster_kernel(RasterParams p) {
     pdl_wait();
     __shared__ RasterShared<kMode, kTw, kTh> sh;
-    if (p.tile_count && blockIdx.x >= *p.tile_count) return;
-    raster_tile<kMode, kTw, kTh>(p, p.tile_order[blockIdx.x], sh);
+    const uint32_t tile = p.tile_order[blockIdx.x];
+    // denoised mode's fallback: all tiles in the frame's order, heaviest first, those
+    // within the budget leaving at once (a list of the others in the order in which
+    // the network finished them left the SMs idle for a third of the pass)
+    if (p.tile_err && !(p.tile_err[tile] >= p.err_budget)) return;
+    raster_tile<kMode, kTw, kTh>(p, tile, sh);
 }
 
 // Many frames in one persistent launch: work item w is tile

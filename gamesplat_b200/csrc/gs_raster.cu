@@ -11,18 +11,21 @@
 // walked front to back (reverse of the reference's back-to-front draw order,
 // so equal depth keys are visited in descending splat index, which
 // reproduces "later instance on top").  Batches of 128 64-byte RasterRecords
-// are staged into shared memory by TMA 1-D bulk copies (cp.async.bulk,
-// completion on an mbarrier), double buffered so the next batch lands while
-// the current one is composited.  When a batch lands, one thread per record turns its pixel
-// rectangle into tile-relative column and row bit masks, so a pixel's
-// coverage test is one AND and one compare (in alpha mode the mask is also
-// written into the staged record next to g, b: one 16-byte load per splat).
+// are gathered into shared memory by cp.async, 16 bytes a lane, double buffered
+// so the next batch lands while the current one is composited.  (One TMA bulk
+// copy a record is one instruction where this takes four, but the copy engine of
+// an SM works off some one every 11 cycles, and that was what the rasterizers
+// waited for: 250 us against 210 us for 3M Gaussians in the room at 1080p, 644
+// against 531 us for 6M at 2160p.)  When a batch lands, one thread per record
+// turns its pixel rectangle into tile-relative column and row bit masks, written
+// into the staged record next to g, b, so a pixel's coverage test is one
+// operation; drops the 8x8 blocks that its ellipse cannot reach; and each warp
+// lists the records it has to shade.
 //
 // The two pixels of a thread share a column; their arithmetic runs as packed
 // f32x2 operations (add/mul/fma .rn on float pairs, each element rounded like
 // the scalar operation), which halves the issue slots of the per-pixel math.
-// In alpha mode a warp takes its splats two per loop trip (one loop test and
-// one "all pixels done" vote per pair).  CTA b rasterizes tile
+// CTA b rasterizes tile
 // tile_order[b]: the heaviest tiles first, so they do not form the last wave.
 //
 // Alpha mode: premultiplied "over" in FP32, front to back:
@@ -55,7 +58,6 @@
 
 #include "gs_common.cuh"
 #include "gs_internal.h"
-#include "gs_tma.cuh"
 
 namespace gs {
 
@@ -98,6 +100,15 @@ __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
 }
 
 __device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
@@ -209,33 +220,27 @@ __device__ __forceinline__ typename TileShape<kTw, kTh>::Mask rect_bits(uint32_t
     return (M)(cols | (rows << S::kRowShift));
 }
 
-// Lower bound of the splat's quadratic form q(d) = A dx^2 + B dx dy + C dy^2
-// over the box [X0,X1] x [Y0,Y1] of pixel-centre offsets.  With A, C > 0, q is
-// convex along every box edge, and when the box does not hold the origin its
-// minimum lies on an edge (a convex q has its only interior stationary point
-// at the origin; an indefinite one has none that is a minimum), at the
-// clamped stationary point of that edge's 1-D quadratic.
-__device__ __forceinline__ float min_q_box(float A, float B, float C, float X0, float X1, float Y0, float Y1) {
-    if (X0 <= 0.0f && X1 >= 0.0f && Y0 <= 0.0f && Y1 >= 0.0f) return 0.0f;
-    const float ia = -0.5f * B / A, ic = -0.5f * B / C;
-    float m = 3.0e38f;
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const float X = e ? X1 : X0, Y = e ? Y1 : Y0;
-        const float dy = fminf(fmaxf(ic * X, Y0), Y1);
-        m = fminf(m, fmaf(fmaf(C, dy, B * X), dy, A * X * X));
-        const float dx = fminf(fmaxf(ia * Y, X0), X1);
-        m = fminf(m, fmaf(fmaf(A, dx, B * Y), dx, C * Y * Y));
-    }
-    return m;
+// Minimum of the splat's quadratic form q(d) = A dx^2 + B dx dy + C dy^2 (A, C > 0)
+// over the box [X0,X1] x [Y0,Y1] of pixel-centre offsets, or more where that
+// is above every value in [0, inf) that q takes there: q(t d) = t^2 q(d), so a point of
+// the box with such a value has one no larger on an edge that faces the
+// origin, and along an edge q is convex with its minimum at the clamped
+// stationary point.  X and Y are those edges' coordinates; a box that spans an
+// axis gives an inner line instead, one that holds the origin gives q(0) = 0.
+// ia = -B / 2A, ic = -B / 2C.
+__device__ __forceinline__ float min_q_box(float A, float B, float C, float ia, float ic, float X0, float X1, float Y0,
+                                           float Y1) {
+    const float X = fminf(fmaxf(0.0f, X0), X1), Y = fminf(fmaxf(0.0f, Y0), Y1);
+    const float dy = fminf(fmaxf(ic * X, Y0), Y1), dx = fminf(fmaxf(ia * Y, X0), X1);
+    return fminf(fmaf(fmaf(C, dy, B * X), dy, A * X * X), fmaf(fmaf(A, dx, B * Y), dx, C * Y * Y));
 }
 
 // One CTA of 128 threads per 16x16 tile; warp w owns the 8x8 block
 // (w & 1, w >> 1); lane l shades pixels (l & 7, l >> 3) and (l & 7, (l >> 3) + 4)
 // of it: the two pixels share a column, hence dx, the column test and the
 // first term of the Gaussian exponent.
-// Shared memory of one CTA's tile: two staging buffers of records, their
-// barriers, the records' warp-block masks and the warps' lists.
+// Shared memory of one CTA's tile: two staging buffers of records, the records'
+// warp-block masks and the warps' lists.
 // A staged record and 16 bytes of padding: at an 80-byte stride the 16-byte
 // loads of 8 consecutive records (one record per thread in the staging pass)
 // fall in distinct banks, and a 32-bit field of 32 consecutive records spreads
@@ -258,7 +263,6 @@ struct StateColours<0> {};
 template <int kMode, int kTw = 16, int kTh = 16, int kStates = 0>
 struct __align__(128) RasterShared : StateColours<kStates> {
     StagedRecord rec[2][kBatch];
-    uint64_t bar[2];
     uint8_t mask[kBatch];
     // per warp the staged records it shades, as byte offsets from the first, nearest first
     __align__(16) uint16_t list[4][kBatch];
@@ -288,13 +292,6 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
     const uint2 range = p.tile_ranges[tile];
     const uint32_t n = range.y > range.x ? range.y - range.x : 0u;
     const uint32_t* __restrict__ vals = p.tile_plan->vfinal;
-
-    if (threadIdx.x == 0) {
-        mbar_init(&sh.bar[0], 1);
-        mbar_init(&sh.bar[1], 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
 
     const float fcx = (float)px + 0.5f, fcy0 = (float)py0 + 0.5f, fcy1 = (float)py1 + 0.5f;
     const float2 fcy = make_float2(fcy0, fcy1);
@@ -326,21 +323,36 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
         S1[k] = {in1 ? kFarD24 : 0u, 0xFFFFFFFFu, 0.0f, 0.0f, 0.0f};
     }
     uint32_t last_z = 0;   // D24 of the last splat this warp went through
-    bool failed = false;
     const uint32_t nb = (n + kBatch - 1) / kBatch;
-    uint32_t phase0 = 0, phase1 = 0;
 
+    // A warp copies the 32 records of a batch that it stages, 4 lanes a record
+    // (16 bytes each); the list entries of the next batch are loaded a batch ahead.
+    static_assert(kBatch == kRasterThreads, "one record a thread in the staging pass");
+    auto entry = [&](uint32_t b) -> uint32_t {
+        const uint32_t i = b * kBatch + threadIdx.x;
+        return i < n ? min(vals[range.x + i], p.record_cap - 1u) : 0u;
+    };
+    uint32_t ahead = entry(0);
     auto issue = [&](uint32_t b) {
-        const uint32_t first = b * kBatch;
-        const uint32_t cnt = min((uint32_t)kBatch, n - first);
-        uint64_t* bar = &sh.bar[b & 1];
-        constexpr uint32_t kColBytes = 12u * kStates;
-        if (threadIdx.x == 0) mbar_arrive_expect_tx(bar, cnt * ((uint32_t)sizeof(RasterRecord) + kColBytes));
-        for (uint32_t i = threadIdx.x; i < cnt; i += kRasterThreads) {
-            const uint32_t s = min(vals[range.x + first + i], p.record_cap - 1u);
-            bulk_g2s(&sh.rec[b & 1][i].r, p.records + s, (uint32_t)sizeof(RasterRecord), bar);
-            if constexpr (kStates > 0)
-                bulk_g2s(&sh.col[b & 1][i][0], p.colours + (size_t)s * (kColBytes / 16), kColBytes, bar);
+        const uint32_t cnt = min((uint32_t)kBatch, n - b * kBatch);
+        const uint32_t mine = ahead;
+        ahead = entry(b + 1);
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t r = 8 * j + (lane >> 2), i = warp * 32 + r;
+            const uint32_t s = __shfl_sync(0xffffffffu, mine, r);
+            if (i < cnt)
+                cp_async16(reinterpret_cast<uint4*>(&sh.rec[b & 1][i].r) + (lane & 3),
+                           reinterpret_cast<const uint4*>(p.records + s) + (lane & 3));
+        }
+        if constexpr (kStates > 0) {
+            constexpr uint32_t kQ = 3 * kStates / 4;   // 16-byte pieces of a record's colours
+#pragma unroll
+            for (uint32_t j = 0; j < kQ; ++j) {
+                const uint32_t r = (32 * j + lane) / kQ, q = (32 * j + lane) % kQ, i = warp * 32 + r;
+                const uint32_t s = __shfl_sync(0xffffffffu, mine, r);
+                if (i < cnt) cp_async16(&sh.col[b & 1][i][q], p.colours + (size_t)s * kQ + q);
+            }
         }
     };
     auto pixels_done = [&]() -> bool {
@@ -353,11 +365,12 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
     };
 
     if (nb > 0) issue(0);
+    cp_async_commit();
     for (uint32_t b = 0; b < nb; ++b) {
         if (b + 1 < nb) issue(b + 1);
-        const uint32_t ph = (b & 1) ? phase1 : phase0;
-        if (!mbar_wait_bounded(&sh.bar[b & 1], ph)) failed = true;
-        if (b & 1) phase1 ^= 1u; else phase0 ^= 1u;
+        cp_async_commit();
+        cp_async_wait<1>();
+        __syncwarp();
         const uint32_t cnt = min((uint32_t)kBatch, n - b * kBatch);
         const StagedRecord* recs = sh.rec[b & 1];
         // Coverage bits of each staged record and which of the four 8x8 warp
@@ -365,7 +378,7 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
         // touches, minus those where the splat's ellipse q(d) <= s_max misses
         // every covered pixel centre (tested with a 2 % + 0.02 margin over
         // s_max, far above the rounding of q and of the exact per-pixel sum).
-        for (uint32_t i = threadIdx.x; i < cnt; i += kRasterThreads) {
+        if (const uint32_t i = threadIdx.x; i < cnt) {
             const RasterRecord* R = &recs[i].r;
             const uint2 rr = reinterpret_cast<const uint2*>(R)[5];
             Mask bits;
@@ -404,7 +417,6 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
                     if (kMode == 2) W->hash_z = hash_z(add(id, p.frame_seed2));
                     W->rect_y = __float_as_uint(g_min(R->opacity, 0.99f));
                 }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             // block w = (w % kBx, w / kBx): bit w set iff its 8 columns and 8 rows are covered
             uint32_t blocks = 0u;
@@ -417,6 +429,7 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
             const float2 q1 = reinterpret_cast<const float2*>(R)[2];
             const float A = q0.z, B = q0.w, C = q1.x;
             if (blocks && A > 0.0f && C > 0.0f) {
+                const float ia = __fdividef(-0.5f * B, A), ic = __fdividef(-0.5f * B, C);
                 const float thr = fmaf(R->s_max, 1.02f, 0.02f);
                 for (uint32_t todo_w = blocks; todo_w; todo_w &= todo_w - 1u) {
                     const int w = __ffs(todo_w) - 1;
@@ -425,7 +438,7 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
                     const uint32_t rb = (uint32_t)(bits >> (kRs + 8 * byw)) & 0xFFu;
                     const float bx = (float)(x0 + 8 * bxw) + 0.5f - cen_x;
                     const float by = (float)(y0 + 8 * byw) + 0.5f - cen_y;
-                    const float m = min_q_box(A, B, C, bx + (float)(__ffs(cb) - 1), bx + (float)(31 - __clz(cb)),
+                    const float m = min_q_box(A, B, C, ia, ic, bx + (float)(__ffs(cb) - 1), bx + (float)(31 - __clz(cb)),
                                               by + (float)(__ffs(rb) - 1), by + (float)(31 - __clz(rb)));
                     if (m > thr) blocks &= ~(1u << w);
                 }
@@ -434,7 +447,7 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
         }
         __syncthreads();
         // Warp-uniform control flow only; per-pixel work is predicated.
-        bool warp_done = __any_sync(0xffffffffu, failed) || __all_sync(0xffffffffu, pixels_done());
+        bool warp_done = __all_sync(0xffffffffu, pixels_done());
         if (!warp_done) {
             // the warp's list of the batch
             uint16_t* list = sh.list[warp];
@@ -557,16 +570,9 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
                 warp_done = __all_sync(0xffffffffu, pixels_done());
             }
         }
-        const int all_done = __syncthreads_and(warp_done || pixels_done() || failed);
-        if (all_done) {
-            if (b + 1 < nb) {
-                const uint32_t ph2 = ((b + 1) & 1) ? phase1 : phase0;
-                if (!mbar_wait_bounded(&sh.bar[(b + 1) & 1], ph2)) failed = true;
-            }
-            break;
-        }
+        if (__syncthreads_and(warp_done)) break;
     }
-    if (failed) atomicOr(&p.fc->error_flags, kErrRasterWait);
+    cp_async_wait<0>();   // a batch that was not needed
     if constexpr (kStates > 0) {
         const size_t o0 = (size_t)(p.height - 1 - py0) * p.width + px;
         const size_t o1 = (size_t)(p.height - 1 - py1) * p.width + px;
@@ -603,9 +609,10 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
 // which the fused multiply-adds, packed two pixels to one, are the smaller part.
 // What is the same for the pixels of a warp is therefore done once a record in
 // the staging pass, the warp's splats are listed before they are shaded, and the
-// stochastic modes leave a pixel's termination to the warp's vote.  3M Gaussians,
-// room, 1920x1080: alpha 310 -> 255 us, four stochastic samples 1644 -> 1357 us,
-// two samples and their fallback (denoised mode) 1057 -> 796 us.
+// stochastic modes leave a pixel's termination to the warp's vote.  Room of 3M
+// Gaussians, 1920x1080: alpha 310 -> 210 us, four stochastic samples 1644 -> 1200
+// us, two samples and their fallback (denoised mode) 1057 -> 605 us; 6M at
+// 3840x2160 798 -> 531 us.
 template <int kMode, int kTw = 16, int kTh = 16>
 __global__ void __launch_bounds__(kRasterThreads) raster_kernel(RasterParams p) {
     pdl_wait();

@@ -553,7 +553,7 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
             // warp vote (trips of 2 / 4 / 8 measured at 3M room 1080p: alpha 269 / 266 /
             // 255 us, four stochastic samples 1390 / 1357 / 1475 us; eight state frames of
             // 1M take 1577 / 1515 / 1480 us a batch; 16 to a trip was slower again, 264 us)
-            constexpr uint32_t kTrip = kMode == 0 ? 8 : kMode == 1 ? 4 : 2;
+            constexpr uint32_t kTrip = kMode == 0 ? 8 : 4;
             struct __align__(2 * kTrip) Trip { uint32_t pair[kTrip / 2]; };
             uint32_t k = 0;
             for (; k + kTrip <= mine_n; k += kTrip) {

@@ -26,6 +26,7 @@
 #include <type_traits>
 
 #include "gs_common.cuh"
+#include "gs_copy.cuh"
 #include "gs_internal.h"
 #include "gs_tma.cuh"
 
@@ -232,15 +233,11 @@ __device__ __forceinline__ void project_visible(const float4* row, float4 c0, fl
 }
 
 // Stage one group of 32 compacted visible rows: lane l copies the first
-// kChunks 16-byte chunks of row ids[first + l] (if first + l < count) to
-// stage row l with one TMA bulk copy; completion is counted on `bar`.
-// Returns the lane's row id, or kSentinel past the end.
-template <int kChunks, int kRowChunks = 16, int kStride = kStageStride>
-__device__ __forceinline__ uint32_t stage_group(const float4* rows, const uint32_t* ids, uint32_t first,
-                                                uint32_t count, float4* stage, uint64_t* bar, int lane,
-                                                uint64_t policy) {
-    const uint32_t idx = first + (uint32_t)lane;
-    const uint32_t id = idx < count ? ids[idx] : kSentinel;
+// kChunks 16-byte chunks of row `id` (kSentinel: none) to stage row l with one
+// TMA bulk copy; completion is counted on `bar`.
+template <int kChunks>
+__device__ __forceinline__ void stage_group(const float4* rows, uint32_t id, float4* stage, uint64_t* bar, int lane,
+                                            uint64_t policy) {
     const uint32_t mask = __ballot_sync(0xffffffffu, id != kSentinel);
     if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)__popc(mask) * (uint32_t)(kChunks * 16));
     __syncwarp();
@@ -248,8 +245,26 @@ __device__ __forceinline__ uint32_t stage_group(const float4* rows, const uint32
     // the in-place gsanim deltas) before the async-proxy refill
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (id != kSentinel)
-        bulk_g2s_hint(stage + lane * kStride, rows + (size_t)id * kRowChunks, (uint32_t)(kChunks * 16), bar, policy);
-    return id;
+        bulk_g2s_hint(stage + lane * kStageStride, rows + (size_t)id * 16, (uint32_t)(kChunks * 16), bar, policy);
+}
+
+// The same for 144-byte FP16-SH rows, by cp.async: 9 chunks a row over the
+// warp's lanes; complete, for the whole warp, on return.  An SM's copy engine
+// works off some one bulk copy every 11 cycles, less than these short rows
+// need: 6M Gaussians of the room (4M visible) take 276 us in the cull stage
+// against 290, while 256-byte rows are 5 us faster by bulk copy at 3M.
+__device__ __forceinline__ void stage_half_group(const float4* rows, uint32_t id, float4* stage, int lane,
+                                                 uint64_t policy) {
+#pragma unroll
+    for (int j = 0; j < kHalfRowChunks; ++j) {
+        const int r = (32 * j + lane) / kHalfRowChunks, c = (32 * j + lane) % kHalfRowChunks;
+        const uint32_t row = __shfl_sync(0xffffffffu, id, r);
+        if (row != kSentinel)
+            cp_async16_hint(stage + r * kHalfStageStride + c, rows + (size_t)row * kHalfRowChunks + c, policy);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncwarp();
 }
 
 // gsanim int8 appearance deltas applied in place to a staged row
@@ -479,12 +494,19 @@ __global__ void __launch_bounds__(kCullThreads, 6) cull_project_kernel(CullParam
     // the base state), and (1 - w) x + w x need not round to x
     const bool animated = p.anim_deltas != nullptr && (p.anim_state_a != 0 || p.anim_weight > 0.0f);
     const uint64_t stream_policy = l2_policy_evict_first();
+    // the row ids of a group, loaded a group ahead
+    auto row_id = [&](uint32_t g) -> uint32_t {
+        const uint32_t i = g * 32u + (uint32_t)lane;
+        return g < groups && i < n_vis ? p.ids_out[i] : kSentinel;
+    };
+    uint32_t next_id = row_id(wg);
     bool stage_failed = false;
     uint32_t phase = 0;   // parity of the next completion of the warp's barrier
     uint32_t d0 = 0, d2 = 0, d3 = 0, d4 = 0, d6 = 0, d7 = 0, m1 = 0, m5 = 0;
     for (uint32_t g = wg; g < groups; g += nw) {
-        const uint32_t id = stage_group<kChunks>(p.rows, p.ids_out, g * 32u, n_vis, stage0, &s_bar[warp], lane,
-                                                 stream_policy);
+        const uint32_t id = next_id;
+        next_id = row_id(g + nw);
+        stage_group<kChunks>(p.rows, id, stage0, &s_bar[warp], lane, stream_policy);
         if (!mbar_wait_bounded(&s_bar[warp], phase)) stage_failed = true;
         phase ^= 1u;
         if (id != kSentinel) {
@@ -666,16 +688,11 @@ __device__ __forceinline__ void sh_eval_tc(const float4* stage, int lane, float 
 // bytes per visible row, with the SH colour from sh_eval_tc and everything
 // else (covariance, conic, radius, centre, depth) in FP32 as for full rows.
 __global__ void __launch_bounds__(kCullThreads, 6) cull_project_half_kernel(CullParams p) {
+    pdl_wait();
     extern __shared__ float4 smem4[];
-    __shared__ __align__(8) uint64_t s_bar[kCullWarps];
     __shared__ __align__(16) __half s_y[kCullWarps][1024];
     __shared__ float s_out[kCullWarps][96];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-        mbar_init(&s_bar[warp], 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
     float4* const stage0 = smem4 + (size_t)warp * 32 * kHalfStageStride;
     const uint32_t n_vis = p.fc->visible_count;
     const uint32_t groups = (n_vis + 31) / 32;
@@ -683,14 +700,17 @@ __global__ void __launch_bounds__(kCullThreads, 6) cull_project_half_kernel(Cull
     CamRegs cam;
     load_cam(p.cam, cam);
     const uint64_t stream_policy = l2_policy_evict_first();
-    bool stage_failed = false;
-    uint32_t phase = 0;
+    // the row ids of a group, loaded a group ahead
+    auto row_id = [&](uint32_t g) -> uint32_t {
+        const uint32_t i = g * 32u + (uint32_t)lane;
+        return g < groups && i < n_vis ? p.ids_out[i] : kSentinel;
+    };
+    uint32_t next_id = row_id(wg);
     uint32_t d0 = 0, d2 = 0, d3 = 0, d4 = 0, d6 = 0, d7 = 0, m1 = 0, m5 = 0;
     for (uint32_t g = wg; g < groups; g += nw) {
-        const uint32_t id = stage_group<kHalfRowChunks, kHalfRowChunks, kHalfStageStride>(
-            p.rows, p.ids_out, g * 32u, n_vis, stage0, &s_bar[warp], lane, stream_policy);
-        if (!mbar_wait_bounded(&s_bar[warp], phase)) stage_failed = true;
-        phase ^= 1u;
+        const uint32_t id = next_id;
+        next_id = row_id(g + nw);
+        stage_half_group(p.rows, id, stage0, lane, stream_policy);
         const bool valid = id != kSentinel;
         float4* row = stage0 + lane * kHalfStageStride;
         const float4 c0 = row[0];
@@ -736,7 +756,6 @@ __global__ void __launch_bounds__(kCullThreads, 6) cull_project_half_kernel(Cull
         }
         __syncwarp();
     }
-    if (stage_failed) atomicOr(&p.fc->error_flags, kErrCullStage);
     if (p.collect_stats) {
         const uint32_t s0 = __reduce_add_sync(0xffffffffu, d0), s2 = __reduce_add_sync(0xffffffffu, d2);
         const uint32_t s3 = __reduce_add_sync(0xffffffffu, d3), s4 = __reduce_add_sync(0xffffffffu, d4);
@@ -989,7 +1008,7 @@ int launch_cull(const CullParams& p, uint32_t num_sms, cudaStream_t s) {
     uint32_t pgrid = num_sms * 6;
     if (pgrid * kCullWarps > groups_cap) pgrid = (groups_cap + kCullWarps - 1) / kCullWarps;
     if (p.half_rows) {
-        cull_project_half_kernel<<<pgrid, kCullThreads, kCullHalfSmem, s>>>(p);
+        launch_pdl(cull_project_half_kernel, dim3(pgrid), dim3(kCullThreads), kCullHalfSmem, s, p);
         return 2;
     }
     switch (deg) {

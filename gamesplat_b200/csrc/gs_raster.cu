@@ -57,6 +57,7 @@
 #include <type_traits>
 
 #include "gs_common.cuh"
+#include "gs_copy.cuh"
 #include "gs_internal.h"
 
 namespace gs {
@@ -100,15 +101,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int kLeft>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
 }
 
 __device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }

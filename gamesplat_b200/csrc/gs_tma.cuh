@@ -48,26 +48,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t phase,
     return false;
 }
 
-// 1-D bulk copy global -> shared, completion counted on `bar` (bytes and
-// addresses must be multiples of 16).
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// L2 policy for data read once per frame (the Gaussian rows): evict first,
-// so the stream does not push out the frame's intermediates that the next
-// kernels re-read (projected records, sort buffers).
-__device__ __forceinline__ uint64_t l2_policy_evict_first() {
-    uint64_t pol;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-    return pol;
-}
-
-// bulk_g2s with an L2 cache policy.
+// 1-D bulk copy global -> shared under an L2 cache policy, completion counted on
+// `bar` (bytes and addresses must be multiples of 16).
 __device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, uint32_t bytes, uint64_t* bar,
                                               uint64_t policy) {
     asm volatile(

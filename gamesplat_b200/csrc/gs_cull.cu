@@ -347,118 +347,136 @@ int launch_pack_half_rows(const float4* rows, float4* half_rows, uint32_t n, uin
     return 1;
 }
 
-// Pass 1 (visibility and compaction): each CTA takes one 2048-row tile by
-// ticket (tickets follow CTA start order, so every tile a look-back waits on
-// belongs to a CTA that is already running), loads 8 heads per thread
-// (coalesced, all in flight at once), tests visibility
-// (shaders/cull.glsl:209-220), computes the depth keys (:230-232) and places
-// the tile's visible (key, id) pairs in index order: a block scan of the
-// per-(row group, warp) counts, then one warp-level decoupled look-back per
-// tile.  The key-digit histograms of the depth sort (9-bit digits of the biased
-// key, see kDepthKeyBias) are accumulated in
-// shared memory; the top digit (sign and high exponent bits, a handful of
-// values in a scene) is aggregated per warp first, since 32 lanes adding to
-// one shared word would serialize.
-__global__ void __launch_bounds__(kCullVisThreads) cull_visible_kernel(CullParams p) {
+// Pass 1 (visibility and compaction): each CTA takes one tile of rows by ticket
+// (tickets follow CTA start order, so every tile that another waits on belongs
+// to a CTA that is already running), loads the heads (coalesced, 8 a thread in
+// flight), tests visibility (shaders/cull.glsl:209-220), computes the depth keys
+// (:230-232) and compacts the visible (key, row) pairs in index order: a warp's
+// rows follow one another, so it appends to its own run in shared memory and the
+// tile's runs meet in one scan of the warps' counts.  The tile's place in the
+// output is the sum of the counts of the tiles before it: of its own round of
+// tiles (as many as are resident at a time) the counts themselves, all loaded at
+// once by the CTA's threads, of earlier rounds the prefix that a round's last
+// tile publishes.  The key-digit histograms of the depth sort (9-bit digits of
+// the biased key, see kDepthKeyBias) are accumulated in shared memory; the top
+// digit (sign and high exponent bits, a handful of values in a scene) is
+// aggregated per warp first, since 32 lanes adding to one shared word would
+// serialize.
+//
+// The rows are cut into whole rounds of equal tiles, 8 to 20 rows a thread (tiles
+// of 2048 rows at n / 2048 CTAs left a last round half empty, and their
+// look-backs walked through hundreds of counts published at about the same
+// time).  Bound by the latency of load, count and write in turn: 3M Gaussians 36
+// -> 25 us, 6M 67 -> 49 us, where the heads and pairs take 10 and 20 at the copy rate.
+__global__ void __launch_bounds__(kCullVisThreads, kVisPerSm) cull_visible_kernel(CullParams p, int items,
+                                                                                  uint32_t round) {
     pdl_wait();
     constexpr int kWarps = kCullVisThreads / 32;
-    static_assert(kCullVisItems * kWarps == 64, "the count scan gives each lane two (row group, warp) counts");
     __shared__ uint32_t s_hist[4][kDepthRadix];
-    __shared__ uint32_t s_cnt[kCullVisItems * kWarps];   // (row group, warp) order = index order
-    __shared__ uint32_t s_tile, s_excl;
+    __shared__ uint32_t s_key[kWarps][kVisItemsMax * 32];
+    __shared__ uint16_t s_row[kWarps][kVisItemsMax * 32];   // row in the warp's range
+    __shared__ uint32_t s_cnt[kWarps], s_sum[kWarps];
+    __shared__ uint32_t s_tile;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     for (int i = t; i < 4 * kDepthRadix; i += kCullVisThreads) (&s_hist[0][0])[i] = 0u;
     if (t == 0) s_tile = atomicAdd(&p.fc->cull_ticket, 1u);
     __syncthreads();
     const uint32_t tile = s_tile;
-    const uint32_t num_tiles = (p.n + kCullVisTile - 1) / kCullVisTile;
+    const uint32_t tile_rows = (uint32_t)(items * kCullVisThreads);
+    const uint32_t num_tiles = (p.n + tile_rows - 1) / tile_rows;
     if (tile >= num_tiles) return;   // uniform over the CTA
-    const uint32_t base = tile * kCullVisTile;
+    const uint32_t base = tile * tile_rows + (uint32_t)(warp * items * 32);
     const float* V = p.cam.view;
     const float P0 = p.cam.proj[0], P5 = p.cam.proj[5], ortho = p.cam.orthographic;
-    float4 c0[kCullVisItems];
+    uint32_t cnt = 0;
+    for (int k0 = 0; k0 < items; k0 += 8) {
+        float4 c0[8];
 #pragma unroll
-    for (int k = 0; k < kCullVisItems; ++k) {
-        const uint32_t g = base + k * kCullVisThreads + t;
-        c0[k] = g < p.n ? __ldg(p.heads + g) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    uint32_t mask[kCullVisItems], key[kCullVisItems];
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t g = base + (uint32_t)((k0 + k) * 32 + lane);
+            c0[k] = k0 + k < items && g < p.n ? __ldg(p.heads + g) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
 #pragma unroll
-    for (int k = 0; k < kCullVisItems; ++k) {
-        const uint32_t g = base + k * kCullVisThreads + t;
-        // p_view = view * vec4(position, 1.0)
-        const float vx = add(add(add(mul(V[0], c0[k].x), mul(V[4], c0[k].y)), mul(V[8], c0[k].z)), V[12]);
-        const float vy = add(add(add(mul(V[1], c0[k].x), mul(V[5], c0[k].y)), mul(V[9], c0[k].z)), V[13]);
-        const float vz = add(add(add(mul(V[2], c0[k].x), mul(V[6], c0[k].y)), mul(V[10], c0[k].z)), V[14]);
-        bool visible = g < p.n && (vz <= -0.2f);
-        if (visible) {
-            float inv_z = dv(-1.0f, vz);
-            float ndc_x = add(mul(mul(mul(P0, vx), inv_z), sub(1.0f, ortho)), mul(mul(P0, vx), ortho));
-            float ndc_y = add(mul(mul(mul(P5, vy), inv_z), sub(1.0f, ortho)), mul(mul(P5, vy), ortho));
-            visible = fabsf(ndc_x) <= 1.3f && fabsf(ndc_y) <= 1.3f;
-        }
-        key[k] = 0xFFFFFFFFu - __float_as_uint(g_max(-vz, 0.0f));
-        mask[k] = __ballot_sync(0xffffffffu, visible);
-        if (lane == 0) s_cnt[k * kWarps + warp] = (uint32_t)__popc(mask[k]);
-        if (!visible && g < p.n && p.write_invisible) {   // shaders/cull.glsl:222-228
-            float4* dst = p.projected + (size_t)g * 4;
-            dst[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-            dst[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-            dst[2] = make_float4(1.f, 0.f, 1.f, 1.f);
-            dst[3] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    }
-    __syncthreads();
-    if (warp == 0) {
-        // exclusive scan of the 64 counts in index order, two per lane
-        const uint32_t a = s_cnt[2 * lane], b = s_cnt[2 * lane + 1];
-        uint32_t incl = a + b;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        s_cnt[2 * lane] = incl - a - b;
-        s_cnt[2 * lane + 1] = incl - b;
-        if (lane == 0)
-            st_relaxed64(p.status + tile, status_word(p.epoch, tile == 0 ? kFlagInc : kFlagAgg, total));
-        uint32_t excl = 0;
-        if (tile > 0) {
-            bool to = false;
-            excl = lookback_warp(p.status, tile, p.epoch, &to);
-            if (lane == 0) {
-                if (to) atomicOr(&p.fc->error_flags, kErrCullLookback);
-                st_relaxed64(p.status + tile, status_word(p.epoch, kFlagInc, excl + total));
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t r = (uint32_t)((k0 + k) * 32 + lane), g = base + r;
+            const bool row = k0 + k < items && g < p.n;
+            // p_view = view * vec4(position, 1.0)
+            const float vx = add(add(add(mul(V[0], c0[k].x), mul(V[4], c0[k].y)), mul(V[8], c0[k].z)), V[12]);
+            const float vy = add(add(add(mul(V[1], c0[k].x), mul(V[5], c0[k].y)), mul(V[9], c0[k].z)), V[13]);
+            const float vz = add(add(add(mul(V[2], c0[k].x), mul(V[6], c0[k].y)), mul(V[10], c0[k].z)), V[14]);
+            bool visible = row && (vz <= -0.2f);
+            if (visible) {
+                float inv_z = dv(-1.0f, vz);
+                float ndc_x = add(mul(mul(mul(P0, vx), inv_z), sub(1.0f, ortho)), mul(mul(P0, vx), ortho));
+                float ndc_y = add(mul(mul(mul(P5, vy), inv_z), sub(1.0f, ortho)), mul(mul(P5, vy), ortho));
+                visible = fabsf(ndc_x) <= 1.3f && fabsf(ndc_y) <= 1.3f;
             }
-        }
-        if (lane == 0) {
-            s_excl = excl;
-            if (tile == num_tiles - 1) p.fc->visible_count = excl + total;
+            const uint32_t mask = __ballot_sync(0xffffffffu, visible);
+            const uint32_t kk = 0xFFFFFFFFu - __float_as_uint(g_max(-vz, 0.0f));
+            if (visible) {
+                const uint32_t o = cnt + (uint32_t)__popc(mask & lt);
+                s_key[warp][o] = kk;
+                s_row[warp][o] = (uint16_t)r;
+                const uint32_t b = kk + kDepthKeyBias;
+                atomicAdd(&s_hist[0][b & 511u], 1u);
+                atomicAdd(&s_hist[1][(b >> 9) & 511u], 1u);
+                atomicAdd(&s_hist[2][(b >> 18) & 511u], 1u);
+            } else if (row && p.write_invisible) {   // shaders/cull.glsl:222-228
+                float4* dst = p.projected + (size_t)g * 4;
+                dst[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+                dst[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                dst[2] = make_float4(1.f, 0.f, 1.f, 1.f);
+                dst[3] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            cnt += (uint32_t)__popc(mask);
+            // invisible lanes match among themselves (512 is no digit) and add nothing
+            const uint32_t d3 = visible ? (kk + kDepthKeyBias) >> 27 : 512u;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d3);
+            if (visible && lane == __ffs(peers) - 1) atomicAdd(&s_hist[3][d3], (uint32_t)__popc(peers));
         }
     }
+    if (lane == 0) s_cnt[warp] = cnt;
     __syncthreads();
-    const uint32_t excl = s_excl;
+    uint32_t before = 0, total = 0;   // the tile's pairs before the warp's, and all
 #pragma unroll
-    for (int k = 0; k < kCullVisItems; ++k) {
-        const bool v = (mask[k] >> lane) & 1u;
-        const uint32_t kk = key[k];
-        if (v) {
-            const uint32_t o = excl + s_cnt[k * kWarps + warp] + (uint32_t)__popc(mask[k] & lt);
-            p.keys_out[o] = kk;
-            p.ids_out[o] = base + k * kCullVisThreads + t;
-            const uint32_t b = kk + kDepthKeyBias;
-            atomicAdd(&s_hist[0][b & 511u], 1u);
-            atomicAdd(&s_hist[1][(b >> 9) & 511u], 1u);
-            atomicAdd(&s_hist[2][(b >> 18) & 511u], 1u);
-        }
-        // invisible lanes match among themselves (256 is no digit) and add nothing
-        const uint32_t d3 = v ? (kk + kDepthKeyBias) >> 27 : 256u;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d3);
-        if (v && lane == __ffs(peers) - 1) atomicAdd(&s_hist[3][d3], (uint32_t)__popc(peers));
+    for (int w = 0; w < kWarps; ++w) {
+        const uint32_t c = s_cnt[w];
+        if (w < warp) before += c;
+        total += c;
     }
+    const uint32_t first = tile / round * round;        // the round's first tile
+    const bool closes = tile == first + round - 1u;     // its last one publishes the prefix alone
+    if (t == 0 && !closes) st_relaxed64(p.status + tile, status_word(p.epoch, kFlagAgg, total));
+    uint32_t sum = 0;
+    bool timed_out = false;
+    for (uint32_t j = (first ? first - 1u : 0u) + (uint32_t)t; j < tile; j += kCullVisThreads) {
+        uint32_t spins = 0;
+        for (;;) {
+            const unsigned long long w = ld_relaxed64(p.status + j);
+            if ((uint32_t)(w >> 32) == p.epoch && ((uint32_t)w & ~kValMask) != 0u) {
+                sum += (uint32_t)w & kValMask;
+                break;
+            }
+            if (++spins > kSpinLimit) { timed_out = true; break; }
+            if (spins > 64) __nanosleep(32);
+        }
+    }
+    if (timed_out) atomicOr(&p.fc->error_flags, kErrCullLookback);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) s_sum[warp] = sum;
     __syncthreads();
+    uint32_t excl = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) excl += s_sum[w];
+    if (t == 0) {
+        if (closes) st_relaxed64(p.status + tile, status_word(p.epoch, kFlagInc, excl + total));
+        if (tile == num_tiles - 1) p.fc->visible_count = excl + total;
+    }
+    for (uint32_t i = (uint32_t)lane; i < cnt; i += 32) {
+        p.keys_out[excl + before + i] = s_key[warp][i];
+        p.ids_out[excl + before + i] = base + s_row[warp][i];
+    }
     for (int i = t; i < 4 * kDepthRadix; i += kCullVisThreads) {
         const uint32_t c = (&s_hist[0][0])[i];
         if (c) atomicAdd(p.key_hist + i, c);
@@ -1000,9 +1018,14 @@ int launch_cull(const CullParams& p, uint32_t num_sms, cudaStream_t s) {
     }
     int deg = pp.sh_degree < 0 ? 0 : (pp.sh_degree > 3 ? 3 : pp.sh_degree);
     if (pp.anim_deltas) deg = 3;   // the delta pass touches every SH slot of the staged row
-    const uint32_t tiles = (p.n + kCullVisTile - 1) / kCullVisTile;
-    if (tiles == 0) return 0;
-    launch_pdl(cull_visible_kernel, dim3(tiles), dim3(kCullVisThreads), 0, s, p);
+    if (p.n == 0) return 0;
+    // tiles: whole rounds of the CTAs resident at a time, equal rows in each
+    const uint32_t round = num_sms * kVisPerSm;
+    const uint64_t most = (uint64_t)round * kVisItemsMax * kCullVisThreads;
+    const uint64_t rounds = (p.n + most - 1) / most, cells = rounds * round * kCullVisThreads;
+    const int items = std::max((int)((p.n + cells - 1) / cells), kCullVisItems);
+    const uint32_t tile_rows = (uint32_t)items * kCullVisThreads;
+    launch_pdl(cull_visible_kernel, dim3((p.n + tile_rows - 1) / tile_rows), dim3(kCullVisThreads), 0, s, p, items, round);
     // projection: persistent, as many CTAs as fit (6 per SM) for the largest possible visible count
     const uint32_t groups_cap = (p.n + 31) / 32;
     uint32_t pgrid = num_sms * 6;

@@ -63,7 +63,9 @@ constexpr uint32_t kDepthKeyBias = 0x3E4CCCCDu;   // bits of 0.2f
 // its 2048-row CTA tiles are the units of the look-back.  Projection pass:
 // 128-thread CTAs, each warp stages and projects 32 visible rows at a time.
 constexpr int kCullVisThreads = 256;
-constexpr int kCullVisItems = 8;
+constexpr int kCullVisItems = 8;     // rows a thread: the fewest of a tile, and the most
+constexpr int kVisItemsMax = 20;
+constexpr int kVisPerSm = 4;         // resident CTAs
 constexpr int kCullVisTile = kCullVisThreads * kCullVisItems;
 constexpr int kCullThreads = 128;
 constexpr int kHalfRowChunks = 9;   // 144-byte FP16-SH row: position/opacity, scale, rotation, 48 half SH

@@ -6,8 +6,8 @@
 // geometry and fill rule as the CPU oracle (gs::quad_rect), (b) writes a
 // 64-byte RasterRecord at position s, and (c) emits one (tile, s) entry per
 // 16x16 tile that can receive a non-discarded fragment.  Entries are written
-// in descending s order (nearest splat first) at offsets found by a
-// decoupled look-back over CTA tiles, so a stable sort on the tile id alone
+// in descending s order (nearest splat first) at offsets found by summing
+// the counts of the earlier CTA tiles, so a stable sort on the tile id alone
 // leaves each tile's list in front-to-back order, the order the rasterizer
 // walks.
 //
@@ -132,7 +132,7 @@ __device__ __forceinline__ BinItem bin_one(const BinParams& p, uint32_t s, uint3
 __global__ void __launch_bounds__(kBinThreads) bin_kernel(BinParams p) {
     pdl_wait();
     __shared__ uint32_t scan_tmp[33];
-    __shared__ uint32_t s_tile, s_excl, s_total;
+    __shared__ uint32_t s_tile, s_part[kBinThreads / 32];
     __shared__ uint32_t s_off[kBinTile];    // exclusive entry offset of each splat in the CTA tile
     __shared__ uint32_t s_org[kBinTile];    // tx0 | ty0 << 16 of its tile rectangle
     __shared__ uint16_t s_w[kBinTile];      // its width in tiles (0: no entries)
@@ -183,35 +183,29 @@ __global__ void __launch_bounds__(kBinThreads) bin_kernel(BinParams p) {
             s_off[t * kBinItems + k] = run;
             run += c[k];
         }
-        if (t < 32) {
-            // warp 0: publish the tile count, resolve the prefix by a
-            // warp-cooperative look-back, publish the inclusive prefix
-            u64* st = p.status + tile;
-            uint32_t excl = 0;
-            if (tile == 0) {
-                if (t == 0) st_relaxed64(st, status_word(p.epoch, kFlagInc, total));
-            } else {
-                if (t == 0) st_relaxed64(st, status_word(p.epoch, kFlagAgg, total));
-                bool to = false;
-                excl = lookback_warp(p.status, tile, p.epoch, &to);
-                if (t == 0) {
-                    if (to) atomicOr(&p.fc->error_flags, kErrBinLookback);
-                    st_relaxed64(st, status_word(p.epoch, kFlagInc, excl + total));
-                }
-            }
-            if (t == 0) {
-                s_excl = excl;
-                s_total = total;
-                if (tile == num_tiles - 1) {
-                    const uint32_t e = excl + total;
-                    p.fc->tile_entries = e < p.entry_cap ? e : p.entry_cap;
-                    p.fc->tile_overflow = e > p.entry_cap ? e - p.entry_cap : 0u;
-                    if (e > p.entry_cap) atomicOr(&p.fc->error_flags, kErrTileOverflow);
-                }
+        // The tile's first entry (a look-back by one warp, 32 tiles at a time, took
+        // the binning stage 3.6 us more at 3M Gaussians and 10 us at 6M).
+        const bool closes = closes_round(tile, gridDim.x);
+        if (t == 0 && !closes) st_relaxed64(p.status + tile, status_word(p.epoch, kFlagAgg, total));
+        bool to = false;
+        uint32_t excl = sum_earlier(p.status, tile, gridDim.x, p.epoch, (uint32_t)t, kBinThreads, &to);
+        if (to) atomicOr(&p.fc->error_flags, kErrBinLookback);
+        excl = __reduce_add_sync(0xffffffffu, excl);
+        if ((t & 31) == 0) s_part[t >> 5] = excl;
+        __syncthreads();
+        excl = 0;
+#pragma unroll
+        for (int w = 0; w < kBinThreads / 32; ++w) excl += s_part[w];
+        if (t == 0) {
+            if (closes) st_relaxed64(p.status + tile, status_word(p.epoch, kFlagInc, excl + total));
+            if (tile == num_tiles - 1) {
+                const uint32_t e = excl + total;
+                p.fc->tile_entries = e < p.entry_cap ? e : p.entry_cap;
+                p.fc->tile_overflow = e > p.entry_cap ? e - p.entry_cap : 0u;
+                if (e > p.entry_cap) atomicOr(&p.fc->error_flags, kErrTileOverflow);
             }
         }
-        __syncthreads();
-        const uint32_t excl = s_excl, cta_total = s_total;
+        const uint32_t cta_total = total;
         // Per-item information for the expansion kernel (coalesced).
         for (int j = t; j < (int)cnt; j += kBinThreads)
             p.item_info[(size_t)tile * kBinTile + j] = make_uint4(excl + s_off[j], s_org[j], s_w[j], 0u);

@@ -292,43 +292,31 @@ __device__ __forceinline__ uint32_t lookback_vec(const u64* status, size_t strid
     return excl;
 }
 
-// Warp-cooperative look-back: all 32 lanes read a window of 32 predecessors
-// at once, the nearest inclusive word is found by ballot and the aggregates
-// after it are summed with a warp reduction.  Every lane returns the same
-// exclusive prefix, and every lane sees *timed_out if any lane's wait ran
-// out.  Bounded like lookback_vec().
-__device__ __forceinline__ uint32_t lookback_warp(const u64* status, uint32_t tile, uint32_t epoch,
-                                                  bool* timed_out, uint32_t spin_limit = kSpinLimit) {
-    const int lane = threadIdx.x & 31;
-    uint32_t excl = 0;
-    long long end = (long long)tile;  // window = [end - 32, end)
-    uint32_t spins = 0;
-    bool ran_out = false;   // this lane's wait gave up (made warp-uniform at the end)
-    while (end > 0) {
-        const long long j = end - 32 + lane;
-        uint32_t flag = kFlagInc, val = 0;   // before tile 0: an inclusive zero
-        if (j >= 0) {
-            for (;;) {
-                const u64 w = ld_relaxed64(status + j);
-                flag = (uint32_t)w & ~kValMask;
-                val = (uint32_t)w & kValMask;
-                if ((uint32_t)(w >> 32) == epoch && flag != 0u) break;
-                if (++spins > spin_limit) { ran_out = true; flag = kFlagInc; val = 0; break; }
-                if (spins > 64) __nanosleep(32);
+// The place of a tile in a scan over tiles that are taken by ticket, in rounds
+// of `round`: one thread's share of the sum over the earlier tiles of its round,
+// whose words hold their counts, and the round before, whose last word holds the
+// prefix through it (a round's last tile publishes nothing else).  Every word is
+// one load of one thread, all in flight at once.  Waits are bounded: *timed_out.
+__device__ __forceinline__ uint32_t sum_earlier(const u64* status, uint32_t tile, uint32_t round, uint32_t epoch,
+                                                uint32_t thread, uint32_t threads, bool* timed_out,
+                                                uint32_t spin_limit = kSpinLimit) {
+    const uint32_t first = tile / round * round;
+    uint32_t sum = 0;
+    for (uint32_t j = (first ? first - 1u : 0u) + thread; j < tile; j += threads) {
+        uint32_t spins = 0;
+        for (;;) {
+            const u64 w = ld_relaxed64(status + j);
+            if ((uint32_t)(w >> 32) == epoch && ((uint32_t)w & ~kValMask) != 0u) {
+                sum += (uint32_t)w & kValMask;
+                break;
             }
+            if (++spins > spin_limit) { *timed_out = true; return sum; }
+            if (spins > 64) __nanosleep(32);
         }
-        const uint32_t inc = __ballot_sync(0xffffffffu, flag == kFlagInc);
-        if (inc) {
-            const int h = 31 - __clz(inc);   // nearest inclusive in the window
-            excl += __reduce_add_sync(0xffffffffu, lane >= h ? val : 0u);
-            break;
-        }
-        excl += __reduce_add_sync(0xffffffffu, val);
-        end -= 32;
     }
-    if (__any_sync(0xffffffffu, ran_out)) *timed_out = true;
-    return excl;
+    return sum;
 }
+__device__ __forceinline__ bool closes_round(uint32_t tile, uint32_t round) { return tile % round == round - 1u; }
 
 // Block-wide exclusive scan of one uint32 per thread (blockDim.x <= 1024,
 // multiple of 32).  `warp_tmp` holds >= 33 words of shared memory.

@@ -7,8 +7,8 @@
 //     per upload by gather_heads_kernel: reading them out of the rows would
 //     fetch at least one 32-byte sector, in practice 128 bytes, per 16 bytes
 //     used), runs the near/frustum test, computes the depth keys and
-//     compacts the visible (key, id) pairs in index order with a decoupled
-//     look-back over 2048-row CTA tiles, so the depth sort runs on N_vis
+//     compacts the visible (key, id) pairs in index order, each CTA tile's
+//     place the sum of the counts of the tiles before it, so the depth sort runs on N_vis
 //     pairs instead of N (the culled tail of the reference's all-N sort is
 //     all-equal (0xFFFFFFFF, 0xFFFFFFFF) pairs, so the result is identical);
 //   * cull_project_kernel walks the compacted ids in groups of 32 and stages
@@ -445,23 +445,10 @@ __global__ void __launch_bounds__(kCullVisThreads, kVisPerSm) cull_visible_kerne
         if (w < warp) before += c;
         total += c;
     }
-    const uint32_t first = tile / round * round;        // the round's first tile
-    const bool closes = tile == first + round - 1u;     // its last one publishes the prefix alone
+    const bool closes = closes_round(tile, round);
     if (t == 0 && !closes) st_relaxed64(p.status + tile, status_word(p.epoch, kFlagAgg, total));
-    uint32_t sum = 0;
     bool timed_out = false;
-    for (uint32_t j = (first ? first - 1u : 0u) + (uint32_t)t; j < tile; j += kCullVisThreads) {
-        uint32_t spins = 0;
-        for (;;) {
-            const unsigned long long w = ld_relaxed64(p.status + j);
-            if ((uint32_t)(w >> 32) == p.epoch && ((uint32_t)w & ~kValMask) != 0u) {
-                sum += (uint32_t)w & kValMask;
-                break;
-            }
-            if (++spins > kSpinLimit) { timed_out = true; break; }
-            if (spins > 64) __nanosleep(32);
-        }
-    }
+    uint32_t sum = sum_earlier(p.status, tile, round, p.epoch, (uint32_t)t, kCullVisThreads, &timed_out);
     if (timed_out) atomicOr(&p.fc->error_flags, kErrCullLookback);
     sum = __reduce_add_sync(0xffffffffu, sum);
     if (lane == 0) s_sum[warp] = sum;

@@ -18,7 +18,7 @@ __global__ void wait_probe_kernel(const unsigned long long* status, FrameCounter
         // reads as "not published yet" on every poll
         if (threadIdx.x < 32) {
             bool to = false;
-            lookback_warp(status, 1, epoch, &to, limit);
+            sum_earlier(status, 1, 2, epoch, threadIdx.x, blockDim.x, &to, limit);
             if (threadIdx.x == 0 && to) atomicOr(&fc->error_flags, kErrCullLookback);
         }
     } else {

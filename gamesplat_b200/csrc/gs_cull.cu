@@ -788,8 +788,10 @@ __global__ void __launch_bounds__(kCullThreads, 6) cull_project_half_kernel(Cull
 // read and evaluated once, and a frame costs its 48 (blended: 96) delta bytes,
 // read as 16-byte loads (a delta row is 48 bytes).  Colours leave through
 // shared memory so that a group's rows are written whole.  Issue-bound: ~13
-// operations a coefficient of a blended frame.  1M rows, 16 blended frames:
-// 16 launches of 182 us (byte loads, row and basis per frame) before.
+// operations a coefficient of a blended frame, and by the latency of the delta
+// loads: 4 CTAs an SM (126 registers) against 3 (165) take the call of 1M rows and
+// 16 blended frames from 1446 to 1367 us (5 spill: 1453); 16 launches of 182 us
+// (byte loads, row and basis per frame) before.
 constexpr int kRecolourThreads = 128;
 
 // int8 k of a word (already xor 0x80808080) as float: 2^23 + 128 + q has q's bits, biased, in its low mantissa byte
@@ -798,7 +800,7 @@ __device__ __forceinline__ float int8_of(uint32_t biased, int k) {
 }
 
 template <int kGroup>
-__global__ void __launch_bounds__(kRecolourThreads) recolour_states_kernel(CullParams p,
+__global__ void __launch_bounds__(kRecolourThreads, 4) recolour_states_kernel(CullParams p,
                                                                            const RasterRecord* __restrict__ records,
                                                                            StateBatch st, int first, int frames,
                                                                            float* __restrict__ colours) {

@@ -652,10 +652,11 @@ __global__ void __launch_bounds__(kRasterThreads) raster_batch_kernel(const Rast
 // staged colours, 48 accumulators) against one frame a tile in the batch
 // kernel.  1M Gaussians, 1920x1080, 16 blended frames: the call 6620 us when
 // every frame rasterized alone (3534 us of it) and was recoloured alone, 1633 us
-// in groups.
+// in groups, 1446 us with the rasterizer's lists and cp.async; 4 CTAs an SM (128
+// registers, 56 bytes spilled) against 3 (142) then 1367 -> 1306 us, 5 (96): 1452.
 template <int kStates, int kTw, int kTh>
-__global__ void __launch_bounds__(kRasterThreads) raster_states_kernel(RasterParams p, StateOuts outs, int first,
-                                                                       uint32_t groups) {
+__global__ void __launch_bounds__(kRasterThreads, kStates == 8 ? 4 : 6)
+    raster_states_kernel(RasterParams p, StateOuts outs, int first, uint32_t groups) {
     pdl_wait();
     __shared__ RasterShared<0, kTw, kTh, kStates> sh;
     __shared__ uint16_t* s_out[kStates];

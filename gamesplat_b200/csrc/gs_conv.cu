@@ -109,20 +109,6 @@ __device__ __forceinline__ uint4 bf16x8_add(uint4 a, uint4 b) {
     return r;
 }
 
-// 8 channels (16 bytes) of input pixel (n, y, x), zero outside the image.
-// kLoad 1: the decoder input, nearest 2x upsampling of `xh` (half
-// resolution) plus `x` at full resolution.
-template <int kCin, int kLoad>
-__device__ __forceinline__ uint4 load_granule(const ConvArgs& a, int n, int y, int x, int g) {
-    if (y < 0 || y >= a.h || x < 0 || x >= a.w) return make_uint4(0u, 0u, 0u, 0u);
-    const size_t pix = ((size_t)n * a.h + y) * a.w + x;
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.x + pix * kCin) + g);
-    if (kLoad == 0) return v;
-    const int hh = a.h >> 1, hw = a.w >> 1;
-    const size_t hp = ((size_t)n * hh + min(y >> 1, hh - 1)) * hw + min(x >> 1, hw - 1);
-    return bf16x8_add(v, __ldg(reinterpret_cast<const uint4*>(a.xh + hp * kCin) + g));
-}
-
 // A run of rows [y0, y1) of one strip; a CTA's share of the units is a sequence of them.
 struct ConvRun {
     int n, x0, y0, y1;
@@ -170,7 +156,10 @@ struct Roles {
 // end of a run), every output written once in 32-byte sectors.  An M = 128, K =
 // 16 MMA with both operands in shared memory takes ~50 cycles for N up to 64
 // and 59 for N = 96 (its A operand is what it reads), so one MMA for three
-// output rows takes a row 7 instead of 18 of them.  Times at launch_fwd.
+// output rows takes a row 7 instead of 18 of them.  1920 x 1080, the layers of the
+// denoised frame: 16 -> 32 pooled 61 us, 32 -> 32 at half size 25, 32 -> 32 from two
+// inputs 86, 32 -> 16 with the head 80 (99, 46, 164, 94 at one MMA a tap and no
+// roles); read and written bytes pass at ~4 TB/s.
 template <int kCin, int kCout, int kLoad, bool kPool>
 __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
     static_assert(kCin % 16 == 0 && (kCout == 16 || kCout == 32), "channel counts");
@@ -509,12 +498,16 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
 // kx pixels further.  Per output row: 3 taps x 8 K-steps MMAs into 3
 // accumulators.  Two stages: the strip after the next is copied (cp.async)
 // while one is multiplied, and MMAs of consecutive strips queue without a
-// wait between them.  The bias gradient is summed from the staged dY by the
-// threads while the MMAs run.  Bound by the shared-memory reads of the MMAs
-// and the L2 reads of the strips (1.5 reads of X for 4 rows); 8 x 256 x 256
-// pixels, 32 -> 32 channels: 262 us (load mode 1) when every tap was gathered
-// from global memory and nothing overlapped; figures now at launch_wgrad.
-constexpr int kWgThreads = 256;
+// wait between them.  Eight warps copy and sum the bias gradient from the staged
+// dY; a ninth issues the MMAs, which a copying warp did before, holding up its
+// own copies.  The strips pass at ~115 cycles an MMA, more loading warps or
+// less issue work change nothing, and an aligned operand takes ~50: presumably the
+// reads of tap kx, whose operand starts kx x 16 bytes off a 128-byte line.  8 x 256 x 256
+// pixels, 32 -> 16, 32 -> 32 (load mode 1) and 16 -> 32 channels: 41 / 59 / 41 us;
+// 52 / 106 / 53 with the MMAs on a copying warp and one granule of mode 1 loaded at
+// a time, 262 (mode 1) when every tap was gathered from global memory and
+// nothing overlapped.  16 copying warps: 44 / 56 / 46.
+constexpr int kWgThreads = 256;   // that copy and sum; one more warp multiplies
 constexpr int kWgPx = 128;    // pixels of a strip
 constexpr int kWgRows = 4;    // output rows of a strip, at most
 // A channel group of a dY row: 2 or 4 of them are copied by a quarter warp (as col_bytes)
@@ -527,7 +520,7 @@ __host__ __device__ constexpr int wg_stage_bytes(int cin, int cout) {
 }
 
 template <int kCin, int kCout, int kLoad>
-__global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(WgradArgs a, int rows) {
+__global__ void __launch_bounds__(kWgThreads + 32) conv_wgrad_kernel(WgradArgs a, int rows) {
     constexpr int kG = kCin / 8, kGo = kCout / 8;
     constexpr int kCol = col_bytes(kCin), kSlot = kG * kCol, kDcol = wg_dcol(kCout), kDrow = kGo * kDcol;
     constexpr int kStage = wg_stage_bytes(kCin, kCout), kX = wg_x_bytes(kCin);
@@ -546,14 +539,13 @@ __global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(WgradArgs a, int
     }
     if (warp == 0) umma::tmem_alloc(&s_taddr, kCols);
     // the slots no strip fills are operands too (their products are never read)
-    for (int i = tid; i < 2 * kStage / 16; i += kWgThreads) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = tid; i < 2 * kStage / 16; i += kWgThreads + 32) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t taddr = s_taddr, base = smem_u32(smem);
     const int strips_x = (a.w + kWgPx - 1) / kWgPx, bands = (a.h + rows - 1) / rows;
     const int total = a.n * bands * strips_x;
-    const ConvArgs ca{a.x, a.xh, a.n, a.h, a.w};
 
     struct Strip {
         int n, y0, x0, rows, px;   // px: pixels in whole K-steps
@@ -574,9 +566,9 @@ __global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(WgradArgs a, int
         uint8_t* xs = smem + stage * kStage;
         uint8_t* ds = xs + kX;
         const int row_q = (s.px + 2) * kG;
-        for (int r = 0; r < s.rows + 2; ++r) {
+        for (int r = 0; kLoad == 0 && r < s.rows + 2; ++r) {
             const int y = s.y0 - 1 + r;
-            if (kLoad == 0) {
+            {
                 const bool row_in = y >= 0 && y < a.h;
                 const __nv_bfloat16* rowp = a.x + ((size_t)s.n * a.h + (row_in ? y : 0)) * a.w * kCin;
                 for (int q = tid; q < row_q; q += kWgThreads) {
@@ -585,12 +577,39 @@ __global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(WgradArgs a, int
                     cp_async16(xs + r * kSlot + g * kCol + hp * 16, in ? rowp + (size_t)x * kCin + g * 8 : a.x,
                                in ? 16u : 0u);
                 }
-            } else {
-                for (int q = tid; q < row_q; q += kWgThreads) {
-                    const int hp = q / kG, g = q % kG;
-                    *reinterpret_cast<uint4*>(xs + r * kSlot + g * kCol + hp * 16) =
-                        load_granule<kCin, kLoad>(ca, s.n, y, s.x0 - 1 + hp, g);
+            }
+        }
+        if (kLoad == 1) {
+            // two rows at a time, all of a thread's granules loaded before the first is stored
+            constexpr int kPer = ((kWgPx + 2) * kG + kWgThreads - 1) / kWgThreads;
+            const int hh = a.h >> 1, hw = a.w >> 1;
+            for (int r0 = 0; r0 < s.rows + 2; r0 += 2) {
+                uint4 v[2][kPer], u[2][kPer];
+#pragma unroll
+                for (int d = 0; d < 2; ++d) {
+                    const int y = s.y0 - 1 + r0 + d;
+                    const bool row_in = r0 + d < s.rows + 2 && y >= 0 && y < a.h;
+                    const size_t row = ((size_t)s.n * a.h + (row_in ? y : 0)) * a.w;
+                    const size_t hrow = ((size_t)s.n * hh + (row_in ? min(y >> 1, hh - 1) : 0)) * hw;
+#pragma unroll
+                    for (int k = 0; k < kPer; ++k) {
+                        const int q = tid + k * kWgThreads, hp = q / kG, g = q % kG, x = s.x0 - 1 + hp;
+                        v[d][k] = u[d][k] = make_uint4(0u, 0u, 0u, 0u);
+                        if (row_in && q < row_q && x >= 0 && x < a.w) {
+                            v[d][k] = __ldg(reinterpret_cast<const uint4*>(a.x + (row + x) * kCin) + g);
+                            u[d][k] = __ldg(reinterpret_cast<const uint4*>(a.xh + (hrow + min(x >> 1, hw - 1)) * kCin) + g);
+                        }
+                    }
                 }
+#pragma unroll
+                for (int d = 0; d < 2; ++d)
+#pragma unroll
+                    for (int k = 0; k < kPer; ++k) {
+                        const int q = tid + k * kWgThreads, hp = q / kG, g = q % kG;
+                        if (r0 + d < s.rows + 2 && q < row_q)
+                            *reinterpret_cast<uint4*>(xs + (r0 + d) * kSlot + g * kCol + hp * 16) =
+                                bf16x8_add(v[d][k], u[d][k]);
+                    }
             }
         }
         for (int r = 0; r < s.rows; ++r) {
@@ -608,7 +627,9 @@ __global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(WgradArgs a, int
     bool failed = false, any = false;
     float db[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // of channel group tid % kGo
     int stage = 0;
-    if ((int)blockIdx.x < total) load(0, blockIdx.x);
+    const bool multiplies = warp == kWgThreads / 32;   // the last warp; the others load and sum
+    const uint32_t elected = lane == 0 ? 1u : 0u;
+    if (!multiplies && (int)blockIdx.x < total) load(0, blockIdx.x);
     for (int item = blockIdx.x; item < total; item += gridDim.x, stage ^= 1) {
         asm volatile("cp.async.wait_all;" ::: "memory");   // this strip, copied while the last one was multiplied
         umma::fence_smem_to_async();
@@ -617,22 +638,22 @@ __global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(WgradArgs a, int
             break;
         }
         const Strip s = strip_at(item);
-        if (tid == 0) {
+        if (multiplies) {
             umma::fence_after_sync();
             const uint32_t xa = base + (uint32_t)(stage * kStage), da = xa + (uint32_t)kX;
-            for (int r = 0; r < s.rows; ++r)
-                for (int kk = 0; kk < s.px / 16; ++kk) {
-                    const uint64_t bd = umma::smem_desc(da + (uint32_t)(r * kDrow + kk * 256), 128u, (uint32_t)kDcol);
+            const uint64_t ad0 = umma::smem_desc(xa, 128u, (uint32_t)kCol), bd0 = umma::smem_desc(da, 128u, (uint32_t)kDcol);
+            const int steps = s.px / 16;
+            for (int r = 0; r < s.rows; ++r) {
+                uint64_t ad = ad0 + (uint64_t)((r * kSlot) >> 4), bd = bd0 + (uint64_t)((r * kDrow) >> 4);
+                for (int kk = 0; kk < steps; ++kk, ad += 16, bd += 16)
 #pragma unroll
-                    for (int kx = 0; kx < 3; ++kx) {
-                        const uint64_t ad =
-                            umma::smem_desc(xa + (uint32_t)(r * kSlot + kx * 16 + kk * 256), 128u, (uint32_t)kCol);
-                        umma::mma_bf16(taddr + (uint32_t)(kx * kCout), ad, bd, kIdesc, (any || r + kk > 0) ? 1u : 0u);
-                    }
-                }
-            umma::commit(&s_bar[stage]);
+                    for (int kx = 0; kx < 3; ++kx)
+                        umma::mma_bf16_elect(taddr + (uint32_t)(kx * kCout), ad + (uint64_t)kx, bd, kIdesc,
+                                             (any || r + kk > 0) ? 1u : 0u, elected);
+            }
+            umma::commit_elect(&s_bar[stage], elected);
         }
-        if (a.db) {   // pixels past the row are zero
+        if (a.db && !multiplies) {   // pixels past the row are zero
             const uint8_t* ds = smem + stage * kStage + kX + (tid % kGo) * kDcol;
             for (int r = 0; r < s.rows; ++r)
                 for (int k = tid / kGo; k < s.px; k += kWgThreads / kGo) {
@@ -647,7 +668,7 @@ __global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(WgradArgs a, int
                 }
         }
         const int next = item + (int)gridDim.x;
-        if (next < total) {
+        if (next < total && !multiplies) {
             // the other stage: its MMAs (the previous strip's) read it to the end, and every
             // thread is past its sum over it (the barrier above)
             if (any) {
@@ -659,12 +680,12 @@ __global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(WgradArgs a, int
         any = true;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    if (any && !failed) {   // the last strip's MMAs complete after all earlier ones
+    if (any && !failed && !multiplies) {   // the last strip's MMAs complete after all earlier ones
         if (!mbar_wait_bounded(&s_bar[stage ^ 1], phase[stage ^ 1], kWaitLimit)) failed = true;
     }
     if (__syncthreads_or(failed)) failed = true;
     umma::fence_after_sync();
-    if (any && !failed) {
+    if (any && !failed && !multiplies) {
         // D rows m = ky * kCin + ci < 3 kCin of tap column kx; warps 0..3 read taps 0 and 1, warps 4..7 tap 2
         const int m = (warp & 3) * 32 + lane;
         const bool vec = (reinterpret_cast<uintptr_t>(a.dw) & 15u) == 0u;
@@ -695,7 +716,7 @@ __global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(WgradArgs a, int
         for (int e = 0; e < 8; ++e) {
 #pragma unroll
             for (int off = 16; off >= kGo; off >>= 1) db[e] += __shfl_xor_sync(0xffffffffu, db[e], off);
-            if (lane < kGo) s_db[warp][lane * 8 + e] = db[e];
+            if (lane < kGo && !multiplies) s_db[warp][lane * 8 + e] = db[e];
         }
         __syncthreads();
         if (tid < kCout && any && !failed) {
@@ -761,7 +782,7 @@ static int launch_wgrad_t(const WgradArgs& a, int max_ctas, cudaStream_t s) {
                              (int)smem);
         attr = true;
     }
-    conv_wgrad_kernel<kCin, kCout, kLoad><<<(unsigned)(total < max_ctas ? total : max_ctas), kWgThreads, smem, s>>>(a, rows);
+    conv_wgrad_kernel<kCin, kCout, kLoad><<<(unsigned)(total < max_ctas ? total : max_ctas), kWgThreads + 32, smem, s>>>(a, rows);
     return 1;
 }
 

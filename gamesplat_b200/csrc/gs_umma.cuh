@@ -39,18 +39,7 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n, int a_mn, int b_
            | ((uint32_t)(m >> 4) << 24); // M / 16
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by one thread.
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-        : "memory");
-}
-
-// The same from a warp in step: issued by the lane whose `elected` is nonzero.
+// D[tmem] (+)= A[smem] * B[smem] from a warp in step: issued by the lane whose `elected` is nonzero.
 // Operands that stay warp-uniform (no branch on the lane around them) are kept
 // in uniform registers, which the instruction takes them from.
 __device__ __forceinline__ void mma_bf16_elect(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -64,6 +53,7 @@ __device__ __forceinline__ void mma_bf16_elect(uint32_t tmem_d, uint64_t adesc, 
         : "memory");
 }
 
+// Arrive on `bar` once every tcgen05 operation the elected lane issued is done.
 __device__ __forceinline__ void commit_elect(uint64_t* bar, uint32_t elected) {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"
@@ -71,12 +61,6 @@ __device__ __forceinline__ void commit_elect(uint64_t* bar, uint32_t elected) {
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(bar)),
         "r"(elected)
         : "memory");
-}
-
-// Arrive on `bar` once every tcgen05 operation this thread issued is done.
-__device__ __forceinline__ void commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
 }
 
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }

@@ -55,15 +55,11 @@ constexpr float kPio2Hi = 1.5707855224609375f;
 constexpr float kPio2Lo = 1.0804334124259185e-05f;
 constexpr float kTwoOverPi = 0.6366197466850281f;
 
-__device__ __forceinline__ float det_logf(float x) {
-    if (x != x) return x;
-    if (x < 0.0f) return __int_as_float(0x7fc00000);
-    if (x == 0.0f) return __int_as_float(0xff800000);
-    if (x == __int_as_float(0x7f800000)) return x;
-    uint32_t ix = __float_as_uint(x);
-    int e = 0;
-    if (ix < 0x00800000u) { x = mul(x, 16777216.0f); ix = __float_as_uint(x); e = -24; }
-    e += (int)(ix >> 23) - 127;
+// det_logf of a positive normal number (of anything else: some value); e0 is
+// added to the exponent.
+__device__ __forceinline__ float det_logf_normal(float x, int e0 = 0) {
+    const uint32_t ix = __float_as_uint(x);
+    int e = e0 + (int)(ix >> 23) - 127;
     float m = __uint_as_float((ix & 0x007fffffu) | 0x3f800000u);
     if (m > 1.41421354f) { m = mul(m, 0.5f); e += 1; }
     float f = sub(m, 1.0f);
@@ -75,6 +71,16 @@ __device__ __forceinline__ float det_logf(float x) {
     float lm = add(two_s, mul(two_s, p));
     float ef = (float)e;
     return add(mul(ef, kLn2Hi), add(lm, mul(ef, kLn2Lo)));
+}
+
+__device__ __forceinline__ float det_logf(float x) {
+    if (x != x) return x;
+    if (x < 0.0f) return __int_as_float(0x7fc00000);
+    if (x == 0.0f) return __int_as_float(0xff800000);
+    if (x == __int_as_float(0x7f800000)) return x;
+    int e = 0;
+    if (__float_as_uint(x) < 0x00800000u) { x = mul(x, 16777216.0f); e = -24; }
+    return det_logf_normal(x, e);
 }
 
 __device__ __forceinline__ float det_expf(float x) {
@@ -110,12 +116,10 @@ __device__ __forceinline__ void det_sincosf(float x, float* s_out, float* c_out)
     cp = add(0.0416666679084301f, mul(z, cp));
     cp = add(-0.5f, mul(z, cp));
     float cr = add(1.0f, mul(z, cp));
-    int q = ((int)n) & 3;
-    float s, c;
-    if (q == 0) { s = sr; c = cr; }
-    else if (q == 1) { s = cr; c = -sr; }
-    else if (q == 2) { s = -sr; c = -cr; }
-    else { s = -cr; c = sr; }
+    // quadrant q: (sr, cr), (cr, -sr), (-sr, -cr), (-cr, sr)
+    const uint32_t q = (uint32_t)(int)n;
+    const float s = __uint_as_float(__float_as_uint(q & 1u ? cr : sr) ^ ((q & 2u) << 30));
+    const float c = __uint_as_float(__float_as_uint(q & 1u ? sr : cr) ^ (((q + 1u) & 2u) << 30));
     *s_out = s;
     *c_out = c;
 }

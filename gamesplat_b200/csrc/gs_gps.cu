@@ -143,8 +143,14 @@ __global__ void __launch_bounds__(256) gps_expand_kernel(GpsParams p, float4* __
     }
 }
 
-__global__ void gps_splat_kernel(GpsParams p, const float4* __restrict__ prepared, const uint2* __restrict__ work,
-                                 unsigned long long* __restrict__ packed) {
+// One work item a thread.  Bound by instructions issued (81 % of the slots): the
+// deterministic inverse dilogarithm, logarithm and sine of a point.  The
+// logarithm's argument is clamped to [1e-7, 1], so its special cases are left out;
+// 31 registers fill the SM.  1M Gaussians, 1280x720, supersample 2: the
+// GPS stage (splat, expansion, clear) 525 -> 496 us, 9 of it by the registers.
+__global__ void __launch_bounds__(256, 8) gps_splat_kernel(GpsParams p, const float4* __restrict__ prepared,
+                                                           const uint2* __restrict__ work,
+                                                           unsigned long long* __restrict__ packed) {
     pdl_wait();   // launched as a programmatic dependent of the frame's previous kernel
     const uint32_t total = min(p.fc->gps_work[0], p.max_work_items);
     const int gw = p.width * (int)p.supersample, gh = p.height * (int)p.supersample;
@@ -176,7 +182,7 @@ __global__ void gps_splat_kernel(GpsParams p, const float4* __restrict__ prepare
             const float r1 = mul(__uint2float_rn(sy), 2.32830643654e-10f);
             float arg = dv(det_inv_dilog(mul(sub(1.0f, r0), sm.z)), sm.y);
             arg = g_clamp(arg, 1.0e-7f, 1.0f);
-            const float radius = __fsqrt_rn(mul(-2.0f, det_logf(arg)));
+            const float radius = __fsqrt_rn(mul(-2.0f, det_logf_normal(arg)));   // a NaN is turned away below
             const float az = mul(6.28318530718f, r1);
             float sn, cs;
             det_sincosf(az, &sn, &cs);
@@ -184,7 +190,7 @@ __global__ void gps_splat_kernel(GpsParams p, const float4* __restrict__ prepare
             const float ptx = mul(add(mb.x, mul(mb.z, lx)), g_max(ss, 1.0f));
             const float pty = mul(add(mb.y, add(mul(mb.w, lx), mul(sm.x, ly))), g_max(ss, 1.0f));
             const float fx = floorf(add(ptx, 0.5f)), fy = floorf(add(pty, 0.5f));
-            if (fx >= 0.0f && fy >= 0.0f && fx < (float)gw && fy < (float)gh) {
+            if (arg == arg && fx >= 0.0f && fy >= 0.0f && fx < (float)gw && fy < (float)gh) {
                 unsigned long long* dst = packed + (size_t)fy * gw + (size_t)fx;
                 if (val < *reinterpret_cast<volatile unsigned long long*>(dst)) atomicMin(dst, val);
             }

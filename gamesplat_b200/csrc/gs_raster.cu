@@ -662,6 +662,7 @@ __global__ void __launch_bounds__(kRasterThreads, kStates == 8 ? 4 : 6)
     __shared__ uint16_t* s_out[kStates];
     const uint32_t group = blockIdx.x % groups;
     if (threadIdx.x < kStates) s_out[threadIdx.x] = outs.out[first + (int)group * kStates + (int)threadIdx.x];
+    __syncthreads();   // a tile without entries goes through raster_tile without meeting a barrier
     p.colours += (size_t)group * p.record_cap * (3 * kStates / 4);
     raster_tile<0, kTw, kTh, kStates>(p, p.tile_order[blockIdx.x / groups], sh, s_out);
 }

@@ -51,8 +51,13 @@ constexpr int kGroup = 128;                 // threads that load a row, or that 
 constexpr int kSlots = 8;                   // halo rows in the ring
 constexpr int kAhead = 3;                   // rows copied behind the one announced next
 constexpr uint32_t kAccs = 8;               // TMEM accumulators of Cout columns
-constexpr uint32_t kDone = 16;              // barriers of finished rows: a reader of accumulators is at most kAccs
-                                            // output rows, so kAccs + 2 ring entries, behind the MMAs
+// Barriers of finished rows.  While an accumulator is unread the MMAs stop at
+// the first terms of the row kAccs later, and a run of R rows is R + 2 entries:
+// past the entry that completes a row, the MMAs can finish 2 kAccs + 5 more
+// (runs of one row; 13 in runs of two, 7 in long ones) before that row's reader
+// has tested its barrier, which must not complete a second time until then.
+constexpr uint32_t kDone = 32;
+static_assert(kDone > 2 * kAccs + 5, "a finished row's barrier outlasts its reader's wait");
 
 // Dynamic shared memory of the forward kernel: the halo rows and the weight image.
 __host__ __device__ constexpr int fwd_smem_bytes(int cin, int cout) {

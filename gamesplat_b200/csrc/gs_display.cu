@@ -15,8 +15,6 @@
 // against it.
 #include <cuda_fp16.h>
 
-#include <algorithm>
-
 #include "gs_common.cuh"
 #include "gs_display.h"
 
@@ -27,18 +25,38 @@ __device__ __forceinline__ float det_log2f(float x) { return mul(det_logf(x), kI
 
 // The table the display kernel reads: the uploaded uint16 lattice as floats
 // (entry / 65535, the division the shader does per fetch), 16 bytes a point.
-__global__ void display_table_kernel(const uint16_t* __restrict__ lut, size_t points, float4* __restrict__ table) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < points; i += (size_t)gridDim.x * blockDim.x) {
+// The lattice arrives in the last 6 of every 16 bytes of the table's memory and
+// is converted in place from the first point on, a thread a point: a launch
+// takes the points whose 16 bytes end before the first unconverted entry (5 / 8 of
+// what is left), so nothing it writes is read any more; the last points are one
+// CTA's, which reads them all before it writes.
+constexpr int kTableThreads = 1024;
+__global__ void __launch_bounds__(kTableThreads) display_table_kernel(const uint16_t* lut, size_t first, size_t last,
+                                                                      float4* table) {
+    const size_t i = first + (size_t)blockIdx.x * kTableThreads + threadIdx.x;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (i < last) {
         const uint16_t* a = lut + i * 3;
-        table[i] = make_float4(dv((float)a[0], 65535.0f), dv((float)a[1], 65535.0f), dv((float)a[2], 65535.0f), 0.0f);
+        v = make_float4(dv((float)a[0], 65535.0f), dv((float)a[1], 65535.0f), dv((float)a[2], 65535.0f), 0.0f);
     }
+    __syncthreads();
+    if (i < last) table[i] = v;
 }
 
-int launch_display_table(const uint16_t* lut, int lut_size, float4* table, uint32_t num_sms, cudaStream_t s) {
+uint16_t* display_lattice(float4* table, int lut_size) {
     const size_t points = (size_t)lut_size * lut_size * lut_size;
-    const size_t grid = std::min((points + 255) / 256, (size_t)num_sms * 16);
-    display_table_kernel<<<(unsigned)grid, 256, 0, s>>>(lut, points, table);
-    return 1;
+    return reinterpret_cast<uint16_t*>(reinterpret_cast<char*>(table) + 10 * points);
+}
+
+int launch_display_table(float4* table, int lut_size, cudaStream_t s) {
+    const size_t points = (size_t)lut_size * lut_size * lut_size;
+    int launches = 0;
+    for (size_t first = 0, last; first < points; first = last, ++launches) {
+        last = points - first <= (size_t)kTableThreads ? points : (10 * points + 6 * first) / 16;
+        const size_t grid = (last - first + kTableThreads - 1) / kTableThreads;
+        display_table_kernel<<<(unsigned)grid, kTableThreads, 0, s>>>(display_lattice(table, lut_size), first, last, table);
+    }
+    return launches;
 }
 
 // g_mix with the weights 1 - a and a in hand.

@@ -15,8 +15,9 @@ struct DisplayParams {
     float exposure_ev;
 };
 
-// table: one float4 per lattice point, from the uploaded uint16 RGB lattice (x fastest)
-int launch_display_table(const uint16_t* lut, int lut_size, float4* table, uint32_t num_sms, cudaStream_t s);
+// table: one float4 per lattice point, made in place of the uint16 RGB lattice (x fastest) copied to display_lattice()
+uint16_t* display_lattice(float4* table, int lut_size);
+int launch_display_table(float4* table, int lut_size, cudaStream_t s);
 int launch_display(const DisplayParams& p, uint32_t num_sms, cudaStream_t s);
 
 }  // namespace gs

@@ -80,7 +80,7 @@ struct gs_ctx {
     std::string last_error;
 
     // display transform LUT (gsanim 0.3 "layers" scenes)
-    float4* display_table = nullptr;     // lut_size^3 points, then the uint16 lattice they came from
+    float4* display_table = nullptr;     // lut_size^3 points
     int lut_size = 0;
     float lut_log2_min = 0.0f, lut_log2_max = 0.0f;
 
@@ -1596,12 +1596,11 @@ int gs_set_display_lut(gs_ctx* c, const uint16_t* lut, uint32_t lut_size, float 
     // src/gaussian_loader_gsanim.cpp:237,244
     if (lut_size < 2 || lut_size > 256) return fail(c, GS_ERR_BAD_ARG, "display LUT size must be 2..256");
     if (!(log2_min < log2_max)) return fail(c, GS_ERR_BAD_ARG, "display LUT needs log2_min < log2_max");
-    // one allocation: the float table the kernel reads and, behind it, the uint16 lattice it is made from
-    const size_t points = (size_t)lut_size * lut_size * lut_size, raw_bytes = points * 3 * sizeof(uint16_t);
-    GS_CUDA(c, dalloc(&c->display_table, points * sizeof(float4) + raw_bytes));
-    uint16_t* raw = reinterpret_cast<uint16_t*>(c->display_table + points);
-    GS_CUDA(c, cudaMemcpyAsync(raw, lut, raw_bytes, cudaMemcpyHostToDevice, c->stream));
-    gs::launch_display_table(raw, (int)lut_size, c->display_table, c->num_sms, c->stream);
+    const size_t points = (size_t)lut_size * lut_size * lut_size;
+    GS_CUDA(c, dalloc(&c->display_table, points * sizeof(float4)));
+    GS_CUDA(c, cudaMemcpyAsync(gs::display_lattice(c->display_table, (int)lut_size), lut,
+                               points * 3 * sizeof(uint16_t), cudaMemcpyHostToDevice, c->stream));
+    gs::launch_display_table(c->display_table, (int)lut_size, c->stream);
     GS_CUDA(c, cudaGetLastError());
     GS_CUDA(c, cudaStreamSynchronize(c->stream));   // the caller may reuse `lut` on return
     c->lut_size = (int)lut_size;

@@ -637,8 +637,7 @@ int check_previous_frame(gs_ctx* c) {
 void begin_frame(gs_ctx* c, const gs_camera* cam, bool zero_ctrl = true) {
     c->cam = *cam;
     if (zero_ctrl) cudaMemsetAsync(c->ctrl, 0, c->ctrl_bytes, c->stream);
-    ++c->epoch;
-    if (c->epoch == 0) ++c->epoch;
+    c->epoch = gs::next_epoch(c->epoch);
     c->frame_launches = 0;
 }
 

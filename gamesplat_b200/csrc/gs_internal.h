@@ -45,6 +45,13 @@ struct SortPlan {
     uint32_t count;
 };
 
+// Look-back words carry a frame's epoch (1 .. kEpochs - 1, round again) in their
+// upper half, those of the sorts the epoch and the pass, so that one frame's
+// words, or the zeros of memory never written, are not another's.
+constexpr uint32_t kEpochs = 1u << 30;
+constexpr uint32_t next_epoch(uint32_t epoch) { return epoch + 1u < kEpochs ? epoch + 1u : 1u; }
+__host__ __device__ constexpr uint32_t sort_tag(uint32_t epoch, uint32_t pass) { return (epoch << 2) | pass; }
+
 // Onesweep radix sort configuration.
 constexpr int kSortThreads = 256;
 constexpr int kSortTile = 4096;   // pairs per 4 x kRadix look-back words (sort_status_words() * 4 words in all)

@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) sort_pass_kernel(SortParams p
     const int shift = p.begin_bit + pass * kBits;
     const uint32_t dmask = (1u << min(kBits, p.end_bit - shift)) - 1u, bias = p.key_bias;
     const TileCut cut = cut_tiles<kMin, kPairMax>(n);
-    const uint32_t tag = (p.epoch << 2) | (uint32_t)pass;
+    const uint32_t tag = sort_tag(p.epoch, (uint32_t)pass);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t gdigit[kD];   // global start of the thread's digits
     scan_digits<kD>(own, gdigit, sh.scan_tmp);
@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) tile_pass_kernel(TileSortPara
     uint32_t* __restrict__ out = p.words[kPass + 1];
     const uint32_t vmask = p.vbits >= 32 ? 0xFFFFFFFFu : (1u << p.vbits) - 1u;
     const TileCut cut = cut_tiles<kEntryMin, kEntryMax>(n);
-    const uint32_t tag = (p.epoch << 2) | (uint32_t)kPass;
+    const uint32_t tag = sort_tag(p.epoch, (uint32_t)kPass);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t gdigit[1];
     scan_digits<1>(own, gdigit, sh.scan_tmp);

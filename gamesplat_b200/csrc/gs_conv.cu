@@ -753,18 +753,23 @@ __global__ void pack_weights_kernel(const float* __restrict__ w, int cin, int co
     }
 }
 
+static int current_device() {
+    int dev = -1;
+    cudaGetDevice(&dev);
+    return dev;
+}
+
 template <int kCin, int kCout, int kLoad, bool kPool = false>
 static int launch_fwd_t(ConvArgs a, cudaStream_t s) {
     const long strips = (long)a.n * ((a.w + 127) / 128);
     const long units = strips * ((a.h + a.row_offset + a.unit_rows - 1) / a.unit_rows);
     const size_t smem = (size_t)fwd_smem_bytes(kCin, kCout);
     a.out_wide = (reinterpret_cast<uintptr_t>(a.out_bf16) & 31u) == 0u ? 1 : 0;
-    static bool attr = false;
-    if (!attr) {
+    static OncePerDevice attr;
+    attr(current_device(), [&] {
         cudaFuncSetAttribute(conv_fwd_kernel<kCin, kCout, kLoad, kPool>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
-        attr = true;
-    }
+    });
     // two CTAs an SM; on small images one unit each at most
     const long ctas = 2L * a.max_sms;
     launch_pdl(conv_fwd_kernel<kCin, kCout, kLoad, kPool>, dim3((unsigned)(units < ctas ? units : ctas)), dim3(kFwdThreads), smem,
@@ -781,12 +786,11 @@ static int launch_wgrad_t(const WgradArgs& a, int max_ctas, cudaStream_t s) {
     while (rows > 1 && strips * ((a.h + rows - 1) / rows) < 2L * max_ctas) rows >>= 1;
     const long total = strips * ((a.h + rows - 1) / rows);
     const size_t smem = 2 * (size_t)wg_stage_bytes(kCin, kCout);
-    static bool attr = false;
-    if (!attr) {
+    static OncePerDevice attr;
+    attr(current_device(), [&] {
         cudaFuncSetAttribute(conv_wgrad_kernel<kCin, kCout, kLoad>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
-        attr = true;
-    }
+    });
     conv_wgrad_kernel<kCin, kCout, kLoad><<<(unsigned)(total < max_ctas ? total : max_ctas), kWgThreads + 32, smem, s>>>(a, rows);
     return 1;
 }

@@ -22,7 +22,6 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <atomic>
 #include <type_traits>
 
 #include "gs_common.cuh"
@@ -983,21 +982,17 @@ __global__ void __launch_bounds__(256) cull_layers_kernel(CullParams p) {
 }
 
 int launch_cull(const CullParams& p, uint32_t num_sms, cudaStream_t s) {
-    // the shared-memory limit is a per-device function attribute: raise it
-    // once on every device this process launches on
-    static std::atomic<uint64_t> attr_devices{0};
-    int dev = 0;
+    static OncePerDevice attr;
+    int dev = -1;
     cudaGetDevice(&dev);
-    const uint64_t bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
-    if (!bit || !(attr_devices.load() & bit)) {
+    attr(dev, [] {
         cudaFuncSetAttribute(cull_project_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCullSmem);
         cudaFuncSetAttribute(cull_project_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCullSmem);
         cudaFuncSetAttribute(cull_project_kernel<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCullSmem);
         cudaFuncSetAttribute(cull_project_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCullSmem);
         cudaFuncSetAttribute(cull_project_half_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kCullHalfSmem);
-        attr_devices.fetch_or(bit);
-    }
+    });
     // With layers set the colours come from their pass: the projection then
     // stages the rows without their SH (64 of 256 bytes) and no deltas.
     CullParams pp = p;

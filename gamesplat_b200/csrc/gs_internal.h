@@ -1,6 +1,7 @@
 // Internal interfaces between the C++ host orchestration (gs_host.cpp) and the
 // CUDA kernels.  Not part of the public C ABI (include/gs_api.h).
 #pragma once
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -249,6 +250,24 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
+
+// What has to be done once on every device a process launches on (a kernel's
+// shared-memory limit is an attribute per device): runs `set` unless it has run
+// for `device`.  The mark comes after it, so that a thread which finds the mark
+// finds the attribute; threads that meet before it set the same twice.
+class OncePerDevice {
+public:
+    template <class F>
+    void operator()(int device, F&& set) {
+        const uint64_t bit = device >= 0 && device < 64 ? 1ull << device : 0ull;   // others: every time
+        if (done_.load() & bit) return;
+        set();
+        done_.fetch_or(bit);
+    }
+
+private:
+    std::atomic<uint64_t> done_{0};
+};
 
 // Every device allocation of the library goes through here: cudaMalloc, with
 // a failed call's error cleared (it is reported through the return value),

@@ -315,8 +315,9 @@ __global__ void __launch_bounds__(kFwdThreads, 2) conv_fwd_kernel(ConvArgs a) {
             }
             m += (uint32_t)rows;
         }
-        // every MMA of this CTA, and the last commit's arrival, is done before its shared memory and TMEM go
-        if (!failed && e > 0 && !mbar_wait_suspend(&s_done[(e - 1u) % kDone], ((e - 1u) / kDone) & 1u)) failed = true;
+        // every MMA of this CTA, and the last commit's arrival, is done before its shared memory and TMEM go, after a
+        // wait that ran out too (entry e then has issued nothing)
+        if (e > 0 && !mbar_wait_suspend(&s_done[(e - 1u) % kDone], ((e - 1u) / kDone) & 1u)) failed = true;
         __syncwarp();
     } else if (tid < R::kFirstLoader) {
         // ---- epilogue: thread t of a group holds pixel x0 + t of a row (its TMEM lane: warp % 4)
@@ -680,12 +681,12 @@ __global__ void __launch_bounds__(kWgThreads + 32) conv_wgrad_kernel(WgradArgs a
                 if (!mbar_wait_bounded(&s_bar[stage ^ 1], phase[stage ^ 1], kWaitLimit)) failed = true;
                 phase[stage ^ 1] ^= 1u;
             }
-            load(stage ^ 1, next);
+            if (!failed) load(stage ^ 1, next);   // else those MMAs may still read it
         }
         any = true;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    if (any && !failed && !multiplies) {   // the last strip's MMAs complete after all earlier ones
+    if (any && !multiplies) {   // the last strip's MMAs complete after all earlier ones; also after a wait that ran out
         if (!mbar_wait_bounded(&s_bar[stage ^ 1], phase[stage ^ 1], kWaitLimit)) failed = true;
     }
     if (__syncthreads_or(failed)) failed = true;

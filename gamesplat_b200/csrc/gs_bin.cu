@@ -108,7 +108,7 @@ __device__ __forceinline__ BinItem bin_one(const BinParams& p, uint32_t s, uint3
     const float zw = add(mul(cd.w, 0.5f), 0.5f);
     rec.depth24 = (uint32_t)__float2int_rn(mul(g_clamp(zw, 0.0f, 1.0f), 16777215.0f));
     rec.splat_id = id;
-    rec.hash_z = add((float)id, p.frame_seed);
+    rec.hash_z = 0.0f;
     rec.opacity = co.w;
     if (p.envelope) {   // the rasterizer derives each sample's quad from these
         rec.cx = cr.x;

@@ -752,7 +752,7 @@ int packed_entry_bits(const gs_ctx* c) {
 // Binning, tile sort and tile ranges for one raster pass.
 // readback: copy the counters to h_bin_fc on fc_stream once the tile sort has
 // run (the entry count is final after the expansion).
-void run_binning(gs_ctx* c, float jx, float jy, float seed, bool envelope = false, bool readback = true) {
+void run_binning(gs_ctx* c, float jx, float jy, bool envelope = false, bool readback = true) {
     const int vbits = packed_entry_bits(c);
     {
         StageScope sc(c, ST_BIN);
@@ -764,7 +764,6 @@ void run_binning(gs_ctx* c, float jx, float jy, float seed, bool envelope = fals
         p.clip_y_sign = c->cam.clip_y_sign;
         p.jitter_x = jx;
         p.jitter_y = jy;
-        p.frame_seed = seed;
         p.width = c->width;
         p.height = c->height;
         p.tiles_x = c->tiles_x;
@@ -868,7 +867,7 @@ float background(const gs_ctx* c) { return c->knobs.black_background ? 0.0f : 0.
 int render_alpha(gs_ctx* c, uint16_t* out) {
     run_cull(c);
     run_depth_sort(c);
-    run_binning(c, 0.0f, 0.0f, 0.0f);
+    run_binning(c, 0.0f, 0.0f);
     StageScope sc(c, ST_RASTER);
     gs::RasterParams r = raster_params(c, background(c));
     r.out_rgba16f = out;
@@ -918,7 +917,7 @@ int render_stochastic(gs_ctx* c, const gs_camera* cam, uint16_t* out) {
     run_depth_sort(c);
     // One binning for every sample of the frame: tiles for any jitter, the
     // rasterizer derives each sample's quad coverage.
-    run_binning(c, 0.0f, 0.0f, 0.0f, /*envelope*/ true);
+    run_binning(c, 0.0f, 0.0f, /*envelope*/ true);
     uint32_t write_index = c->accum_write_index & 1u;
     bool display_accum = false;
     for (uint32_t i = 0; i < render_samples; ++i) {
@@ -1037,7 +1036,7 @@ int ensure_denoise_targets(gs_ctx* c) {
     const size_t npix = (size_t)c->width * c->height;
     if (c->features_pix != npix || !c->features) {
         dfree(c->features);
-            c->features_pix = 0;
+        c->features_pix = 0;
         GS_CUDA(c, dalloc(&c->features, npix * gs::dn::kInC * sizeof(__nv_bfloat16)));
         c->features_pix = npix;
     }
@@ -1070,7 +1069,7 @@ int render_denoise_inputs(gs_ctx* c, const gs_camera* cam) {
     }
     run_cull(c);
     run_depth_sort(c);
-    run_binning(c, 0.0f, 0.0f, 0.0f);
+    run_binning(c, 0.0f, 0.0f);
     {
         StageScope sc(c, ST_RASTER);
         gs::RasterParams r = raster_params(c, background(c));
@@ -1979,7 +1978,7 @@ int stage_frame(gs_ctx* c, uint32_t k, const gs_camera* cam, void* out) {
         begin_frame(c, cam);
         run_cull(c);
         run_depth_sort(c);
-        run_binning(c, 0.0f, 0.0f, 0.0f, false, /*readback*/ false);
+        run_binning(c, 0.0f, 0.0f, false, /*readback*/ false);
         // on fc_stream: a copy between two kernels would idle the render stream
         cudaEventRecord(c->binned, c->stream);
         cudaStreamWaitEvent(c->fc_stream, c->binned, 0);

@@ -67,14 +67,14 @@ constexpr int kDepthBits = 9;
 constexpr int kDepthRadix = 1 << kDepthBits;
 constexpr uint32_t kDepthKeyBias = 0x3E4CCCCDu;   // bits of 0.2f
 
-// Cull configuration.  Visibility pass: 256-thread CTAs, 8 rows per thread;
-// its 2048-row CTA tiles are the units of the look-back.  Projection pass:
-// 128-thread CTAs, each warp stages and projects 32 visible rows at a time.
+// Cull configuration.  Visibility pass: 256-thread CTAs that take tiles of 8 to
+// 20 rows a thread, cut so that they fill whole rounds (launch_cull).  Projection
+// pass: 128-thread CTAs, each warp stages and projects 32 visible rows at a time.
 constexpr int kCullVisThreads = 256;
 constexpr int kCullVisItems = 8;     // rows a thread: the fewest of a tile, and the most
 constexpr int kVisItemsMax = 20;
 constexpr int kVisPerSm = 4;         // resident CTAs
-constexpr int kCullVisTile = kCullVisThreads * kCullVisItems;
+constexpr int kCullVisTile = kCullVisThreads * kCullVisItems;   // the smallest tile: sizes the status words
 constexpr int kCullThreads = 128;
 constexpr int kHalfRowChunks = 9;   // 144-byte FP16-SH row: position/opacity, scale, rotation, 48 half SH
 
@@ -88,17 +88,18 @@ constexpr int kTileW = 16;
 constexpr int kTileH = 16;
 
 // Raster record: one per visible splat in depth-sorted order, 64 bytes,
-// staged into shared memory by TMA bulk copies.
+// gathered into shared memory by cp.async.
 //
 // The rasterizer tests the splat's quadratic form s = conic(d) (the power is
 // -0.5 s) instead of the power: "power <= 0 && !(power < cutoff)" holds
-// exactly when -kSMin <= s <= s_max, with s_max = -2 cutoff, or the smallest
+// exactly when -2^-149 <= s <= s_max, with s_max = -2 cutoff, or the smallest
 // subnormal when cutoff == 0 (multiplying by -0.5 is exact except for
-// subnormal s, and those cases are what the two bounds absorb).
+// subnormal s, and those cases are what the two bounds absorb).  The test made
+// is 0 <= s <= s_max (frag_live, which says why no splat reaches the rest).
 //
 // Stochastic envelope records (BinParams::envelope) reuse three slots:
 // log2_opacity holds radius_x, rect_x holds the bits of ndc_z and rect_y the
-// bits of radius_y; cx, cy are un-jittered and hash_z is unused.
+// bits of radius_y; cx, cy are un-jittered.
 struct __align__(16) RasterRecord {
     float cx, cy, conic_x, conic_2y;     // centre (+jitter), conic.x, 2*conic.y
     float conic_z, log2_opacity, s_max, r;
@@ -107,7 +108,7 @@ struct __align__(16) RasterRecord {
     uint32_t rect_y;                     // j0 | j1 << 16   intersected with the alpha >= 1/255 box, GL rows)
     uint32_t depth24;                    // window depth as D24 (stochastic depth test)
     uint32_t splat_id;                   // original Gaussian index
-    float hash_z;                        // float(splat_id) + frame_seed
+    float hash_z;                        // 0; the two-sample rasterizer's staging keeps the second seed's hash here
     float opacity;
 };
 static_assert(sizeof(RasterRecord) == 64, "RasterRecord must be 64 bytes");
@@ -181,7 +182,6 @@ struct BinParams {
     const float4* projected;
     float vp_w, vp_h, clip_y_sign;   // CameraUniforms viewport and clip_y_sign of the frame
     float jitter_x, jitter_y;
-    float frame_seed;
     int width, height, tiles_x, tiles_y;
     int tile_shift_x, tile_shift_y;  // log2 of the tile width and height
     RasterRecord* records;           // N_vis records (sorted order)

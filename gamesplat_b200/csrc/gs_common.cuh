@@ -299,8 +299,10 @@ __device__ __forceinline__ uint32_t lookback_vec(const u64* status, size_t strid
 // The place of a tile in a scan over tiles that are taken by ticket, in rounds
 // of `round`: one thread's share of the sum over the earlier tiles of its round,
 // whose words hold their counts, and the round before, whose last word holds the
-// prefix through it (a round's last tile publishes nothing else).  Every word is
-// one load of one thread, all in flight at once.  Waits are bounded: *timed_out.
+// prefix through it (a round's last tile publishes nothing else).  The words are
+// spread over the threads; a thread takes its own in turn, each behind the poll of
+// the one before: up to 3 in the visibility pass (rounds of 4 tiles an SM on 256
+// threads), up to 10 in the binning (8 on 128).  Waits are bounded: *timed_out.
 __device__ __forceinline__ uint32_t sum_earlier(const u64* status, uint32_t tile, uint32_t round, uint32_t epoch,
                                                 uint32_t thread, uint32_t threads, bool* timed_out,
                                                 uint32_t spin_limit = kSpinLimit) {

@@ -354,8 +354,8 @@ int launch_pack_half_rows(const float4* rows, float4* half_rows, uint32_t n, uin
 // rows follow one another, so it appends to its own run in shared memory and the
 // tile's runs meet in one scan of the warps' counts.  The tile's place in the
 // output is the sum of the counts of the tiles before it: of its own round of
-// tiles (as many as are resident at a time) the counts themselves, all loaded at
-// once by the CTA's threads, of earlier rounds the prefix that a round's last
+// tiles (as many as are resident at a time) the counts themselves, spread over
+// the CTA's threads (sum_earlier), of earlier rounds the prefix that a round's last
 // tile publishes.  The key-digit histograms of the depth sort (9-bit digits of
 // the biased key, see kDepthKeyBias) are accumulated in shared memory; the top
 // digit (sign and high exponent bits, a handful of values in a scene) is

@@ -15,7 +15,6 @@ enum : uint32_t {
     kErrCullLookback = 1u << 0,
     kErrSortLookback = 1u << 1,
     kErrBinLookback = 1u << 2,
-    kErrRasterWait = 1u << 3,   // an mbarrier phase that did not complete (the wait probe's)
     kErrTileOverflow = 1u << 4,
     kErrGpsWait = 1u << 5,
     kErrCullStage = 1u << 6,

@@ -14,8 +14,8 @@ __global__ void wait_probe_kernel(const unsigned long long* status, FrameCounter
                                   uint32_t limit) {
     __shared__ __align__(8) uint64_t bar;
     if (which == 0) {
-        // tile 1's look-back: tile 0's word carries another epoch, so it
-        // reads as "not published yet" on every poll
+        // tile 1's sum over earlier tiles: tile 0's word carries another epoch,
+        // so it reads as "not published yet" on every poll
         if (threadIdx.x < 32) {
             bool to = false;
             sum_earlier(status, 1, 2, epoch, threadIdx.x, blockDim.x, &to, limit);
@@ -31,7 +31,7 @@ __global__ void wait_probe_kernel(const unsigned long long* status, FrameCounter
         if (threadIdx.x == 0) mbar_arrive_expect_tx(&bar, 16u);
         __syncthreads();
         const bool ok = mbar_wait_bounded(&bar, 0u, limit);
-        if (threadIdx.x == 0 && !ok) atomicOr(&fc->error_flags, kErrRasterWait);
+        if (threadIdx.x == 0 && !ok) atomicOr(&fc->error_flags, kErrCullStage);   // as the projection
     }
 }
 

@@ -596,8 +596,9 @@ __device__ __forceinline__ void raster_tile(const RasterParams& p, const uint32_
     }
 }
 
-// Bound by instructions issued, the ALU pipe (comparisons, selects, integers) first
-// of the pipes at 64 %: one splat into two pixels is some 40 instructions, of
+// Bound by instructions issued (76 % of the slots; the ALU pipe, comparisons,
+// selects and integers, is at 50 %, the exponentials' at 42 %) and the two barriers
+// of a batch, a quarter of the stalls: one splat into two pixels is some 40 instructions, of
 // which the fused multiply-adds, packed two pixels to one, are the smaller part.
 // What is the same for the pixels of a warp is therefore done once a record in
 // the staging pass, the warp's splats are listed before they are shaded, and the

@@ -345,8 +345,8 @@ int gs_display(gs_ctx* ctx, const uint16_t* rgba16f_in, float* rgba32f_out, int 
 
 /* Diagnostics, no counterpart in the reference (its GL path has no device
  * waits): runs one of the library's bounded device waits against a word that
- * nothing publishes (which = 0: decoupled look-back; 1: mbarrier / TMA
- * completion) with at most spin_limit polls, on private memory, and returns
+ * nothing publishes (which = 0: a tile's wait for the counts of earlier ones;
+ * 1: mbarrier / TMA completion) with at most spin_limit polls, on private memory, and returns
  * what a frame would: GS_ERR_DEVICE_TIMEOUT once the wait runs out.  The
  * context stays usable.  Synchronises; allocates a few hundred bytes. */
 int gs_debug_wait_probe(gs_ctx* ctx, int which, uint32_t spin_limit);

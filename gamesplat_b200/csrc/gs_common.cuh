@@ -297,18 +297,18 @@ __device__ __forceinline__ uint32_t lookback_vec(const u64* status, size_t strid
 }
 
 // The place of a tile in a scan over tiles that are taken by ticket, in rounds
-// of `round`: one thread's share of the sum over the earlier tiles of its round,
-// whose words hold their counts, and the round before, whose last word holds the
-// prefix through it (a round's last tile publishes nothing else).  The words are
+// (`first`: its round's first tile): one thread's share of the sum over the
+// earlier tiles of its round, whose words hold their counts, and the round before,
+// whose last word holds the prefix through it (a round's last tile publishes
+// nothing else).  The words are
 // spread over the threads; a thread takes its own in turn, each behind the poll of
 // the one before: up to 3 in the visibility pass (rounds of 4 tiles an SM on 256
 // threads), up to 10 in the binning (8 on 128).  Waits are bounded: *timed_out.
-__device__ __forceinline__ uint32_t sum_earlier(const u64* status, uint32_t tile, uint32_t round, uint32_t epoch,
+__device__ __forceinline__ uint32_t sum_earlier(const u64* status, uint32_t tile, uint32_t first, uint32_t epoch,
                                                 uint32_t thread, uint32_t threads, bool* timed_out,
                                                 uint32_t spin_limit = kSpinLimit) {
-    const uint32_t first = tile / round * round;
     uint32_t sum = 0;
-    for (uint32_t j = (first ? first - 1u : 0u) + thread; j < tile; j += threads) {
+    for (uint32_t j = (first ? first - 1u : 0u) + thread; j < tile && !*timed_out; j += threads) {
         uint32_t spins = 0;
         for (;;) {
             const u64 w = ld_relaxed64(status + j);
@@ -316,13 +316,12 @@ __device__ __forceinline__ uint32_t sum_earlier(const u64* status, uint32_t tile
                 sum += (uint32_t)w & kValMask;
                 break;
             }
-            if (++spins > spin_limit) { *timed_out = true; return sum; }
+            if (++spins > spin_limit) { *timed_out = true; break; }
             if (spins > 64) __nanosleep(32);
         }
     }
     return sum;
 }
-__device__ __forceinline__ bool closes_round(uint32_t tile, uint32_t round) { return tile % round == round - 1u; }
 
 // Block-wide exclusive scan of one uint32 per thread (blockDim.x <= 1024,
 // multiple of 32).  `warp_tmp` holds >= 33 words of shared memory.

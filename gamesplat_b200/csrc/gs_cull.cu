@@ -444,10 +444,11 @@ __global__ void __launch_bounds__(kCullVisThreads, kVisPerSm) cull_visible_kerne
         if (w < warp) before += c;
         total += c;
     }
-    const bool closes = closes_round(tile, round);
+    const uint32_t first = tile / round * round;
+    const bool closes = tile == first + round - 1u;
     if (t == 0 && !closes) st_relaxed64(p.status + tile, status_word(p.epoch, kFlagAgg, total));
     bool timed_out = false;
-    uint32_t sum = sum_earlier(p.status, tile, round, p.epoch, (uint32_t)t, kCullVisThreads, &timed_out);
+    uint32_t sum = sum_earlier(p.status, tile, first, p.epoch, (uint32_t)t, kCullVisThreads, &timed_out);
     if (timed_out) atomicOr(&p.fc->error_flags, kErrCullLookback);
     sum = __reduce_add_sync(0xffffffffu, sum);
     if (lane == 0) s_sum[warp] = sum;

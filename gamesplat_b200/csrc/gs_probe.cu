@@ -18,7 +18,7 @@ __global__ void wait_probe_kernel(const unsigned long long* status, FrameCounter
         // so it reads as "not published yet" on every poll
         if (threadIdx.x < 32) {
             bool to = false;
-            sum_earlier(status, 1, 2, epoch, threadIdx.x, blockDim.x, &to, limit);
+            sum_earlier(status, 1, 0, epoch, threadIdx.x, blockDim.x, &to, limit);
             if (threadIdx.x == 0 && to) atomicOr(&fc->error_flags, kErrCullLookback);
         }
     } else {

@@ -281,7 +281,10 @@ int launch_pack_half_rows(const float4* rows, float4* half_rows, uint32_t n, uin
 // State batches (gs_render_anim_batch): frames of one geometry that differ in
 // colours only.  The frames are taken in groups of 8 (the last one of 4 when
 // that holds the rest); a group's colours lie together per record, channel
-// by channel: 3 x group-width floats, group after group, cap records each.
+// by channel: 3 x group-width floats, group after group, cap records each.  1M
+// Gaussians, 1920x1080: one to four frames take 534, 558, 588, 611 us in a group of
+// 4 (667, 1087, 1479, 1923 when each was drawn alone), five to eight 732 to 792 in
+// one of 8.
 constexpr int kMaxBatchFrames = 256;
 struct StateBatch {
     int32_t a[kMaxBatchFrames], b[kMaxBatchFrames];   // appearance states of each frame and

@@ -217,10 +217,17 @@ def run_reference(args):
     the CPU oracle's restatement of that path (cull + SH + sort + composite,
     kind "port"), with rows and cameras built by the reference's own loader
     and camera code; the reference's own CPU cull + sort is timed beside it.
+    Where that code is not built (its sources are missing) the line says so.
     Rank 0 alone runs; the other ranks exit without work."""
     rank = int(os.environ.get("RANK", "0"))
     world = int(os.environ.get("WORLD_SIZE", str(args.gpus)))
     if rank != 0:
+        return
+    from oracle import oracle as O
+
+    if not O.ref_available():
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref not built (needs the reference sources)"}),
+              flush=True)
         return
     cores = os.cpu_count() or 1
     os.environ.setdefault("OMP_NUM_THREADS", str(cores))

@@ -122,8 +122,9 @@ __device__ __forceinline__ float2 hash13(const PixelHash2& h, float p2) {
 // also admit s = -0 and the negative subnormal of the last place; s, a sum of
 // conic_x dx^2 >= +0, a product and conic_z dy^2 >= +0, never is -0, and is that
 // subnormal only if all terms are below 2^-125, a splat of sigma above 2^38
-// pixels.  These tests are the loop's comparisons, on the ALU pipe that bounds
-// the rasterizers (see raster_kernel): 310 -> 287 us for the alpha frame there.
+// pixels.  These tests are the loop's comparisons, on the rasterizers' busiest
+// pipe, the ALU's (64 % before them): 310 -> 287 us for the alpha frame of
+// raster_kernel.
 template <class M>
 __device__ __forceinline__ bool frag_live(M bits, M need, float s, float s_max) {
     return (need & ~bits) == (M)0 && __float_as_uint(s) <= __float_as_uint(s_max);
